@@ -59,6 +59,10 @@ struct gwl_analysis {
   float* freq_f = nullptr;
   float2* basis = nullptr;
   double4* ftab = nullptr;  // float64 TaylorF2: {f^(1/3), ln(f) / 3, f^(-5/3), f^(-7/6)} per bin
+  uint4* wide_phi = nullptr;  // float64 TaylorF2: LaunchArgs::wide_phi, wide_tab, wide_w, wide_scale, wide_lnref
+  float4* wide_tab = nullptr;
+  uint4* wide_w[kMaxDet] = {};
+  double wide_scale[kNumBasis] = {}, wide_lnref = 0, step_lo = 0;
   float* anchors = nullptr;
   int64_t n_anchors = 0;
   double* strain[kMaxDet] = {};
@@ -179,6 +183,8 @@ struct gwl_analysis {
   double* d_params = nullptr;
   double* d_out = nullptr;
   PointRec* d_rec = nullptr;
+  uint64_t* d_wide = nullptr;  // float64 TaylorF2: [kWideWords][wide_B], from the first such evaluation on
+  int64_t wide_B = 0;
   double* d_part = nullptr;
   size_t part_bytes = 0;
   int32_t* d_order = nullptr;       // [ws_B] point ordering of the mixed TaylorF2 kernel
@@ -232,6 +238,7 @@ void free_workspace(gwl_analysis* a) {
   cudaFree(a->d_params);
   cudaFree(a->d_out);
   cudaFree(a->d_rec);
+  cudaFree(a->d_wide);
   cudaFree(a->d_part);
   cudaFree(a->d_order);
   cudaFree(a->d_order_hist);
@@ -244,6 +251,8 @@ void free_workspace(gwl_analysis* a) {
   a->h_params = a->h_out = nullptr;
   a->d_params = a->d_out = a->d_part = a->d_tm = nullptr;
   a->d_rec = nullptr;
+  a->d_wide = nullptr;
+  a->wide_B = 0;
   a->d_order = a->d_order_hist = nullptr;
   a->last_rf_count = nullptr;
   a->ws_B = 0;
@@ -314,6 +323,69 @@ void basis_taylor(double f, double df, double T[kAnchorOrders][kNumBasis]) {
   }
 }
 
+// The basis functions at frequency f (wide_lnref subtracted from ln f) as
+// float64 pairs hi + lo; lo = 0 for the last four, whose coefficients stay
+// within tens of cycles.
+void wide_basis(double f, double lnref, double* hi, double* lo) {
+  const double y = std::cbrt(f), p = y * y, pe = std::fma(y, y, -p), t = p * y, te = std::fma(p, y, -t) + pe * y;
+  const double yl = ((f - t) - te) / (3.0 * p);
+  const double h3 = 1.0 / y, l3 = (std::fma(-h3, y, 1.0) - h3 * yl) * h3;
+  const double h2 = h3 * h3, l2 = std::fma(h3, h3, -h2) + 2.0 * h3 * l3;
+  const double h1 = 1.0 / f, l1 = std::fma(-h1, f, 1.0) * h1;
+  hi[0] = h1 * h2;
+  lo[0] = std::fma(h1, h2, -hi[0]) + (h1 * l2 + l1 * h2);
+  hi[1] = h1;
+  lo[1] = l1;
+  hi[2] = h2;
+  lo[2] = l2;
+  hi[3] = h3;
+  lo[3] = l3;
+  const double ln = std::log(f) - lnref;
+  hi[4] = ln > 0 ? ln : 0.0;
+  hi[5] = y;
+  hi[6] = y * hi[4];
+  hi[7] = p;
+  for (int b = 4; b < kNumBasis; ++b) lo[b] = 0.0;
+}
+
+// hi + lo in [0, 1) as 0.64 fixed point
+uint64_t wide_fraction(double hi, double lo) {
+  return (uint64_t)std::ldexp(hi, 64) + (uint64_t)(int64_t)std::llrint(std::ldexp(lo, 64));
+}
+
+// LaunchArgs::wide_phi over the increasing positive frequencies f[k0 .. n)
+// (zero elsewhere), scaled by powers of two above each function's largest
+// value there.
+void wide_table(const double* f, int64_t k0, int64_t n, int64_t pad, std::vector<uint4>* out, double* scale,
+                double* lnref) {
+  out->assign((size_t)pad * (kNumBasis / 2), make_uint4(0u, 0u, 0u, 0u));
+  for (int b = 0; b < kNumBasis; ++b) scale[b] = 1.0;
+  while (k0 < n && !(f[k0] > 0)) ++k0;
+  if (k0 >= n) return;
+  *lnref = std::log(f[k0]);
+  double top[kNumBasis], end[kNumBasis], lo[kNumBasis];
+  wide_basis(f[k0], *lnref, top, lo);
+  wide_basis(f[n - 1], *lnref, end, lo);
+  double inv[kNumBasis];
+  for (int b = 0; b < kNumBasis; ++b) {
+    int e = 0;
+    std::frexp(std::max({top[b], end[b], 1e-300}) * (1.0 + 1e-9), &e);
+    scale[b] = std::ldexp(1.0, e);
+    inv[b] = std::ldexp(1.0, -e);
+  }
+  for (int64_t k = k0; k < n; ++k) {
+    double h[kNumBasis], l[kNumBasis];
+    wide_basis(f[k], *lnref, h, l);
+    uint64_t v[kNumBasis];  // rounded to 58 bits (below 1: the scale leaves a margin of 1e-9)
+    for (int b = 0; b < kNumBasis; ++b) v[b] = (wide_fraction(h[b] * inv[b], l[b] * inv[b]) + 32) >> 6;
+    for (int b = 0; b < kNumBasis / 2; ++b) {
+      const uint64_t x = v[2 * b], y = v[2 * b + 1];
+      (*out)[(size_t)k * (kNumBasis / 2) + b] =
+          make_uint4((uint32_t)(x & 0x7ffffff), (uint32_t)(x >> 27), (uint32_t)(y & 0x7ffffff), (uint32_t)(y >> 27));
+    }
+  }
+}
+
 int g_sm_count = 0;
 
 int sm_count() {
@@ -374,6 +446,12 @@ LaunchArgs make_args(gwl_analysis* a, int64_t B, int precision) {
   L.freq_f = a->freq_f;
   L.basis = a->basis;
   L.ftab = a->ftab;
+  L.wide_phi = a->wide_phi;
+  L.wide_tab = a->wide_tab;
+  for (int d = 0; d < a->n_det; ++d) L.wide_w[d] = a->wide_w[d];
+  for (int b = 0; b < kNumBasis; ++b) L.wide_scale[b] = a->wide_scale[b];
+  L.wide_lnref = a->wide_lnref;
+  L.step_lo = a->step_lo;
   L.anchors = a->anchors;
   L.n_anchors = a->n_anchors;
   L.status = a->d_status;
@@ -869,6 +947,19 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
     }
     return GWL_OK;
   }
+  const bool wide = precision == GWL_PRECISION_FP64 && a->model == GWL_MODEL_TAYLORF2 && !(a->time_marg && d_out);
+  if (wide) {
+    L.cplx = a->phase_marg;  // the real part suffices unless |<d|h>| is needed
+    if (B > a->wide_B) {
+      GWL_CUDA(cudaStreamSynchronize(s));
+      cudaFree(a->d_wide);
+      a->d_wide = nullptr;
+      a->wide_B = 0;
+      if ((rc = dev_alloc(a, &a->d_wide, (size_t)kWideWords * a->ws_B, false))) return rc;
+      a->wide_B = a->ws_B;
+    }
+    L.wide_c = a->d_wide;
+  }
   if (d_dh) L.cplx = 1;  // complex <d|h> requested
   const bool ordered = precision == GWL_PRECISION_MIXED && a->model == GWL_MODEL_TAYLORF2 && !(a->time_marg && d_out);
   if (ordered) {
@@ -878,6 +969,14 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
     if (a->time_marg && d_out) L.rf_tol = 0.0;  // the time-marginalised kernel has its own integrand
     ordering_with_marks(L);
     a->last_rf_count = L.rf_count;
+    GWL_CUDA(cudaMemsetAsync(L.order_hist, 0, sizeof(int32_t) * (2 * L.order_keys + 1), s));
+  } else if (wide && B >= kWideOrderPoints) {
+    // a warp's points stop at nearly the same bin (LaunchArgs::order)
+    L.rf_tol = 0.0;
+    L.order = a->d_order;
+    L.order_hist = a->d_order_hist;
+    ordering_with_marks(L);
+    L.rf_count = nullptr;
     GWL_CUDA(cudaMemsetAsync(L.order_hist, 0, sizeof(int32_t) * (2 * L.order_keys + 1), s));
   } else if (precision == GWL_PRECISION_MIXED && a->model == GWL_MODEL_SINEGAUSSIAN && !(a->time_marg && d_out)) {
     // sine-Gaussian: points ordered by centre frequency; the finalize marks
@@ -929,7 +1028,9 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
     GWL_CUDA(side_fork(a->side, s));
     GWL_CUDA(launch_mixed_acc(L, a->side.stream));
   }
-  if (precision == GWL_PRECISION_FP64) {
+  if (wide) {
+    GWL_CUDA(launch_wide(L, s));
+  } else if (precision == GWL_PRECISION_FP64) {
     GWL_CUDA(launch_plain(L, s));
   } else {
     GWL_CUDA(launch_mixed(L, s));
@@ -939,6 +1040,7 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
     a->ev_pending = 1;
   }
   if (acc) GWL_CUDA(side_join(a->side, s));
+  if (wide) return GWL_OK;  // launch_wide ends with the totals
   GWL_CUDA(launch_finalize(L, s));
   if (precision == GWL_PRECISION_MIXED && a->model == GWL_MODEL_SINEGAUSSIAN && L.rf_tol > 0)
     GWL_CUDA(launch_sg_refine(L, s));
@@ -1051,6 +1153,7 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
   const double* f = desc->frequency;
   // The kernels take f_k = k * step (bilby's linspace(0, fs/2, N) grid).
   a->step = f[N - 1] / (double)(N - 1);
+  a->step_lo = std::fma(-a->step, (double)(N - 1), f[N - 1]) / (double)(N - 1);
   for (int64_t k = 0; k < N; ++k) {
     if (std::fabs(f[k] - k * a->step) > 1e-9 * std::max(1.0, f[N - 1])) {
       set_error("frequency_array is not the uniform grid k * df starting at 0");
@@ -1143,6 +1246,11 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
         ft[k] = make_double4(std::cbrt(x), std::log(x) / 3.0, std::pow(x, -5.0 / 3.0), std::pow(x, -7.0 / 6.0));
       }
       if ((rc = upload(a, &a->ftab, ft))) goto fail;
+      {
+        std::vector<uint4> phi;
+        wide_table(f, a->k_fmin, N, P, &phi, a->wide_scale, &a->wide_lnref);
+        if ((rc = upload(a, &a->wide_phi, phi))) goto fail;
+      }
       // Taylor tables of the basis every kAnchorStep bins (f = k * df)
       a->n_anchors = N / kAnchorStep + 2;
       std::vector<float> anc((size_t)a->n_anchors * kAnchorFloats, 0.f);
@@ -1167,8 +1275,26 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
         ct[q] = make_float4(ch, (float)(c - (double)ch), sh, (float)(sn - (double)sh));
       }
       if ((rc = upload(a, &a->cos_tab, ct))) goto fail;
+      std::vector<float4> wt(kWideTable);
+      for (int q = 0; q < kWideTable; ++q) {
+        const double x = 2.0 * M_PI * q / kWideTable;
+        const double c = q % (kWideTable / 4) == 0 ? std::round(std::cos(x)) : std::cos(x);
+        const double t = -2.0 * M_PI / kWideTable * (q % (kWideTable / 4) == 0 ? std::round(std::sin(x)) : std::sin(x));
+        const float2 cf = split_ff(c), tf = split_ff(t);
+        wt[q] = make_float4(cf.x, cf.y, tf.x, tf.y);
+      }
+      if ((rc = upload(a, &a->wide_tab, wt))) goto fail;
     }
     a->noise_lnl = 0.0;
+    std::vector<double> f76, f73;  // f^(-7/6), f^(-7/3)
+    if (a->model == GWL_MODEL_TAYLORF2) {
+      f76.resize((size_t)N);
+      f73.resize((size_t)N);
+      for (int64_t k = 0; k < N; ++k) {
+        f76[k] = f[k] > 0 ? std::pow(f[k], -7.0 / 6.0) : 0.0;  // (no model at zero frequency)
+        f73[k] = f[k] > 0 ? std::pow(f[k], -7.0 / 3.0) : 0.0;
+      }
+    }
     for (int d = 0; d < a->n_det; ++d) {
       const gwl_detector& det = desc->detectors[d];
       std::vector<double> s(2 * P, 0.0), ip(P, 0.0);
@@ -1190,7 +1316,7 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
       double wmax = 0.0, vmax = 0.0;
       for (int64_t k = 0; k < N; ++k) {
         if (ip[k] == 0.0) continue;
-        const double amp = a->model == GWL_MODEL_TAYLORF2 ? std::pow(f[k], -7.0 / 6.0) : 1.0;
+        const double amp = a->model == GWL_MODEL_TAYLORF2 ? f76[k] : 1.0;
         wr[k] = amp * s[2 * k] * ip[k];
         wi[k] = amp * s[2 * k + 1] * ip[k];
         wmax = std::max(wmax, std::max(std::fabs(wr[k]), std::fabs(wi[k])));
@@ -1207,14 +1333,23 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
       if ((rc = upload(a, &a->w[d], wf))) goto fail;
       if (a->model == GWL_MODEL_TAYLORF2) {
         std::vector<uint2> wpol(P, make_uint2(0u, 0u));
+        std::vector<uint4> wide(P, make_uint4(0u, 0u, 0u, 0u));
         for (int64_t k = 0; k < N; ++k) {
           const double x = wr[k] / a->w_scale[d], y = wi[k] / a->w_scale[d];
           // odd bins carry -|w| at arg(w) + 1/2 cycle (the same term): a mean
           // error of the float32 cosine then cancels between neighbouring bins
           // instead of adding up coherently with the positive magnitudes
           const bool odd = (k & 1) != 0;
-          const float mag = (float)(odd ? -std::hypot(x, y) : std::hypot(x, y));
-          double cyc = std::atan2(y, x) / (2.0 * M_PI) + (odd ? 0.5 : 0.0);
+          const double abs_w = std::hypot(x, y), turn = std::atan2(y, x) / (2.0 * M_PI);
+          const float2 wm = split_ff(abs_w);
+          const uint64_t wt = wide_fraction(turn < 0 ? turn + 1.0 : turn, 0.0);
+          uint32_t* pair = reinterpret_cast<uint32_t*>(&wide[k & ~(int64_t)1]);
+          std::memcpy(pair + (k & 1), &wm.x, 4);
+          std::memcpy(pair + 2 + (k & 1), &wm.y, 4);
+          pair[4 + 2 * (k & 1)] = (uint32_t)wt;
+          pair[5 + 2 * (k & 1)] = (uint32_t)(wt >> 32);
+          const float mag = (float)(odd ? -abs_w : abs_w);
+          double cyc = turn + (odd ? 0.5 : 0.0);
           cyc -= std::floor(cyc);
           const uint32_t th = (uint32_t)(uint64_t)std::llround(cyc * 4294967296.0);  // 2^32 wraps to 0
           uint32_t mb;
@@ -1222,6 +1357,7 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
           wpol[k] = make_uint2(mb, th);
         }
         if ((rc = upload(a, &a->wp[d], wpol))) goto fail;
+        if ((rc = upload(a, &a->wide_w[d], wide))) goto fail;
         // the fast kernel's pairs: magnitudes side by side, then the angle at
         // the first bin of each 8-bin block and the increment over the
         // previous bin elsewhere (P is a multiple of 16)
@@ -1245,7 +1381,7 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
         std::vector<double> pre(N + 1, 0.0);
         KahanSum acc;
         for (int64_t k = 0; k < N; ++k) {
-          if (ip[k] != 0.0 && f[k] > 0) acc.add(std::pow(f[k], -7.0 / 3.0) * ip[k]);
+          if (ip[k] != 0.0 && f[k] > 0) acc.add(f73[k] * ip[k]);
           pre[k + 1] = acc.value();
         }
         if ((rc = upload(a, &a->hh_prefix[d], pre))) goto fail;

@@ -41,6 +41,10 @@ constexpr double kRefineL1 = 1e-7;
 constexpr double kRefineLoudPower = 10.0;
 constexpr double kRefineDefaultTol = 5e-4;
 constexpr int kCosTable = 1024;        // angles of the float-float cos / sin table of the accurate kernel
+constexpr int kWideOrderPoints = 64;   // ... and from this size on, ordered by band end
+constexpr int kWideFewPoints = 24;     // float64 TaylorF2 batches up to this size run one CTA per (chunk, point)
+constexpr int kWideWords = kNumBasis + 2 + 2 * kMaxDet;  // words per point of LaunchArgs::wide_c
+constexpr int kWideTable = 2048;       // angles of the float-float cosine table of gwl_wide.cuh
 constexpr int kRoqSplits = 8;          // node groups of the mixed ROQ time-marginalised matrix products
 
 // Per-point quantities computed once per evaluation by the float64 prologue.
@@ -110,6 +114,18 @@ struct LaunchArgs {
   double w_scale[kMaxDet], v_scale[kMaxDet];
   const float2* basis;                  // [n_pad][kNumBasis] float-float phase basis
   const double4* ftab;                  // [n_pad] {f^(1/3), ln(f) / 3, f^(-5/3), f^(-7/6)} (float64 TaylorF2)
+  // float64 TaylorF2 (gwl_wide.cu): the phase basis and the weights f^(-7/6) d / S
+  // in fixed point and float-float, and per point the phase coefficients
+  const uint4* wide_phi;                // [n_pad][kNumBasis / 2] two basis functions / wide_scale each, 0.58 fixed
+                                        // point {low 27 bits, high 31 bits}
+  const float4* wide_tab;               // [kWideTable] {cos hi, lo, -2 pi / kWideTable sin hi, lo}
+  const uint4* wide_w[kMaxDet];         // [n_pad] per bin pair {|w| / w_scale of both, hi words then lo (floats)},
+                                        // {arg(w) of both, 0.64 cycles {lo, hi} each}
+  double wide_scale[kNumBasis];         // powers of two above each basis function's largest value
+  double wide_lnref;                    // ln f of the basis functions is ln f - wide_lnref
+  double step_lo;                       // step + step_lo: the grid spacing to twice float64's digits
+  uint64_t* wide_c;                     // [kWideWords][B]: c_b wide_scale_b 2^(58 - s), the constant, s + 2, per
+                                        // detector the shift per bin and the offset (cycles, 64-bit fractions)
   const float* anchors;                 // [n_anchors][kAnchorFloats] Taylor tables of the basis
   int64_t n_anchors;
   const double* params;                 // [GWL_NPARAM][B]
@@ -305,6 +321,8 @@ cudaError_t launch_multi(const MultiArgs& m, const int* ctas, const int* ctas_ac
 int multi_tf2_ctas_per_sm(int q, bool acc);
 cudaError_t launch_prologue(const LaunchArgs& a, cudaStream_t s);
 cudaError_t launch_plain(const LaunchArgs& a, cudaStream_t s);
+// The float64 TaylorF2 likelihood (gwl_wide.cu): partial sums, totals and lnL.
+cudaError_t launch_wide(const LaunchArgs& a, cudaStream_t s);
 cudaError_t launch_mixed(const LaunchArgs& a, cudaStream_t s);
 // The accurate kernel for the marked points (nothing when rf_tol <= 0).
 cudaError_t launch_mixed_acc(const LaunchArgs& a, cudaStream_t s);

@@ -45,6 +45,63 @@ __device__ __forceinline__ int order_key(const LaunchArgs& a, const PointRec& r)
 }
 
 // ---------------------------------------------------------------------------
+// The fixed-point coefficients of gwl_wide.cu (LaunchArgs::wide_c) of point i.
+// ---------------------------------------------------------------------------
+// frac(x + lo) as a 64-bit fraction, |lo| < 1/2
+__device__ __forceinline__ uint64_t to_wide(double x, double lo) {
+  double fr = ldexp(x - floor(x), 64);
+  if (!(fr >= 0.0 && fr < 18446744073709551616.0)) fr = 0.0;
+  return (uint64_t)fr + (uint64_t)(int64_t)ldexp(lo, 64);
+}
+
+__device__ __noinline__ void wide_coefficients(const LaunchArgs& a, const PointRec& r, int64_t i, double m1, double m2,
+                                               const double* c, double cconst) {
+  uint64_t* w = a.wide_c + i;
+  // c_0 = 3 / (128 eta) (pi M)^(-5/3) / (2 pi) = K M^(1/3) / (m1 m2) to twice
+  // float64's digits: its relative error is the same in every bin, where the
+  // phase reaches 10^4 cycles
+  const double kh = 388209.13757985964, kl = -1.9320279142889344e-11;  // 3 / (256 pi) (pi G M_sun / c^3)^(-5/3)
+  const double m = m1 + m2, ml = m1 > m2 ? m2 - (m - m1) : m1 - (m - m2);
+  const double y = cbrt(m), p = y * y, pe = fma(y, y, -p), t = p * y, te = fma(p, y, -t) + pe * y;
+  const double yl = ((m - t) - te + ml) / (3.0 * p);
+  const double nh = kh * y, nl = fma(kh, y, -nh) + (kh * yl + kl * y);
+  const double dh = m1 * m2, dl = fma(m1, m2, -dh);
+  const double q0 = nh / dh, q1 = (fma(-q0, dh, nh) + (nl - q0 * dl)) / dh;
+  // the others as the mixed kernels have them, u = (pi M)^(1/3); ln f relative to wide_lnref
+  double x[kNumBasis], xl = q1;
+  x[0] = q0;
+  const double P = 3.0 / (128.0 * r.eta) / kTwoPi, pm = kPi * r.m_sec, u = cbrt(pm);
+  x[1] = P * r.a[2] / pm;
+  x[2] = P * r.a[3] * u / pm;
+  x[3] = P * r.a[4] / u;
+  x[4] = c[4];
+  x[5] = c[5] + c[6] * a.wide_lnref;
+  x[6] = c[6];
+  x[7] = c[7];
+  // integers of 2^(58 - s), s the exponent above the largest of them, as {high, low 27 bits}
+  double top = 0.0;
+#pragma unroll
+  for (int b = 0; b < kNumBasis; ++b) {
+    x[b] *= a.wide_scale[b];
+    top = fmax(top, fabs(x[b]));
+  }
+  xl *= a.wide_scale[0];
+  const int s = top > 1.0 && isfinite(top) ? min(ilogb(top) + 1, 58) : 1;
+#pragma unroll
+  for (int b = 0; b < kNumBasis; ++b) {
+    const int64_t n = __double2ll_rn(ldexp(x[b], 58 - s)) + (b == 0 ? __double2ll_rn(ldexp(xl, 58 - s)) : 0);
+    w[(int64_t)b * a.B] = ((uint64_t)(uint32_t)(int32_t)(n >> 27) << 32) | (uint32_t)(n & 0x7ffffff);
+  }
+  w[(int64_t)kNumBasis * a.B] = to_wide(cconst + c[4] * a.wide_lnref, 0.0);
+  w[(int64_t)(kNumBasis + 1) * a.B] = (uint64_t)(s + 2);
+  for (int d = 0; d < a.n_det; ++d) {
+    const double v = r.dt[d] * a.step, e = fma(r.dt[d], a.step, -v) + r.dt[d] * a.step_lo;
+    w[(int64_t)(kNumBasis + 2 + d) * a.B] = to_wide(v, e);
+    w[(int64_t)(kNumBasis + 2 + kMaxDet + d) * a.B] = ((uint64_t)r.qfix[d][1] << 32) | r.qfix[d][0];
+  }
+}
+
+// ---------------------------------------------------------------------------
 // prologue: per-point float64 set-up (sky frame, antenna, delays, model scalars)
 // ---------------------------------------------------------------------------
 __device__ __noinline__ void prologue_point(const LaunchArgs& a, int64_t i) {
@@ -169,6 +226,7 @@ __device__ __noinline__ void prologue_point(const LaunchArgs& a, int64_t i) {
     const ff s = ff_from_double(cconst - floor(cconst));
     r.c_hi[kNumBasis] = s.hi;
     r.c_lo[kNumBasis] = s.lo;
+    if (a.wide_c) wide_coefficients(a, r, i, m1, m2, c, cconst);
   }
   r.valid = ok ? 1 : 0;
   if (a.rf_tol > 0 && a.rf_count && r.valid && a.model == GWL_MODEL_TAYLORF2) {
@@ -377,101 +435,6 @@ __global__ void __launch_bounds__(kPointsPerCta) k_plain_sg(LaunchArgs a) {
     out[0 * a.B] = dre[d];
     out[1 * a.B] = dim[d];
     out[2 * a.B] = hh[d];
-  }
-}
-
-// TaylorF2, float64.  Per bin: v = u f^(1/3), ln v = ln u + ln(f) / 3 and
-// the f^(-5/3), f^(-7/6) factors from the per-analysis table, the 3.5PN phase
-// by Horner's rule, one sincos, and each detector's time shift e^{-2 pi i f dt}
-// by rotation on the chunk's uniform grid.  <h|h> comes from the analysis's
-// prefix sums of f^(-7/3) / S (finalize), so only <d|h> is summed here.
-template <int D>
-__global__ void __launch_bounds__(kPointsPerCta) k_plain_tf2(LaunchArgs a) {
-  constexpr int CH = kChunkPlain;
-  __shared__ double s_f[CH];
-  __shared__ double4 s_t[CH];
-  __shared__ double2 s_d[D][CH];
-  __shared__ double s_is[D][CH];
-  const int64_t k0 = a.k_base + (int64_t)blockIdx.y * CH;
-  for (int j = threadIdx.x; j < CH; j += blockDim.x) {
-    const int64_t k = k0 + j;
-    s_f[j] = a.freq[k];
-    s_t[j] = a.ftab[k];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      s_d[d][j] = reinterpret_cast<const double2*>(a.strain[d])[k];
-      s_is[d][j] = a.inv_psd[d][k];
-    }
-  }
-  __syncthreads();
-  const int64_t i = (int64_t)blockIdx.x * kPointsPerCta + threadIdx.x;
-  if (i >= a.B) return;
-  const PointRec& r = a.rec[i];
-  double dre[D], dim[D], fp[D], fx[D];
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    dre[d] = dim[d] = 0.0;
-    fp[d] = r.fp[d];
-    fx[d] = r.fx[d];
-  }
-  if (r.valid && k0 < r.k_end && k0 + CH > r.k_start) {
-    double ak[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) ak[k] = r.a[k];
-    const double l5 = r.l[5], l6 = r.l[6];
-    const double u = cbrt(kPi * r.m_sec), lnu = log(u);
-    const double amp0 = r.amp, ci = r.cos_i, f_isco = r.f_isco;
-    const double pu5 = 3.0 / (128.0 * r.eta) / (u * u * u * u * u), cphase = -2.0 * r.phase - kPi / 4;
-    const double pfac = (1.0 + ci * ci) / 2.0;
-    double zc[D], zs[D], rc[D], rs[D];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      const double w2 = 2.0 * kPi * r.dt[d];
-      sincos(w2 * s_f[0], &zs[d], &zc[d]);
-      sincos(w2 * a.step, &rs[d], &rc[d]);
-    }
-    for (int j = 0; j < CH; ++j) {
-      const double f = s_f[j];
-      if (f >= a.fmin && f < f_isco) {
-        // the TaylorF2 model (oracle/taylorf2.py) evaluated in float64
-        const double4 t = s_t[j];
-        const double v = u * t.x;
-        const double lnv = lnu + t.y;
-        double s = ak[7];
-#pragma unroll
-        for (int k = 6; k >= 0; --k) s = s * v + ak[k];
-        const double v5 = v * v * v * v * v;
-        s = s + lnv * (l5 + l6 * v) * v5;
-        const double psi = cphase + pu5 * s * t.z;
-        const double amp = amp0 * t.w;
-        double sp, cp;
-        sincos(psi, &sp, &cp);  // exp(-i psi) = cp - i sp
-        const double ere = amp * cp, eim = -amp * sp;
-        // h_+ = pfac * e, h_x = -i ci * e
-        const double hpre = pfac * ere, hpim = pfac * eim;
-        const double hxre = ci * eim, hxim = -ci * ere;
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-          const double is = s_is[d][j];
-          const double sre = hpre * fp[d] + hxre * fx[d];
-          const double sim = hpim * fp[d] + hxim * fx[d];
-          const double sn = zs[d], cs = zc[d];  // exp(-i w f) = cs - i sn
-          const double hre = sre * cs + sim * sn;
-          const double him = sim * cs - sre * sn;
-          const double2 dd = s_d[d][j];
-          dre[d] += (hre * dd.x + him * dd.y) * is;
-          dim[d] += (hre * dd.y - him * dd.x) * is;
-        }
-      }
-#pragma unroll
-      for (int d = 0; d < D; ++d) rotate(zc[d], zs[d], rc[d], rs[d]);
-    }
-  }
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    double* out = a.part + (((int64_t)blockIdx.y * D + d) * kPartStride) * a.B + i;
-    out[0 * a.B] = dre[d];
-    out[1 * a.B] = dim[d];
   }
 }
 
@@ -1148,7 +1111,6 @@ __global__ void __launch_bounds__(kSgPointsPerCta) k_mixed_sg(LaunchArgs a) {
 // arithmetic), one CTA per point, fixed-order reduction, then the point's
 // lnL replaces the mixed one.
 constexpr int kSgRefineThreads = 256;
-__device__ void finish_point(const LaunchArgs& a, const PointRec& r, int64_t i, double dr, double di, double hh);
 
 template <int D>
 __global__ void __launch_bounds__(kSgRefineThreads) k_sg_refine(LaunchArgs a) {
@@ -1224,8 +1186,6 @@ __global__ void __launch_bounds__(kSgRefineThreads) k_sg_refine(LaunchArgs a) {
 // ---------------------------------------------------------------------------
 // finalize: fixed-order reduction over chunks, <d|h>, <h|h>, marginalisation
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double neg_huge() { return -1.7976931348623157e308; }  // nan_to_num(-inf)
-
 // p[t] = sum over groups c = 0, 1, ... (in that order) of the partial sums
 // of detector d; the loads of 8 (or 4) groups are issued before their adds.
 template <int NQ>
@@ -1268,25 +1228,15 @@ __device__ void detector_totals(const LaunchArgs& a, int64_t i, int64_t G, const
   double sdr = 0.0, sdi = 0.0, shh = 0.0;
   for (int d = 0; d < a.n_det; ++d) {
     double p[kPartStride] = {0, 0, 0, 0, 0, 0};
-    if (a.precision == GWL_PRECISION_FP64) {
-      if (a.model == GWL_MODEL_SINEGAUSSIAN) sum_groups<3>(a, i, d, G, p);
-      else sum_groups<2>(a, i, d, G, p);
-    } else if (a.model == GWL_MODEL_SINEGAUSSIAN) sum_groups<4>(a, i, d, G, p);
+    if (a.precision == GWL_PRECISION_FP64) sum_groups<3>(a, i, d, G, p);
+    else if (a.model == GWL_MODEL_SINEGAUSSIAN) sum_groups<4>(a, i, d, G, p);
     else if (a.cplx) sum_groups<2>(a, i, d, G, p);
     else sum_groups<1>(a, i, d, G, p);
     double dr, di, h;
-    if (a.precision == GWL_PRECISION_FP64 && a.model == GWL_MODEL_SINEGAUSSIAN) {
+    if (a.precision == GWL_PRECISION_FP64) {
       dr = norm * p[0];
       di = norm * p[1];
       h = norm * p[2];
-    } else if (a.precision == GWL_PRECISION_FP64) {
-      // <h|h> = A0^2 |Q|^2 sum_band f^(-7/3) / S
-      dr = norm * p[0];
-      di = norm * p[1];
-      const double ci = r.cos_i;
-      const double qr = r.fp[d] * (1.0 + ci * ci) / 2.0, qi = -r.fx[d] * ci;
-      const int64_t k1 = min(r.k_end, a.n_bins), k0 = min(r.k_start, k1);
-      h = norm * r.amp * r.amp * (qr * qr + qi * qi) * (a.hh_prefix[d][k1] - a.hh_prefix[d][k0]);
     } else if (a.model == GWL_MODEL_SINEGAUSSIAN) {
       // conj(h) = M (a hp + i c hx) e^{+i theta}, M = |(Fp P, Fx X)| (see k_mixed_sg)
       const double M = hypot(r.fp[d] * r.amp, r.fx[d] * r.amp2), ws = a.w_scale[d], vs = a.v_scale[d];
@@ -1295,22 +1245,7 @@ __device__ void detector_totals(const LaunchArgs& a, int64_t i, int64_t G, const
       h = norm * vs * M * M * p[2];
       if (err) *err += kSgRandomErr * norm * ws * M * sqrt(fmax(p[3], 0.0));
     } else {
-      // conj(h_det) = A0 f^(-7/6) conj(Q) e^{+i Phi},  Q = Fp (1 + c^2)/2 - i Fx c
-      const double ci = r.cos_i;
-      const double qr = r.fp[d] * (1.0 + ci * ci) / 2.0, qi = -r.fx[d] * ci;
-      const double s = norm * a.w_scale[d] * r.amp;
-      if (a.cplx) {
-        // (qr - i qi) * (p0 + i p1)
-        dr = s * (qr * p[0] + qi * p[1]);
-        di = s * (qr * p[1] - qi * p[0]);
-      } else {
-        // p0 = Re sum w e^{i (phase + alpha_d)} (see PointRec::qfix)
-        dr = s * r.qabs[d] * p[0];
-        di = 0.0;
-      }
-      const int64_t k1 = min(r.k_end, a.n_bins), k0 = min(r.k_start, k1);
-      const double* pre = a.hh_prefix[d];
-      h = norm * r.amp * r.amp * (qr * qr + qi * qi) * (pre[k1] - pre[k0]);
+      tf2_detector_totals(a, r, d, p, &dr, &di, &h);
     }
     sdr += dr;
     sdi += di;
@@ -1321,19 +1256,10 @@ __device__ void detector_totals(const LaunchArgs& a, int64_t i, int64_t G, const
   *hh = shh;
 }
 
-__device__ double distance_marginalized(const LaunchArgs& a, double dh_re, double dh_im, double hh, double dist) {
-  // base.py:775-784, 879-885
-  const double hh_ref = hh * dist * dist / (a.ref_dist * a.ref_dist);
-  const double sr = dist / a.ref_dist;
-  const double dr = dh_re * sr, di = dh_im * sr;
-  const double x = a.phase_marg ? sqrt(dr * dr + di * di) : dr;
-  return bicubic_eval(a.tx, a.nx, a.ty, a.ny, a.tc, a.bbox, x, hh_ref);
-}
-
 // Components of a partial-sum record: <d|h> re/im and <h|h> (float64 kernels),
 // the six sums of the sine-Gaussian mixed kernel, re/im for TaylorF2 mixed.
 __device__ __host__ __forceinline__ int part_components(const LaunchArgs& a) {
-  if (a.precision == GWL_PRECISION_FP64) return a.model == GWL_MODEL_SINEGAUSSIAN ? 3 : 2;
+  if (a.precision == GWL_PRECISION_FP64) return 3;  // (TaylorF2 in float64 has its own finalize, gwl_wide.cu)
   return a.model == GWL_MODEL_SINEGAUSSIAN ? 4 : (a.cplx ? 2 : 1);
 }
 
@@ -1362,28 +1288,6 @@ __global__ void k_reduce_parts(LaunchArgs a) {
   if (idx >= a.B * a.n_det * nq) return;
   const int64_t i = idx % a.B, r = idx / a.B;
   reduce_chain(a, i, (int)(r / nq), (int)(r % nq));
-}
-
-// lnL of point i from its totals <d|h> = dr + i di and <h|h> (base.py:448-477
-// without time marginalisation), with the optional outputs of the totals.
-__device__ void finish_point(const LaunchArgs& a, const PointRec& r, int64_t i, double dr, double di, double hh) {
-  if (a.dh_out) {
-    a.dh_out[2 * i] = dr;
-    a.dh_out[2 * i + 1] = di;
-  }
-  if (a.hh_out) a.hh_out[i] = hh;
-  if (!a.out) return;
-  double lnl;
-  if (!r.valid) {
-    lnl = neg_huge();
-  } else if (a.dist_marg) {
-    lnl = distance_marginalized(a, dr, di, hh, r.dist);
-  } else if (a.phase_marg) {
-    lnl = ln_i0(sqrt(dr * dr + di * di)) - hh / 2;  // base.py:786-792
-  } else {
-    lnl = dr - hh / 2;  // base.py:475
-  }
-  a.out[i] = lnl;
 }
 
 // G: the groups still to be summed (1 after k_reduce_parts)
@@ -1904,11 +1808,7 @@ cudaError_t launch_prologue(const LaunchArgs& a, cudaStream_t s) {
 
 cudaError_t launch_plain(const LaunchArgs& a, cudaStream_t s) {
   dim3 grid((unsigned)((a.B + kPointsPerCta - 1) / kPointsPerCta), (unsigned)a.n_chunks);
-  if (a.model == GWL_MODEL_SINEGAUSSIAN) {
-    GWL_DISPATCH_D(k_plain_sg, grid, kPointsPerCta, 0, s, a);
-  } else {
-    GWL_DISPATCH_D(k_plain_tf2, grid, kPointsPerCta, 0, s, a);
-  }
+  GWL_DISPATCH_D(k_plain_sg, grid, kPointsPerCta, 0, s, a);
   return cudaGetLastError();
 }
 

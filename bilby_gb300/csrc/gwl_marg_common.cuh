@@ -269,6 +269,61 @@ __device__ inline double tm_sensitivity(const LaunchArgs& a, double xpk, double 
   return fmin(sr * (1.25 * d + 5e-3), 1e6);  // an undefined difference gives 1e6
 }
 
+__device__ __forceinline__ double neg_huge() { return -1.7976931348623157e308; }  // nan_to_num(-inf)
+
+__device__ inline double distance_marginalized(const LaunchArgs& a, double dh_re, double dh_im, double hh, double dist) {
+  // base.py:775-784, 879-885
+  const double hh_ref = hh * dist * dist / (a.ref_dist * a.ref_dist);
+  const double sr = dist / a.ref_dist;
+  const double dr = dh_re * sr, di = dh_im * sr;
+  const double x = a.phase_marg ? sqrt(dr * dr + di * di) : dr;
+  return bicubic_eval(a.tx, a.nx, a.ty, a.ny, a.tc, a.bbox, x, hh_ref);
+}
+
+// lnL of point i from its totals <d|h> = dr + i di and <h|h> (base.py:448-477
+// without time marginalisation), with the optional outputs of the totals.
+__device__ inline void finish_point(const LaunchArgs& a, const PointRec& r, int64_t i, double dr, double di, double hh) {
+  if (a.dh_out) {
+    a.dh_out[2 * i] = dr;
+    a.dh_out[2 * i + 1] = di;
+  }
+  if (a.hh_out) a.hh_out[i] = hh;
+  if (!a.out) return;
+  double lnl;
+  if (!r.valid) {
+    lnl = neg_huge();
+  } else if (a.dist_marg) {
+    lnl = distance_marginalized(a, dr, di, hh, r.dist);
+  } else if (a.phase_marg) {
+    lnl = ln_i0(sqrt(dr * dr + di * di)) - hh / 2;  // base.py:786-792
+  } else {
+    lnl = dr - hh / 2;  // base.py:475
+  }
+  a.out[i] = lnl;
+}
+
+// <d|h>_d = dr + i di and <h|h>_d of TaylorF2 from the sums p of f^(-7/6) d / S
+// e^{i phase}: conj(h_d) = A0 f^(-7/6) conj(Q) e^{+i Phi}, Q = Fp (1 + c^2) / 2 - i Fx c
+__device__ inline void tf2_detector_totals(const LaunchArgs& a, const PointRec& r, int d, const double* p, double* dr,
+                                           double* di, double* h) {
+  const double norm = 4.0 / a.duration;
+  const double ci = r.cos_i;
+  const double qr = r.fp[d] * (1.0 + ci * ci) / 2.0, qi = -r.fx[d] * ci;
+  const double s = norm * a.w_scale[d] * r.amp;
+  if (a.cplx) {
+    // (qr - i qi) * (p0 + i p1)
+    *dr = s * (qr * p[0] + qi * p[1]);
+    *di = s * (qr * p[1] - qi * p[0]);
+  } else {
+    // p0 = Re sum w e^{i (phase + alpha_d)} (see PointRec::qfix)
+    *dr = s * r.qabs[d] * p[0];
+    *di = 0.0;
+  }
+  const int64_t k1 = min(r.k_end, a.n_bins), k0 = min(r.k_start, k1);
+  const double* pre = a.hh_prefix[d];
+  *h = norm * r.amp * r.amp * (qr * qr + qi * qi) * (pre[k1] - pre[k0]);
+}
+
 // exp(-2 pi i t / L) for t < L / 2 in float64 and float32, one pair of tables
 // per (device, FFT length), kept for the life of the process (gwl_marg.cu).
 struct TwiddleTables {

@@ -1,0 +1,119 @@
+// Double precision without the float64 pipe.
+//
+// GB300 issues float64 at 1/64 of the float32 rate, so kernels that form
+// sines and products per (point, bin) in float64 are bound by that pipe
+// alone.  The helpers here do the same arithmetic with 32-bit instructions:
+//
+// * a phase in cycles is a 0.64 fixed-point fraction (modulo one cycle), a
+//   sum of integer products of coefficients and table entries whose absolute
+//   error stays well below that of a float64 phase;
+// * its cosine is a float-float pair (hi + lo) from a table of kWideTable angles
+//   rotated by the remainder, with an error of about 3e-14;
+// * products with a float-float weight are added by TwoSum.
+//
+// A float32 instruction pair (f32x2) works on two bins at a time.
+#pragma once
+
+#include <cstdint>
+#include <cuda_runtime.h>
+
+#include "gwl_internal.h"
+#include "gwl_phase.cuh"
+
+namespace gwl {
+
+__device__ __forceinline__ float2 splat2(float x) { return make_float2(x, x); }
+// a - b, one rounding per lane
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return fma2(b, splat2(-1.f), a); }
+
+// s + e = a + b exactly (Knuth), lane by lane
+__device__ __forceinline__ void two_sum2(float2 a, float2 b, float2& s, float2& e) {
+  s = add2(a, b);
+  const float2 bb = sub2(s, a);
+  e = add2(sub2(a, sub2(s, bb)), sub2(b, bb));
+}
+
+// One basis function's share of the phase, c phi: the coefficient as the signed
+// 59-bit integer c 2^(58 - s) = ch 2^27 + cl, the table entry phi / scale as the
+// 58-bit fraction mh 2^-31 + ml 2^-58.  The leading partial product goes to
+// acc, the two cross ones to cross (16 of which stay below 2^62), in units of
+// 2^(s - 62) and 2^(s - 89) cycles.
+__device__ __forceinline__ void wide_mac(int64_t& acc, int64_t& cross, int32_t ch, int32_t cl, int32_t ml, int32_t mh) {
+  acc += (int64_t)ch * mh;
+  cross += (int64_t)ch * ml;
+  cross += (int64_t)cl * mh;
+}
+
+// The phase in cycles modulo one as 0.64 fixed point (shift = s + 2): an error
+// of about 2^(s - 58) cycles, where a float64 phase of up to 2^s cycles has
+// several 2^(s - 53).
+__device__ __forceinline__ uint64_t wide_fraction(int64_t acc, int64_t cross, int shift) {
+  return (uint64_t)(acc + (cross >> 27)) << shift;
+}
+
+// The remainder of a 0.64 fixed-point angle about the nearest of the table's
+// kWideTable = 2^11 angles: q the table index, a + b the remainder in units of
+// the table's step, a in [-1/2, 1/2) in multiples of 2^-23 and b in [0, 2^-23)
+// of 2^-46, both exact (the angle's lowest 7 bits are dropped: 2^-57 cycle).
+static_assert(kWideTable == 2048, "wide_remainder splits the angle as 11 + 53 bits");
+__device__ __forceinline__ void wide_remainder(uint64_t angle, uint32_t& q, uint32_t& a, uint32_t& b) {
+  const uint32_t hi = (uint32_t)(angle >> 32) + (1u << 20), lo = (uint32_t)angle;
+  q = hi >> 21;
+  // 1 + a' and 2^-23 (1 + b') as float bits, a' = a + 1/2 and b' in [0, 1) of 23 bits
+  a = 0x3f800000u | (__funnelshift_l(lo, hi, 2) & 0x7fffffu);
+  b = 0x34000000u | ((lo >> 7) & 0x7fffffu);
+}
+
+// cos of the two angles q + a + b from the table entries t0, t1 = {C hi, C lo, T
+// hi, T lo} at q, C the cosine and T = -2 pi / kWideTable times the sine:
+// with u = a + b and v = (2 pi / kWideTable)^2 u^2,
+//   cos = C + T u (1 - v/6) + C (-v/2 + v^2/24)
+// (truncation below 3e-18).  T a, the largest correction (1.5e-3 at most), is an
+// error-free product; the rest is at most 1.2e-6, in float32: an error of about
+// 3e-14 rms.  |C| >= |T a| or C = 0, so three operations add them exactly.
+// sin(q + a + b) is the same function at table entry q - kWideTable / 4.
+struct WideArg {
+  float2 a, b, v, m;  // u^2 (in table steps), -v/2 + v^2/24
+};
+__device__ __forceinline__ WideArg wide_arg2(uint32_t a0, uint32_t b0, uint32_t a1, uint32_t b1) {
+  constexpr float k = 9.41238823040901e-06f;  // (2 pi / 2048)^2
+  WideArg x;
+  x.a = add2(make_float2(__uint_as_float(a0), __uint_as_float(a1)), splat2(-1.5f));
+  x.b = add2(make_float2(__uint_as_float(b0), __uint_as_float(b1)), splat2(-1.1920928955078125e-07f));  // 2^-23
+  const float2 u = add2(x.a, x.b);
+  x.v = mul2(u, u);
+  x.m = mul2(x.v, fma2(x.v, splat2(k * k / 24.0f), splat2(-0.5f * k)));
+  return x;
+}
+__device__ __forceinline__ void wide_cos2(const float4 t0, const float4 t1, const WideArg& x, float2& ch, float2& cl) {
+  constexpr float k6 = -9.41238823040901e-06f / 6.0f;
+  const float2 Ch = make_float2(t0.x, t1.x), Cl = make_float2(t0.y, t1.y);
+  const float2 Th = make_float2(t0.z, t1.z), Tl = make_float2(t0.w, t1.w);
+  const float2 p = mul2(Th, x.a);
+  float2 r = fma2(Th, x.a, mul2(p, splat2(-1.f)));
+  r = fma2(Th, x.b, r);
+  r = fma2(Tl, x.a, r);
+  r = fma2(Ch, x.m, r);
+  r = fma2(mul2(p, x.v), splat2(k6), r);
+  ch = add2(Ch, p);
+  const float2 e = sub2(p, sub2(ch, Ch));
+  cl = add2(e, add2(r, Cl));
+}
+
+// p + e = (wh + wl)(ch + cl)
+__device__ __forceinline__ void wide_term2(float2 wh, float2 wl, float2 ch, float2 cl, float2& p, float2& e) {
+  p = mul2(wh, ch);
+  e = fma2(wh, ch, mul2(p, splat2(-1.f)));
+  e = fma2(wh, cl, e);
+  e = fma2(wl, ch, e);
+}
+
+// hi + lo += p + e
+__device__ __forceinline__ void wide_add2(float2& hi, float2& lo, float2 p, float2 e) {
+  float2 s, err;
+  two_sum2(hi, p, s, err);
+  hi = s;
+  lo = add2(lo, add2(err, e));
+}
+
+}  // namespace gwl
