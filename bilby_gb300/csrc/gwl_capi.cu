@@ -15,6 +15,7 @@
 
 #include "gwl_internal.h"
 #include "gwl_math.cuh"
+#include "gwl_wide_basis.cuh"
 
 namespace gwl {
 
@@ -61,8 +62,26 @@ struct gwl_analysis {
   double4* ftab = nullptr;  // float64 TaylorF2: {f^(1/3), ln(f) / 3, f^(-5/3), f^(-7/6)} per bin
   uint4* wide_phi = nullptr;  // float64 TaylorF2: LaunchArgs::wide_phi, wide_tab, wide_w, wide_scale, wide_lnref
   float4* wide_tab = nullptr;
+  uint64_t* wide_v[kMaxDet] = {};  // sine-Gaussian: LaunchArgs::wide_v, wide_ve, wide_exp
+  int32_t* wide_ve[kMaxDet] = {};
+  uint64_t* wide_exp = nullptr;
   uint4* wide_w[kMaxDet] = {};
-  double wide_scale[kNumBasis] = {}, wide_lnref = 0, step_lo = 0;
+  double wide_scale[kNumBasis] = {}, wide_lnref = 0, step_lo = 0, wide_wscale[kMaxDet] = {};
+  // float64 TaylorF2 multi-banding on the same kernels (mb_wide: its tables are set)
+  int mb_wide = 0, mbw_bands = 0;
+  int64_t mbw_chunks = 0;
+  uint4* mbw_phi = nullptr;
+  uint4* mbw_w[kMaxDet] = {};
+  double mbw_scale[kNumBasis] = {}, mbw_lnref = 0, mbw_wscale[kMaxDet] = {};
+  int2* mbw_sub = nullptr;
+  int4* mbw_band = nullptr;
+  double* mbw_q[kMaxDet] = {};
+  // ... and relative binning (rb_wide)
+  int rb_wide = 0;
+  uint4* rbw_phi = nullptr;
+  uint4* rbw_w[kMaxDet] = {};
+  double rbw_scale[kNumBasis] = {}, rbw_lnref = 0, rbw_wscale[kMaxDet] = {}, rbw_mscale[kMaxDet] = {};
+  double* rbw_q[kMaxDet] = {};
   float* anchors = nullptr;
   int64_t n_anchors = 0;
   double* strain[kMaxDet] = {};
@@ -234,6 +253,38 @@ int upload(gwl_analysis* a, T** dst, const std::vector<T>& src) {
   return GWL_OK;
 }
 
+// The tables of gwl_analysis_create: those up to kStageBytes go to the device in
+// one allocation and one copy (an allocation and a copy each cost some 20 us,
+// and an analysis has twenty to forty tables).
+constexpr size_t kStageBytes = 256 << 10;
+
+struct TableStage {
+  gwl_analysis* a;
+  std::vector<unsigned char> host;
+  std::vector<std::pair<void**, size_t>> where;
+
+  template <class T>
+  int add(T** dst, const std::vector<T>& src) {
+    const size_t bytes = src.size() * sizeof(T);
+    if (bytes > kStageBytes) return upload(a, dst, src);
+    const size_t at = (host.size() + 255) / 256 * 256;
+    host.resize(at + std::max<size_t>(bytes, 1));
+    if (bytes) std::memcpy(host.data() + at, src.data(), bytes);
+    where.emplace_back(reinterpret_cast<void**>(dst), at);
+    return GWL_OK;
+  }
+
+  int flush() {
+    if (where.empty()) return GWL_OK;
+    unsigned char* base = nullptr;
+    int rc = dev_alloc(a, &base, host.size());
+    if (rc) return rc;
+    GWL_CUDA(cudaMemcpy(base, host.data(), host.size(), cudaMemcpyHostToDevice));
+    for (auto& w : where) *w.first = base + w.second;
+    return GWL_OK;
+  }
+};
+
 void free_workspace(gwl_analysis* a) {
   cudaFree(a->d_params);
   cudaFree(a->d_out);
@@ -323,67 +374,80 @@ void basis_taylor(double f, double df, double T[kAnchorOrders][kNumBasis]) {
   }
 }
 
-// The basis functions at frequency f (wide_lnref subtracted from ln f) as
-// float64 pairs hi + lo; lo = 0 for the last four, whose coefficients stay
-// within tens of cycles.
-void wide_basis(double f, double lnref, double* hi, double* lo) {
-  const double y = std::cbrt(f), p = y * y, pe = std::fma(y, y, -p), t = p * y, te = std::fma(p, y, -t) + pe * y;
-  const double yl = ((f - t) - te) / (3.0 * p);
-  const double h3 = 1.0 / y, l3 = (std::fma(-h3, y, 1.0) - h3 * yl) * h3;
-  const double h2 = h3 * h3, l2 = std::fma(h3, h3, -h2) + 2.0 * h3 * l3;
-  const double h1 = 1.0 / f, l1 = std::fma(-h1, f, 1.0) * h1;
-  hi[0] = h1 * h2;
-  lo[0] = std::fma(h1, h2, -hi[0]) + (h1 * l2 + l1 * h2);
-  hi[1] = h1;
-  lo[1] = l1;
-  hi[2] = h2;
-  lo[2] = l2;
-  hi[3] = h3;
-  lo[3] = l3;
-  const double ln = std::log(f) - lnref;
-  hi[4] = ln > 0 ? ln : 0.0;
-  hi[5] = y;
-  hi[6] = y * hi[4];
-  hi[7] = p;
-  for (int b = 4; b < kNumBasis; ++b) lo[b] = 0.0;
-}
-
 // hi + lo in [0, 1) as 0.64 fixed point
 uint64_t wide_fraction(double hi, double lo) {
   return (uint64_t)std::ldexp(hi, 64) + (uint64_t)(int64_t)std::llrint(std::ldexp(lo, 64));
 }
 
-// LaunchArgs::wide_phi over the increasing positive frequencies f[k0 .. n)
-// (zero elsewhere), scaled by powers of two above each function's largest
-// value there.
-void wide_table(const double* f, int64_t k0, int64_t n, int64_t pad, std::vector<uint4>* out, double* scale,
-                double* lnref) {
-  out->assign((size_t)pad * (kNumBasis / 2), make_uint4(0u, 0u, 0u, 0u));
+// The scaling of LaunchArgs::wide_phi over positive frequencies between lo and hi:
+// powers of two above each function's largest value, ln lo.
+void wide_scaling(double lo, double hi, double* scale, double* lnref) {
   for (int b = 0; b < kNumBasis; ++b) scale[b] = 1.0;
-  while (k0 < n && !(f[k0] > 0)) ++k0;
-  if (k0 >= n) return;
-  *lnref = std::log(f[k0]);
-  double top[kNumBasis], end[kNumBasis], lo[kNumBasis];
-  wide_basis(f[k0], *lnref, top, lo);
-  wide_basis(f[n - 1], *lnref, end, lo);
-  double inv[kNumBasis];
+  *lnref = 0.0;
+  if (!(lo > 0 && hi >= lo && std::isfinite(hi))) return;
+  *lnref = std::log(lo);
+  double x[kNumBasis], y[kNumBasis], e[kNumBasis];
+  wide_basis(lo, *lnref, x, e);
+  wide_basis(hi, *lnref, y, e);
   for (int b = 0; b < kNumBasis; ++b) {
-    int e = 0;
-    std::frexp(std::max({top[b], end[b], 1e-300}) * (1.0 + 1e-9), &e);
-    scale[b] = std::ldexp(1.0, e);
-    inv[b] = std::ldexp(1.0, -e);
+    int n = 0;
+    std::frexp(std::max({x[b], y[b], 1e-300}) * (1.0 + 1e-9), &n);
+    scale[b] = std::ldexp(1.0, n);
   }
-  for (int64_t k = k0; k < n; ++k) {
-    double h[kNumBasis], l[kNumBasis];
-    wide_basis(f[k], *lnref, h, l);
-    uint64_t v[kNumBasis];  // rounded to 58 bits (below 1: the scale leaves a margin of 1e-9)
-    for (int b = 0; b < kNumBasis; ++b) v[b] = (wide_fraction(h[b] * inv[b], l[b] * inv[b]) + 32) >> 6;
-    for (int b = 0; b < kNumBasis / 2; ++b) {
-      const uint64_t x = v[2 * b], y = v[2 * b + 1];
-      (*out)[(size_t)k * (kNumBasis / 2) + b] =
-          make_uint4((uint32_t)(x & 0x7ffffff), (uint32_t)(x >> 27), (uint32_t)(y & 0x7ffffff), (uint32_t)(y >> 27));
+}
+
+// |w| (float pair) and arg(w) (0.64 cycles) of point k into LaunchArgs::wide_w
+void wide_weight(std::vector<uint4>* out, int64_t k, double x, double y) {
+  const double turn = std::atan2(y, x) / (2.0 * M_PI);
+  const float2 m = split_ff(std::hypot(x, y));
+  const uint64_t t = wide_fraction(turn < 0 ? turn + 1.0 : turn, 0.0);
+  uint32_t* pair = reinterpret_cast<uint32_t*>(&(*out)[k & ~(int64_t)1]);
+  std::memcpy(pair + (k & 1), &m.x, 4);
+  std::memcpy(pair + 2 + (k & 1), &m.y, 4);
+  pair[4 + 2 * (k & 1)] = (uint32_t)t;
+  pair[5 + 2 * (k & 1)] = (uint32_t)(t >> 32);
+}
+
+// 2^(-i / kExpTable) as 0.64 fixed-point fractions: Taylor's series of
+// e^(-i ln 2 / kExpTable) in float64 pairs.
+const std::vector<uint64_t>& wide_exp_table() {
+  static const std::vector<uint64_t> table = [] {
+    std::vector<uint64_t> t(kExpTable);
+    const double lh = 0.0027076061740622863, ll = 9.058776616587108e-20;  // ln 2 / 256
+    static_assert(kExpTable == 256, "the constant above");
+    for (int i = 0; i < kExpTable; ++i) {
+      const double xh = -i * lh, xl = std::fma(-(double)i, lh, -xh) - i * ll;
+      double th = 1.0, tl = 0.0, sh = 1.0, sl = 0.0;
+      for (int n = 1; n < 26; ++n) {
+        const double p = th * xh, e = std::fma(th, xh, -p) + (th * xl + tl * xh);  // term *= x / n
+        const double q = (p + e) / n;
+        tl = (std::fma(-q, (double)n, p) + e) / n;
+        th = q;
+        const double s = sh + th, b = s - sh;
+        sl += (sh - (s - b)) + (th - b) + tl;
+        sh = s;
+      }
+      t[i] = i == 0 ? ~0ull : wide_fraction(sh, sl);
     }
-  }
+    return t;
+  }();
+  return table;
+}
+
+// LaunchArgs::wide_tab
+const std::vector<float4>& wide_cos_table() {
+  static const std::vector<float4> table = [] {
+    std::vector<float4> wt(kWideTable);
+    for (int q = 0; q < kWideTable; ++q) {
+      const double x = 2.0 * M_PI * q / kWideTable;
+      const double c = q % (kWideTable / 4) == 0 ? std::round(std::cos(x)) : std::cos(x);
+      const double t = -2.0 * M_PI / kWideTable * (q % (kWideTable / 4) == 0 ? std::round(std::sin(x)) : std::sin(x));
+      const float2 cf = split_ff(c), tf = split_ff(t);
+      wt[q] = make_float4(cf.x, cf.y, tf.x, tf.y);
+    }
+    return wt;
+  }();
+  return table;
 }
 
 int g_sm_count = 0;
@@ -448,9 +512,18 @@ LaunchArgs make_args(gwl_analysis* a, int64_t B, int precision) {
   L.ftab = a->ftab;
   L.wide_phi = a->wide_phi;
   L.wide_tab = a->wide_tab;
-  for (int d = 0; d < a->n_det; ++d) L.wide_w[d] = a->wide_w[d];
+  for (int d = 0; d < a->n_det; ++d) {
+    L.wide_w[d] = a->wide_w[d];
+    L.wide_v[d] = a->wide_v[d];
+    L.wide_ve[d] = a->wide_ve[d];
+  }
+  L.wide_exp = a->wide_exp;
   for (int b = 0; b < kNumBasis; ++b) L.wide_scale[b] = a->wide_scale[b];
   L.wide_lnref = a->wide_lnref;
+  L.wide_base = a->k_base;
+  L.wide_chunks = a->n_chunks_plain;
+  L.wide_norm = 4.0 / a->duration;
+  for (int d = 0; d < a->n_det; ++d) L.wide_wscale[d] = a->wide_wscale[d];
   L.step_lo = a->step_lo;
   L.anchors = a->anchors;
   L.n_anchors = a->n_anchors;
@@ -571,8 +644,8 @@ LaunchArgs make_args(gwl_analysis* a, int64_t B, int precision) {
 }
 
 int ensure_workspace(gwl_analysis* a, int64_t B, const LaunchArgs& L) {
-  const size_t part = (size_t)std::max(a->n_chunks_plain, a->n_chunks_mixed) * B * a->n_det * kPartStride *
-                      sizeof(double);
+  const size_t part = (size_t)std::max({a->n_chunks_plain, a->n_chunks_mixed, a->mbw_chunks}) * B * a->n_det *
+                      kPartStride * sizeof(double);
   size_t tm = 0;
   if (a->time_marg && !a->roq) {  // ROQ marginalises without an FFT
     // the float64 kernel over the whole FFT keeps one transform per resident
@@ -817,6 +890,35 @@ int run_mb_fft(gwl_analysis* a, LaunchArgs& L, cudaStream_t s) {
   return GWL_OK;
 }
 
+// A launch of the float64 kernels on the 32-bit pipes: the real part suffices
+// unless |<d|h>| is needed, and the prologue fills the points' coefficients.
+int prepare_wide(gwl_analysis* a, LaunchArgs& L, cudaStream_t s) {
+  L.cplx = a->phase_marg;
+  if (L.B > a->wide_B) {
+    GWL_CUDA(cudaStreamSynchronize(s));
+    cudaFree(a->d_wide);
+    a->d_wide = nullptr;
+    a->wide_B = 0;
+    int rc = dev_alloc(a, &a->d_wide, (size_t)kWideWords * a->ws_B, false);
+    if (rc) return rc;
+    a->wide_B = a->ws_B;
+  }
+  L.wide_c = a->d_wide;
+  return GWL_OK;
+}
+
+// ... larger batches ordered so that a warp's points visit nearly the same bins
+// (LaunchArgs::order; launch_order follows the prologue)
+cudaError_t order_wide(gwl_analysis* a, LaunchArgs& L, cudaStream_t s) {
+  if (L.B < kWideOrderPoints) return cudaSuccess;
+  L.order = a->d_order;
+  L.order_hist = a->d_order_hist;
+  ordering_with_marks(L);
+  if (a->model == GWL_MODEL_SINEGAUSSIAN) L.order_keys = kOrderMaxKeys;  // 16 x 256 buckets (order_key)
+  L.rf_count = nullptr;
+  return cudaMemsetAsync(L.order_hist, 0, sizeof(int32_t) * (2 * L.order_keys + 1), s);
+}
+
 int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, double* d_out, double* d_dh,
              double* d_hh, cudaStream_t s, double* d_series = nullptr) {
   if (precision != GWL_PRECISION_FP64 && precision != GWL_PRECISION_MIXED) {
@@ -913,10 +1015,50 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
     // per point over the bin edges, banded frequencies or nodes (no marking
     // for the accurate kernel: it serves the full-grid TaylorF2 kernels)
     L.rf_tol = 0.0;
+    const bool mbw = a->multiband && a->mb_wide && precision == GWL_PRECISION_FP64;
+    if (mbw) {
+      if ((rc = prepare_wide(a, L, s))) return rc;
+      if (d_dh) L.cplx = 1;
+      L.wide_phi = a->mbw_phi;
+      for (int d = 0; d < a->n_det; ++d) {
+        L.wide_w[d] = a->mbw_w[d];
+        L.wide_wscale[d] = a->mbw_wscale[d];
+        L.wide_q[d] = a->mbw_q[d];
+      }
+      for (int b = 0; b < kNumBasis; ++b) L.wide_scale[b] = a->mbw_scale[b];
+      L.wide_lnref = a->mbw_lnref;
+      L.wide_base = 0;
+      L.wide_chunks = a->mbw_chunks;
+      L.wide_norm = 1.0;
+      L.wide_sub = a->mbw_sub;
+      L.wide_band = a->mbw_band;
+      L.wide_bands = a->mbw_bands;
+      GWL_CUDA(order_wide(a, L, s));
+    }
+    const bool rbw = a->relbin && a->rb_wide;
+    if (rbw) {
+      // (float64 results for either precision)
+      if ((rc = prepare_wide(a, L, s))) return rc;
+      if (d_dh) L.cplx = 1;
+      L.wide_phi = a->rbw_phi;
+      for (int d = 0; d < a->n_det; ++d) {
+        L.wide_w[d] = a->rbw_w[d];
+        L.wide_wscale[d] = a->rbw_wscale[d];
+        L.wide_q[d] = a->rbw_q[d];
+        L.rbw_scale[d] = a->rbw_mscale[d];
+      }
+      for (int b = 0; b < kNumBasis; ++b) L.wide_scale[b] = a->rbw_scale[b];
+      L.wide_lnref = a->rbw_lnref;
+    }
     GWL_CUDA(launch_prologue(L, s));
+    if (mbw && L.order) GWL_CUDA(launch_order(L, s));
     if (a->profiling) GWL_CUDA(cudaEventRecord(a->ev_begin, s));
     if (a->multiband && a->mb_fft && (rc = run_mb_fft(a, L, s))) return rc;
-    if (a->relbin) {
+    if (mbw) {
+      GWL_CUDA(launch_wide(L, s));
+    } else if (rbw) {
+      GWL_CUDA(launch_wide_relbin(L, s));
+    } else if (a->relbin) {
       GWL_CUDA(launch_relbin(L, s));
     } else if (a->multiband) {
       if (precision == GWL_PRECISION_MIXED && a->model == GWL_MODEL_TAYLORF2) {
@@ -947,19 +1089,8 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
     }
     return GWL_OK;
   }
-  const bool wide = precision == GWL_PRECISION_FP64 && a->model == GWL_MODEL_TAYLORF2 && !(a->time_marg && d_out);
-  if (wide) {
-    L.cplx = a->phase_marg;  // the real part suffices unless |<d|h>| is needed
-    if (B > a->wide_B) {
-      GWL_CUDA(cudaStreamSynchronize(s));
-      cudaFree(a->d_wide);
-      a->d_wide = nullptr;
-      a->wide_B = 0;
-      if ((rc = dev_alloc(a, &a->d_wide, (size_t)kWideWords * a->ws_B, false))) return rc;
-      a->wide_B = a->ws_B;
-    }
-    L.wide_c = a->d_wide;
-  }
+  const bool wide = precision == GWL_PRECISION_FP64 && !(a->time_marg && d_out);
+  if (wide && (rc = prepare_wide(a, L, s))) return rc;
   if (d_dh) L.cplx = 1;  // complex <d|h> requested
   const bool ordered = precision == GWL_PRECISION_MIXED && a->model == GWL_MODEL_TAYLORF2 && !(a->time_marg && d_out);
   if (ordered) {
@@ -970,14 +1101,9 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
     ordering_with_marks(L);
     a->last_rf_count = L.rf_count;
     GWL_CUDA(cudaMemsetAsync(L.order_hist, 0, sizeof(int32_t) * (2 * L.order_keys + 1), s));
-  } else if (wide && B >= kWideOrderPoints) {
-    // a warp's points stop at nearly the same bin (LaunchArgs::order)
+  } else if (wide) {
     L.rf_tol = 0.0;
-    L.order = a->d_order;
-    L.order_hist = a->d_order_hist;
-    ordering_with_marks(L);
-    L.rf_count = nullptr;
-    GWL_CUDA(cudaMemsetAsync(L.order_hist, 0, sizeof(int32_t) * (2 * L.order_keys + 1), s));
+    GWL_CUDA(order_wide(a, L, s));
   } else if (precision == GWL_PRECISION_MIXED && a->model == GWL_MODEL_SINEGAUSSIAN && !(a->time_marg && d_out)) {
     // sine-Gaussian: points ordered by centre frequency; the finalize marks
     // the points whose error bound exceeds the tolerance and counts them
@@ -1029,9 +1155,7 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
     GWL_CUDA(launch_mixed_acc(L, a->side.stream));
   }
   if (wide) {
-    GWL_CUDA(launch_wide(L, s));
-  } else if (precision == GWL_PRECISION_FP64) {
-    GWL_CUDA(launch_plain(L, s));
+    GWL_CUDA(a->model == GWL_MODEL_SINEGAUSSIAN ? launch_wide_sg(L, s) : launch_wide(L, s));
   } else {
     GWL_CUDA(launch_mixed(L, s));
   }
@@ -1127,6 +1251,33 @@ const char* gwl_last_error(void) { return t_last_error.c_str(); }
 
 const char* gwl_version(void) { return "bilby_gb300 gwlnl 0.1 (sm_103a)"; }
 
+namespace {
+// The float64 kernels' full-grid tables, on the device from the strain, the
+// inverse PSD and the powers of f: one allocation for all of them.
+int build_wide_tables(gwl_analysis* a) {
+  const int64_t P = a->n_pad;
+  const bool tf2 = a->model == GWL_MODEL_TAYLORF2;
+  uint4* base = nullptr;
+  int rc = dev_alloc(a, &base, (size_t)P * (a->n_det + (tf2 ? kNumBasis / 2 : 0)));
+  if (rc) return rc;
+  for (int d = 0; d < a->n_det; ++d) {
+    a->wide_w[d] = base + (size_t)d * P;
+    a->wide_wscale[d] = a->w_scale[d];
+    GWL_CUDA(launch_wide_weights(reinterpret_cast<const double2*>(a->strain[d]), a->inv_psd[d],
+                                 tf2 ? a->ftab : nullptr, 1.0 / a->w_scale[d], P, a->wide_w[d], a->stream));
+  }
+  if (tf2) {
+    int64_t k0 = a->k_fmin;
+    while (k0 < a->n_bins && !(a->h_freq[(size_t)k0] > 0)) ++k0;
+    if (k0 < a->n_bins) wide_scaling(a->h_freq[(size_t)k0], a->h_freq.back(), a->wide_scale, &a->wide_lnref);
+    a->wide_phi = base + (size_t)a->n_det * P;
+    GWL_CUDA(launch_wide_basis(a->freq, k0, a->n_bins, P, a->wide_lnref, a->wide_scale, a->wide_phi, a->stream));
+  }
+  GWL_CUDA(cudaStreamSynchronize(a->stream));
+  return GWL_OK;
+}
+}  // namespace
+
 int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
   if (!desc || !out) {
     set_error("null argument");
@@ -1201,6 +1352,7 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
     }
   const int64_t P = a->n_pad;
   int rc = GWL_OK;
+  TableStage stage{a, {}, {}};
   cudaError_t ce = cudaStreamCreateWithFlags(&a->stream, cudaStreamNonBlocking);
   if (ce == cudaSuccess) ce = side_stream_create(&a->side);
   if (ce != cudaSuccess) {
@@ -1222,9 +1374,15 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
       hf[k] = f[k];
       hff[k] = (float)f[k];
     }
-    if ((rc = upload(a, &a->freq, hf))) goto fail;
+    if ((rc = stage.add(&a->freq, hf))) goto fail;
     a->h_freq.assign(f, f + N);
-    if (a->model == GWL_MODEL_SINEGAUSSIAN && (rc = upload(a, &a->freq_f, hff))) goto fail;
+    if (a->model == GWL_MODEL_SINEGAUSSIAN && (rc = stage.add(&a->freq_f, hff))) goto fail;
+    {
+      if ((rc = stage.add(&a->wide_tab, wide_cos_table()))) goto fail;
+    }
+    if (a->model == GWL_MODEL_SINEGAUSSIAN) {
+      if ((rc = stage.add(&a->wide_exp, wide_exp_table()))) goto fail;
+    }
     if (a->model == GWL_MODEL_TAYLORF2) {
       // float-float phase basis: f^-5/3, f^-1, f^-2/3, f^-1/3, ln f, f^1/3, f^1/3 ln f, f^2/3
       std::vector<float2> basis((size_t)P * kNumBasis, make_float2(0.f, 0.f));
@@ -1237,7 +1395,7 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
                                         lx, c3, c3 * lx, c3 * c3};
         for (int b = 0; b < kNumBasis; ++b) basis[(size_t)k * kNumBasis + b] = split_ff(vals[b]);
       }
-      if ((rc = upload(a, &a->basis, basis))) goto fail;
+      if ((rc = stage.add(&a->basis, basis))) goto fail;
       // float64 powers of f for the plain kernel
       std::vector<double4> ft((size_t)P, make_double4(0.0, 0.0, 0.0, 0.0));
       for (int64_t k = 0; k < N; ++k) {
@@ -1245,12 +1403,7 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
         if (!(x > 0)) continue;
         ft[k] = make_double4(std::cbrt(x), std::log(x) / 3.0, std::pow(x, -5.0 / 3.0), std::pow(x, -7.0 / 6.0));
       }
-      if ((rc = upload(a, &a->ftab, ft))) goto fail;
-      {
-        std::vector<uint4> phi;
-        wide_table(f, a->k_fmin, N, P, &phi, a->wide_scale, &a->wide_lnref);
-        if ((rc = upload(a, &a->wide_phi, phi))) goto fail;
-      }
+      if ((rc = stage.add(&a->ftab, ft))) goto fail;
       // Taylor tables of the basis every kAnchorStep bins (f = k * df)
       a->n_anchors = N / kAnchorStep + 2;
       std::vector<float> anc((size_t)a->n_anchors * kAnchorFloats, 0.f);
@@ -1266,7 +1419,7 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
             if (n < kAnchorFF) dst[kAnchorOrders * kNumBasis + n * kNumBasis + b] = v.y;
           }
       }
-      if ((rc = upload(a, &a->anchors, anc))) goto fail;
+      if ((rc = stage.add(&a->anchors, anc))) goto fail;
       // float-float cos and sin of 2 pi q / kCosTable for the accurate kernel
       std::vector<float4> ct(kCosTable);
       for (int q = 0; q < kCosTable; ++q) {
@@ -1274,16 +1427,7 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
         const float ch = (float)c, sh = (float)sn;
         ct[q] = make_float4(ch, (float)(c - (double)ch), sh, (float)(sn - (double)sh));
       }
-      if ((rc = upload(a, &a->cos_tab, ct))) goto fail;
-      std::vector<float4> wt(kWideTable);
-      for (int q = 0; q < kWideTable; ++q) {
-        const double x = 2.0 * M_PI * q / kWideTable;
-        const double c = q % (kWideTable / 4) == 0 ? std::round(std::cos(x)) : std::cos(x);
-        const double t = -2.0 * M_PI / kWideTable * (q % (kWideTable / 4) == 0 ? std::round(std::sin(x)) : std::sin(x));
-        const float2 cf = split_ff(c), tf = split_ff(t);
-        wt[q] = make_float4(cf.x, cf.y, tf.x, tf.y);
-      }
-      if ((rc = upload(a, &a->wide_tab, wt))) goto fail;
+      if ((rc = stage.add(&a->cos_tab, ct))) goto fail;
     }
     a->noise_lnl = 0.0;
     std::vector<double> f76, f73;  // f^(-7/6), f^(-7/3)
@@ -1309,8 +1453,8 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
         dd.add((s[2 * k] * s[2 * k] + s[2 * k + 1] * s[2 * k + 1]) * ip[k]);
       }
       a->noise_lnl -= std::fabs(4.0 / a->duration * dd.value() / 2.0);
-      if ((rc = upload(a, &a->strain[d], s))) goto fail;
-      if ((rc = upload(a, &a->inv_psd[d], ip))) goto fail;
+      if ((rc = stage.add(&a->strain[d], s))) goto fail;
+      if ((rc = stage.add(&a->inv_psd[d], ip))) goto fail;
       // mixed-precision weights, scaled into float32 range
       std::vector<double> wr(P, 0.0), wi(P, 0.0);
       double wmax = 0.0, vmax = 0.0;
@@ -1330,10 +1474,9 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
         wf[k] = make_float2((float)(wr[k] / a->w_scale[d]), (float)(wi[k] / a->w_scale[d]));
         vf[k] = (float)(ip[k] / a->v_scale[d]);
       }
-      if ((rc = upload(a, &a->w[d], wf))) goto fail;
+      if ((rc = stage.add(&a->w[d], wf))) goto fail;
       if (a->model == GWL_MODEL_TAYLORF2) {
         std::vector<uint2> wpol(P, make_uint2(0u, 0u));
-        std::vector<uint4> wide(P, make_uint4(0u, 0u, 0u, 0u));
         for (int64_t k = 0; k < N; ++k) {
           const double x = wr[k] / a->w_scale[d], y = wi[k] / a->w_scale[d];
           // odd bins carry -|w| at arg(w) + 1/2 cycle (the same term): a mean
@@ -1341,13 +1484,6 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
           // instead of adding up coherently with the positive magnitudes
           const bool odd = (k & 1) != 0;
           const double abs_w = std::hypot(x, y), turn = std::atan2(y, x) / (2.0 * M_PI);
-          const float2 wm = split_ff(abs_w);
-          const uint64_t wt = wide_fraction(turn < 0 ? turn + 1.0 : turn, 0.0);
-          uint32_t* pair = reinterpret_cast<uint32_t*>(&wide[k & ~(int64_t)1]);
-          std::memcpy(pair + (k & 1), &wm.x, 4);
-          std::memcpy(pair + 2 + (k & 1), &wm.y, 4);
-          pair[4 + 2 * (k & 1)] = (uint32_t)wt;
-          pair[5 + 2 * (k & 1)] = (uint32_t)(wt >> 32);
           const float mag = (float)(odd ? -abs_w : abs_w);
           double cyc = turn + (odd ? 0.5 : 0.0);
           cyc -= std::floor(cyc);
@@ -1356,8 +1492,7 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
           std::memcpy(&mb, &mag, 4);
           wpol[k] = make_uint2(mb, th);
         }
-        if ((rc = upload(a, &a->wp[d], wpol))) goto fail;
-        if ((rc = upload(a, &a->wide_w[d], wide))) goto fail;
+        if ((rc = stage.add(&a->wp[d], wpol))) goto fail;
         // the fast kernel's pairs: magnitudes side by side, then the angle at
         // the first bin of each 8-bin block and the increment over the
         // previous bin elsewhere (P is a multiple of 16)
@@ -1368,14 +1503,27 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
           const uint32_t tau1 = wpol[k + 1].y - wpol[k].y;
           wpair[q] = make_uint4(wpol[k].x, wpol[k + 1].x, tau0, tau1);
         }
-        if ((rc = upload(a, &a->wq[d], wpair))) goto fail;
+        if ((rc = stage.add(&a->wq[d], wpair))) goto fail;
       }
       if (a->model == GWL_MODEL_SINEGAUSSIAN) {
         // float-float inverse PSD for the float-float <h|h> of the mixed kernel
         std::vector<float> vl(P, 0.f);
         for (int64_t k = 0; k < N; ++k) vl[k] = (float)(ip[k] / a->v_scale[d] - (double)vf[k]);
-        if ((rc = upload(a, &a->v[d], vf))) goto fail;
-        if ((rc = upload(a, &a->v_lo[d], vl))) goto fail;
+        if ((rc = stage.add(&a->v[d], vf))) goto fail;
+        if ((rc = stage.add(&a->v_lo[d], vl))) goto fail;
+        // 64-bit fractions of a power of two per 32 bins for the float64 <h|h>
+        std::vector<uint64_t> wv(P, 0);
+        std::vector<int32_t> we((size_t)(a->n_chunks_plain * kChunkPlain / 32), 0);
+        for (size_t q = 0; q < we.size(); ++q) {
+          const int64_t k0 = a->k_base + (int64_t)q * 32, k1 = std::min(k0 + 32, N);
+          double top = 0.0;
+          for (int64_t k = k0; k < k1; ++k) top = std::max(top, ip[k]);
+          if (!(top > 0)) continue;
+          std::frexp(top, &we[q]);
+          for (int64_t k = k0; k < k1; ++k) wv[k] = (uint64_t)std::ldexp(ip[k], 64 - we[q]);
+        }
+        if ((rc = stage.add(&a->wide_v[d], wv))) goto fail;
+        if ((rc = stage.add(&a->wide_ve[d], we))) goto fail;
       } else {
         // <h|h> prefix sums of f^(-7/3) / S over the analysis grid
         std::vector<double> pre(N + 1, 0.0);
@@ -1384,7 +1532,7 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
           if (ip[k] != 0.0 && f[k] > 0) acc.add(f73[k] * ip[k]);
           pre[k + 1] = acc.value();
         }
-        if ((rc = upload(a, &a->hh_prefix[d], pre))) goto fail;
+        if ((rc = stage.add(&a->hh_prefix[d], pre))) goto fail;
         // refinement bound: prefix sums of the scaled weight magnitudes |w|^2,
         // and of |w| where the whitened data power 4 |d|^2 / (T S) exceeds
         // kRefineLoudPower (bins dominated by a signal, whose phase a template
@@ -1402,11 +1550,13 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
           p2[k + 1] = acc2.value();
           p1[k + 1] = acc1.value();
         }
-        if ((rc = upload(a, &a->rf_p2[d], p2))) goto fail;
-        if ((rc = upload(a, &a->rf_p1[d], p1))) goto fail;
+        if ((rc = stage.add(&a->rf_p2[d], p2))) goto fail;
+        if ((rc = stage.add(&a->rf_p1[d], p1))) goto fail;
       }
     }
   }
+  if ((rc = stage.flush())) goto fail;
+  if ((rc = build_wide_tables(a))) goto fail;
   *out = a;
   return GWL_OK;
 fail:
@@ -1712,6 +1862,84 @@ int gwl_set_distance_marginalization(gwl_analysis* a, int enable, const double* 
   return GWL_OK;
 }
 
+namespace {
+// The tables of gwl_wide_relbin.cu.  Fiducial waveforms that vanish at an edge
+// (1 / h0 not finite) keep the float64 kernel, whose result is then not finite
+// either (rb_wide = 0).
+int build_wide_relbin(gwl_analysis* a, const std::vector<double>& fe, const double* h0_inverse, const double* summary) {
+  a->rb_wide = 0;
+  const size_t n = fe.size(), nb = n - 1;
+  if (a->model != GWL_MODEL_TAYLORF2 || !(fe.front() > 0)) return GWL_OK;
+  for (size_t q = 0; q < (size_t)a->n_det * n * 2; ++q)
+    if (!std::isfinite(h0_inverse[q])) return GWL_OK;
+  wide_scaling(std::max(fe.front(), std::min(fe.back(), a->fmin)), fe.back(), a->rbw_scale, &a->rbw_lnref);
+  std::vector<double> f = fe, amp(n);
+  for (size_t e = 0; e < n; ++e) {
+    if (!(fe[e] >= a->fmin)) f[e] = 0.0;  // below the band: no phase, no weight
+    amp[e] = f[e] > 0 ? std::pow(f[e], -7.0 / 6.0) : 0.0;
+  }
+  int rc;
+  for (int d = 0; d < a->n_det; ++d) {
+    const double* g = h0_inverse + (size_t)d * n * 2;
+    const double* sm = summary + (size_t)d * nb * 6;
+    std::vector<double> x(n), y(n), m(n, 0.0), turn(n, 0.0), q(n + 1, 0.0);
+    double top = 0.0, mtop = 0.0;
+    KahanSum acc;
+    for (size_t e = 0; e < n; ++e) {
+      double wr = 0.0, wi = 0.0, c = 0.0;
+      if (e > 0) {
+        const double* v = sm + (e - 1) * 6;
+        const double width = fe[e] - fe[e - 1];
+        wr += v[0] / 2 + v[2] / width;
+        wi += v[1] / 2 + v[3] / width;
+        c += v[4] / 4 + v[5] / width;
+      }
+      if (e < nb) {
+        const double* v = sm + e * 6;
+        const double width = fe[e + 1] - fe[e];
+        wr += v[0] / 2 - v[2] / width;
+        wi += v[1] / 2 - v[3] / width;
+        c += v[4] / 4 - v[5] / width;
+        // m = b0 / 2 |g_e| |g_{e+1}|; the phase enters with the opposite sign of arg g
+        m[e] = v[4] / 2 * amp[e] * amp[e + 1] * std::hypot(g[2 * e], g[2 * e + 1]) * std::hypot(g[2 * e + 2], g[2 * e + 3]);
+        turn[e] = (std::atan2(g[2 * e + 1], g[2 * e]) - std::atan2(g[2 * e + 3], g[2 * e + 2])) / (2.0 * M_PI);
+        mtop = std::max(mtop, std::fabs(m[e]));
+      }
+      // w = conj(g) (...) f^(-7/6)
+      x[e] = amp[e] * (g[2 * e] * wr + g[2 * e + 1] * wi);
+      y[e] = amp[e] * (g[2 * e] * wi - g[2 * e + 1] * wr);
+      top = std::max(top, std::max(std::fabs(x[e]), std::fabs(y[e])));
+      acc.add(amp[e] * amp[e] * (g[2 * e] * g[2 * e] + g[2 * e + 1] * g[2 * e + 1]) * c);
+      q[e + 1] = acc.value();
+    }
+    a->rbw_wscale[d] = top > 0 && std::isfinite(top) ? top : 1.0;
+    a->rbw_mscale[d] = mtop > 0 && std::isfinite(mtop) ? mtop : 1.0;
+    // per edge the pair {w, m}
+    std::vector<uint4> w(2 * n, make_uint4(0u, 0u, 0u, 0u));
+    for (size_t e = 0; e < n; ++e) {
+      wide_weight(&w, 2 * (int64_t)e, x[e] / a->rbw_wscale[d], y[e] / a->rbw_wscale[d]);
+      const float2 mf = split_ff(m[e] / a->rbw_mscale[d]);
+      double t = turn[e] - std::floor(turn[e]);
+      if (!(t >= 0 && t < 1)) t = 0.0;
+      const uint64_t u = wide_fraction(t, 0.0);
+      std::memcpy(&w[2 * e].y, &mf.x, 4);
+      std::memcpy(&w[2 * e].w, &mf.y, 4);
+      w[2 * e + 1].z = (uint32_t)u;
+      w[2 * e + 1].w = (uint32_t)(u >> 32);
+    }
+    if ((rc = upload(a, &a->rbw_w[d], w))) return rc;
+    if ((rc = upload(a, &a->rbw_q[d], q))) return rc;
+  }
+  double* fd = nullptr;
+  if ((rc = upload(a, &fd, f))) return rc;
+  if ((rc = dev_alloc(a, &a->rbw_phi, n * (kNumBasis / 2)))) return rc;
+  GWL_CUDA(launch_wide_basis(fd, 0, (int64_t)n, (int64_t)n, a->rbw_lnref, a->rbw_scale, a->rbw_phi, a->stream));
+  GWL_CUDA(cudaStreamSynchronize(a->stream));
+  a->rb_wide = 1;
+  return GWL_OK;
+}
+}  // namespace
+
 int gwl_set_relative_binning(gwl_analysis* a, int enable, int32_t n_edges, const int64_t* edge_index,
                              const double* h0_inverse, const double* summary) {
   if (!a) {
@@ -1755,6 +1983,7 @@ int gwl_set_relative_binning(gwl_analysis* a, int enable, int32_t n_edges, const
   a->rb_edges = n_edges;
   a->h_rb_index = idx;
   a->rb_tm = 0;  // new bins need new time-marginalisation weights
+  if ((rc = build_wide_relbin(a, fe, h0_inverse, summary))) return rc;
   a->relbin = 1;
   return GWL_OK;
 }
@@ -1799,6 +2028,88 @@ int gwl_set_relative_binning_time_weights(gwl_analysis* a, const double* weights
   a->rb_tm = 1;
   return GWL_OK;
 }
+
+namespace {
+// The tables of float64 TaylorF2 multi-banding on the kernels of gwl_wide.cu:
+// the banded points band after band, each band padded to whole sub-blocks of 32.
+// They take frequencies on the analysis grid (each band's first point at grid
+// index I, its points r indices apart), as bands of 1 / T^(b) with T / T^(b) a
+// whole number are; other lists keep the float64 kernel (mb_wide = 0).
+int build_wide_bands(gwl_analysis* a, const std::vector<double>& fr, const std::vector<int64_t>& bs,
+                     const double* linear, const double* quadratic) {
+  a->mb_wide = 0;
+  if (a->model != GWL_MODEL_TAYLORF2) return GWL_OK;
+  const int64_t n = (int64_t)fr.size();
+  std::vector<int4> band;
+  std::vector<int2> sub;
+  std::vector<int64_t> at((size_t)n, -1);  // padded position of each point
+  double lo = 0.0, hi = 0.0;
+  for (size_t b = 0; b + 1 < bs.size(); ++b) {
+    const int64_t m = bs[b + 1] - bs[b];
+    if (m < 1) continue;
+    const double* f = fr.data() + bs[b];
+    const int64_t I = std::llround(f[0] / a->step);
+    const int64_t r = m > 1 ? std::llround((f[m - 1] - f[0]) / a->step / (double)(m - 1)) : 1;
+    if (I < 0 || r < 1 || I + (m - 1) * r > INT32_MAX) return GWL_OK;
+    for (int64_t k = 0; k < m; ++k) {
+      const double g = (double)(I + k * r) * a->step;
+      if (!(std::fabs(f[k] - g) <= 4e-16 * std::fabs(g))) return GWL_OK;
+      if (f[k] > 0) {
+        lo = lo > 0 ? std::min(lo, f[k]) : f[k];
+        hi = std::max(hi, f[k]);
+      }
+    }
+    const int64_t p0 = (int64_t)sub.size() * 32;
+    band.push_back(make_int4((int)p0, (int)m, (int)I, (int)r));
+    for (int64_t k = 0; k < m; ++k) at[(size_t)(bs[b] + k)] = p0 + k;
+    for (int64_t k = 0; k < m; k += 32) sub.push_back(make_int2((int)(I + k * r), (int)r));
+  }
+  if (band.empty() || !(lo > 0)) return GWL_OK;
+  lo = std::max(lo, std::min(hi, a->fmin));  // points below the minimum frequency carry no weight
+  wide_scaling(lo, hi, a->mbw_scale, &a->mbw_lnref);
+  const int64_t chunks = ((int64_t)sub.size() * 32 + kChunkPlain - 1) / kChunkPlain, P = chunks * kChunkPlain;
+  sub.resize((size_t)(P / 32), make_int2(INT32_MAX, 1));  // (beyond every band end)
+  std::vector<double> fp((size_t)P, 0.0);
+  for (int64_t k = 0; k < n; ++k)
+    if (at[(size_t)k] >= 0 && fr[(size_t)k] >= lo) fp[(size_t)at[(size_t)k]] = fr[(size_t)k];
+  int rc;
+  for (int d = 0; d < a->n_det; ++d) {
+    std::vector<double> x((size_t)P, 0.0), y((size_t)P, 0.0), q((size_t)P + 1, 0.0);
+    double top = 0.0;
+    for (int64_t k = 0; k < n; ++k) {
+      const int64_t p = at[(size_t)k];
+      if (p < 0 || !(fr[(size_t)k] > 0) || !(fr[(size_t)k] >= a->fmin)) continue;
+      const double w = std::pow(fr[(size_t)k], -7.0 / 6.0);
+      // conj(s) conj(L): the weight of e^{+i phase} is the conjugate coefficient
+      x[(size_t)p] = linear[((size_t)d * n + k) * 2] * w;
+      y[(size_t)p] = -linear[((size_t)d * n + k) * 2 + 1] * w;
+      top = std::max(top, std::max(std::fabs(x[(size_t)p]), std::fabs(y[(size_t)p])));
+      q[(size_t)p + 1] = w * w * quadratic[(size_t)d * n + k];
+    }
+    a->mbw_wscale[d] = top > 0 ? top : 1.0;
+    std::vector<uint4> w((size_t)P, make_uint4(0u, 0u, 0u, 0u));
+    KahanSum acc;
+    for (int64_t p = 0; p < P; ++p) {
+      wide_weight(&w, p, x[(size_t)p] / a->mbw_wscale[d], y[(size_t)p] / a->mbw_wscale[d]);
+      acc.add(q[(size_t)p + 1]);
+      q[(size_t)p + 1] = acc.value();
+    }
+    if ((rc = upload(a, &a->mbw_w[d], w))) return rc;
+    if ((rc = upload(a, &a->mbw_q[d], q))) return rc;
+  }
+  double* f = nullptr;
+  if ((rc = upload(a, &f, fp))) return rc;
+  if ((rc = dev_alloc(a, &a->mbw_phi, (size_t)P * (kNumBasis / 2)))) return rc;
+  GWL_CUDA(launch_wide_basis(f, 0, P, P, a->mbw_lnref, a->mbw_scale, a->mbw_phi, a->stream));
+  GWL_CUDA(cudaStreamSynchronize(a->stream));
+  if ((rc = upload(a, &a->mbw_sub, sub))) return rc;
+  if ((rc = upload(a, &a->mbw_band, band))) return rc;
+  a->mbw_bands = (int)band.size();
+  a->mbw_chunks = chunks;
+  a->mb_wide = 1;
+  return GWL_OK;
+}
+}  // namespace
 
 int gwl_set_multiband(gwl_analysis* a, int enable, int64_t n_points, const double* frequencies,
                       const double* linear, const double* quadratic, int32_t n_bands, const int64_t* band_start,
@@ -1903,6 +2214,7 @@ int gwl_set_multiband(gwl_analysis* a, int enable, int64_t n_points, const doubl
   a->mb_bands = n_bands;
   a->mb_points = n_points;
   a->mb_tm = 0;  // new bands need new time-marginalisation tables
+  if ((rc = build_wide_bands(a, fr, bs, linear, quadratic))) return rc;
   a->multiband = 1;
   return GWL_OK;
 }

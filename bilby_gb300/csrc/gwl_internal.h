@@ -43,7 +43,8 @@ constexpr double kRefineDefaultTol = 5e-4;
 constexpr int kCosTable = 1024;        // angles of the float-float cos / sin table of the accurate kernel
 constexpr int kWideOrderPoints = 64;   // ... and from this size on, ordered by band end
 constexpr int kWideFewPoints = 24;     // float64 TaylorF2 batches up to this size run one CTA per (chunk, point)
-constexpr int kWideWords = kNumBasis + 2 + 2 * kMaxDet;  // words per point of LaunchArgs::wide_c
+constexpr int kWideEnd = kNumBasis + 2 + 2 * kMaxDet, kWideWords = kWideEnd + 1;  // words per point of LaunchArgs::wide_c
+constexpr int kExpTable = 256;         // entries 2^(-i / 256) of gwl_wide_sg.cu
 constexpr int kWideTable = 2048;       // angles of the float-float cosine table of gwl_wide.cuh
 constexpr int kRoqSplits = 8;          // node groups of the mixed ROQ time-marginalised matrix products
 
@@ -118,14 +119,32 @@ struct LaunchArgs {
   // in fixed point and float-float, and per point the phase coefficients
   const uint4* wide_phi;                // [n_pad][kNumBasis / 2] two basis functions / wide_scale each, 0.58 fixed
                                         // point {low 27 bits, high 31 bits}
+  double wide_wscale[kMaxDet];          // scale of wide_w
+  double wide_norm;                     // factor of the sums: 4 / T, or 1 where the weights carry it
+  int64_t wide_base, wide_chunks;       // first row of the tables and chunks of kChunkPlain rows from it on
+  // rows that are not consecutive bins (multi-banding): per 32 rows the grid
+  // index of the first and the stride; the bands {first row, rows, grid index,
+  // stride}; prefix sums of f^(-7/3) times the quadratic coefficients.  nullptr:
+  // row k is bin k
+  const int2* wide_sub;
+  const int4* wide_band;
+  int wide_bands;
+  const double* wide_q[kMaxDet];
+  double rbw_scale[kMaxDet];            // relative binning: scale of the cross terms' weights (gwl_wide_relbin.cu)
   const float4* wide_tab;               // [kWideTable] {cos hi, lo, -2 pi / kWideTable sin hi, lo}
   const uint4* wide_w[kMaxDet];         // [n_pad] per bin pair {|w| / w_scale of both, hi words then lo (floats)},
                                         // {arg(w) of both, 0.64 cycles {lo, hi} each}
+  const uint64_t* wide_v[kMaxDet];      // sine-Gaussian: [n_pad] mask / S, 0.64 fixed point of 2^wide_ve
+  const int32_t* wide_ve[kMaxDet];      // ... [n_chunks * kChunkPlain / 32] its exponent per 32 bins from k_base on
+  const uint64_t* wide_exp;             // sine-Gaussian: [kExpTable] 2^(-i / kExpTable), 0.64 fixed point
   double wide_scale[kNumBasis];         // powers of two above each basis function's largest value
   double wide_lnref;                    // ln f of the basis functions is ln f - wide_lnref
   double step_lo;                       // step + step_lo: the grid spacing to twice float64's digits
   uint64_t* wide_c;                     // [kWideWords][B]: c_b wide_scale_b 2^(58 - s), the constant, s + 2, per
-                                        // detector the shift per bin and the offset (cycles, 64-bit fractions)
+                                        // detector the shift per bin and the offset (cycles, 64-bit fractions),
+                                        // the grid index of f_ISCO, the grid continued;
+                                        // sine-Gaussian: f0 in bins, sqrt(y) per bin, its shift with the fractional
+                                        // bits of f0, the largest distance, per detector as above with beta
   const float* anchors;                 // [n_anchors][kAnchorFloats] Taylor tables of the basis
   int64_t n_anchors;
   const double* params;                 // [GWL_NPARAM][B]
@@ -320,9 +339,19 @@ constexpr int kMultiCounters = 2 * kMultiClasses + 1;  // unit counters (fast, a
 cudaError_t launch_multi(const MultiArgs& m, const int* ctas, const int* ctas_acc, cudaStream_t s, SideStream* side);
 int multi_tf2_ctas_per_sm(int q, bool acc);
 cudaError_t launch_prologue(const LaunchArgs& a, cudaStream_t s);
-cudaError_t launch_plain(const LaunchArgs& a, cudaStream_t s);
-// The float64 TaylorF2 likelihood (gwl_wide.cu): partial sums, totals and lnL.
+// The float64 likelihood (gwl_wide.cu, gwl_wide_sg.cu): partial sums, totals and lnL.
 cudaError_t launch_wide(const LaunchArgs& a, cudaStream_t s);
+cudaError_t launch_wide_sg(const LaunchArgs& a, cudaStream_t s);
+// Relative binning: rows are the bin edges, pairs of wide_w {|w|, m} and {arg w,
+// arg of the neighbours' ratio}, wide_q prefix sums over the edges.
+cudaError_t launch_wide_relbin(const LaunchArgs& a, cudaStream_t s);
+// Their tables: the basis functions of rows [k0, n) of f (zero where f <= 0 and
+// outside), the weights z u f^(-7/6) inv_scale of n (even) rows (powers of f from
+// ftab, none without it).
+cudaError_t launch_wide_basis(const double* f, int64_t k0, int64_t n, int64_t pad, double lnref, const double* scale,
+                              uint4* out, cudaStream_t s);
+cudaError_t launch_wide_weights(const double2* z, const double* u, const double4* ftab, double inv_scale, int64_t n,
+                                uint4* out, cudaStream_t s);
 cudaError_t launch_mixed(const LaunchArgs& a, cudaStream_t s);
 // The accurate kernel for the marked points (nothing when rf_tol <= 0).
 cudaError_t launch_mixed_acc(const LaunchArgs& a, cudaStream_t s);

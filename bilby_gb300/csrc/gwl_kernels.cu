@@ -34,6 +34,14 @@ __device__ __forceinline__ int order_key(const LaunchArgs& a, const PointRec& r)
     // sine-Gaussian: the bin of the centre frequency, so that the points of a
     // warp walk their Gaussians (k_mixed_sg) over runs of nearly equal length
     if (!r.valid) return 0;
+    if (a.wide_c) {
+      // float64 (gwl_wide_sg.cu): the bins visited, by half octaves of their
+      // number, then by their middle
+      const int n = (int)(a.k_hi - a.k_lo), w = (int)max(r.k_end - r.k_start, (int64_t)1);
+      const int c = min(max((int)(2.f * __log2f((float)n / (float)w)), 0), 15);
+      const int m = (int)(256.f * (float)((r.k_start + r.k_end) / 2 - a.k_lo) / (float)(n + 1));
+      return c * 256 + min(max(m, 0), 255);
+    }
     const double kp = floor((r.sg_f0 - a.freq[a.k_base]) / a.step);
     const double n = (double)(a.n_chunks * a.chunk);
     return (int)((int64_t)fmin(fmax(kp, 0.0), n) >> a.order_shift);
@@ -52,6 +60,12 @@ __device__ __forceinline__ uint64_t to_wide(double x, double lo) {
   double fr = ldexp(x - floor(x), 64);
   if (!(fr >= 0.0 && fr < 18446744073709551616.0)) fr = 0.0;
   return (uint64_t)fr + (uint64_t)(int64_t)ldexp(lo, 64);
+}
+
+// frac(dt df) in cycles per bin
+__device__ __forceinline__ uint64_t wide_shift(const LaunchArgs& a, double dt) {
+  const double v = dt * a.step;
+  return to_wide(v, fma(dt, a.step, -v) + dt * a.step_lo);
 }
 
 __device__ __noinline__ void wide_coefficients(const LaunchArgs& a, const PointRec& r, int64_t i, double m1, double m2,
@@ -95,9 +109,50 @@ __device__ __noinline__ void wide_coefficients(const LaunchArgs& a, const PointR
   w[(int64_t)kNumBasis * a.B] = to_wide(cconst + c[4] * a.wide_lnref, 0.0);
   w[(int64_t)(kNumBasis + 1) * a.B] = (uint64_t)(s + 2);
   for (int d = 0; d < a.n_det; ++d) {
-    const double v = r.dt[d] * a.step, e = fma(r.dt[d], a.step, -v) + r.dt[d] * a.step_lo;
-    w[(int64_t)(kNumBasis + 2 + d) * a.B] = to_wide(v, e);
+    w[(int64_t)(kNumBasis + 2 + d) * a.B] = wide_shift(a, r.dt[d]);
     w[(int64_t)(kNumBasis + 2 + kMaxDet + d) * a.B] = ((uint64_t)r.qfix[d][1] << 32) | r.qfix[d][0];
+  }
+  // a list's frequencies may lie beyond the grid's last
+  int64_t ke = r.k_end;
+  if (ke >= a.n_bins) ke = max(ke, (int64_t)fmin(ceil(r.f_isco / a.step), 9e15));
+  w[(int64_t)kWideEnd * a.B] = (uint64_t)ke;
+}
+
+// ... and of gwl_wide_sg.cu: the centre frequency in bins, sqrt(y) = Q sqrt(log2 e
+// / 2) / f0 per bin to twice float64's digits, the bins to visit, the shifts and
+// arg(Fp P + i Fx X).
+__device__ __noinline__ void wide_coefficients_sg(const LaunchArgs& a, PointRec& r, int64_t i, double Q) {
+  uint64_t* w = a.wide_c + i;
+  const double ch = 0.8493218002880191, cl = -2.5959464104597403e-17;
+  double q0 = r.sg_f0 / a.step, q1 = (fma(-q0, a.step, r.sg_f0) - q0 * a.step_lo) / a.step;
+  const double nh = fabs(Q) * ch, nl = fma(fabs(Q), ch, -nh) + fabs(Q) * cl;
+  double s0 = nh / q0, s1 = (fma(-s0, q0, nh) + (nl - s0 * q1)) / q0;
+  const double far = q0 * 3.469446951953614e-18;  // beyond 2^58 bins f - f0 = -f0 in float64 too
+  if (far > 1.0) {
+    q0 /= far;
+    q1 = 0.0;
+    s0 *= far;
+    s1 *= far;
+  }
+  r.k_start = r.k_end = 0;
+  if (!(q0 > 0.0 && isfinite(far) && s0 > 0.0 && isfinite(s0))) q0 = s0 = 1.0, q1 = s1 = 0.0;  // (an invalid point)
+  const int frac = 61 - ilogb(q0 + (double)a.n_bins + 2.0), es = ilogb(s0) + 1;
+  const uint64_t sm = (uint64_t)ldexp(s0, 64 - es), sv = sm + (uint64_t)(int64_t)ldexp(s1, 64 - es);
+  w[0] = (uint64_t)(__double2ll_rn(ldexp(q0, frac)) + __double2ll_rn(ldexp(q1, frac)));
+  w[a.B] = (sv >> 63) ? sv : sm;
+  w[2 * a.B] = ((uint64_t)frac << 32) | (uint32_t)(es + 58 - frac);
+  w[3 * a.B] = (uint64_t)ldexp(fmin(sqrt(1020.0) / s0, ldexp(1.0, 62 - frac)), frac);
+  // y < 1020 (float64's exponential underflows at 1075) and within 100 of the
+  // smallest in-band y
+  const double lo = (double)a.k_lo, hi = (double)(a.k_hi - 1), x = fmax(0.0, fmax(lo - q0, q0 - hi)), y = s0 * x * (s0 * x);
+  if (y < 1020.0) {
+    const double R = sqrt(fmin(y + 100.0, 1020.0)) / s0;
+    r.k_start = (int64_t)fmin(fmax(ceil(q0 - R), lo), hi);
+    r.k_end = (int64_t)fmin(fmax(floor(q0 + R), lo), hi) + 1;
+  }
+  for (int d = 0; d < a.n_det; ++d) {
+    w[(int64_t)(kNumBasis + 2 + d) * a.B] = wide_shift(a, r.dt[d]);
+    w[(int64_t)(kNumBasis + 2 + kMaxDet + d) * a.B] = to_wide(atan2(r.fx[d] * r.amp2, r.fp[d] * r.amp) / kTwoPi, 0.0);
   }
 }
 
@@ -154,6 +209,7 @@ __device__ __noinline__ void prologue_point(const LaunchArgs& a, int64_t i) {
     r.amp = r.a[0] / r.a[1];
     r.amp2 = r.a[0] / r.a[2];
     ok = ok && isfinite(r.amp) && isfinite(r.amp2) && isfinite(r.sg_a) && f0 > 0;
+    if (a.wide_c) wide_coefficients_sg(a, r, i, Q);
   } else {
     const double m1 = par(a, GWL_P_MASS_1, i), m2 = par(a, GWL_P_MASS_2, i);
     const double chi1 = par(a, GWL_P_CHI_1, i), chi2 = par(a, GWL_P_CHI_2, i);
@@ -352,90 +408,11 @@ __global__ void k_order_scatter(LaunchArgs a) {
   if (i < a.B) order_scatter(a, i);
 }
 
-// ---------------------------------------------------------------------------
-// plain float64 kernels
-// ---------------------------------------------------------------------------
-// (c + i s) *= (rc + i rs): one bin of a uniform-grid rotation.  Over a
-// chunk of kChunkPlain bins its rounding error stays near 1e-13 rad.
+// (c + i s) *= (rc + i rs): one bin of a uniform-grid rotation.
 __device__ __forceinline__ void rotate(double& c, double& s, double rc, double rs) {
   const double t = c * rc - s * rs;
   s = c * rs + s * rc;
   c = t;
-}
-
-template <int D>
-__global__ void __launch_bounds__(kPointsPerCta) k_plain_sg(LaunchArgs a) {
-  constexpr int CH = kChunkPlain;
-  __shared__ double s_f[CH];
-  __shared__ double2 s_d[D][CH];
-  __shared__ double s_is[D][CH];
-  const int64_t k0 = a.k_base + (int64_t)blockIdx.y * CH;
-  for (int j = threadIdx.x; j < CH; j += blockDim.x) {
-    const int64_t k = k0 + j;
-    s_f[j] = a.freq[k];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      s_d[d][j] = reinterpret_cast<const double2*>(a.strain[d])[k];
-      s_is[d][j] = a.inv_psd[d][k];
-    }
-  }
-  __syncthreads();
-  const int64_t i = (int64_t)blockIdx.x * kPointsPerCta + threadIdx.x;
-  if (i >= a.B) return;
-  const PointRec& r = a.rec[i];
-  double dre[D], dim[D], hh[D], fp[D], fx[D], w2[D];
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    dre[d] = dim[d] = hh[d] = 0.0;
-    fp[d] = r.fp[d];
-    fx[d] = r.fx[d];
-    w2[d] = 2.0 * kPi * r.dt[d];
-  }
-  if (r.valid) {
-    const double f0 = r.sg_f0, amp = r.a[0], dplus = r.a[1], dcross = r.a[2], tau2 = r.a[3];
-    const double pi2 = 9.869604401089358;
-    // e^{i w f} on the chunk's uniform grid by rotation from its first bin
-    double zc[D], zs[D], rc[D], rs[D];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      sincos(w2[d] * s_f[0], &zs[d], &zc[d]);
-      sincos(w2[d] * a.step, &rs[d], &rc[d]);
-    }
-    for (int j = 0; j < CH; ++j) {
-      const double f = s_f[j];
-      // source.py:1199-1207
-      const double fm = f - f0, fpl = f + f0;
-      const double neg = exp(-(fm * fm) * pi2 * tau2);
-      const double pos = exp(-(fpl * fpl) * pi2 * tau2);
-      const double hp = amp * (neg + pos) / dplus;       // real
-      const double hx_im = -(amp * (neg - pos) / dcross); // h_x = i * hx_im
-#pragma unroll
-      for (int d = 0; d < D; ++d) {
-        const double is = s_is[d][j];
-        if (is == 0.0) continue;
-        // interferometer.py:341-362
-        const double sre = hp * fp[d];
-        const double sim = hx_im * fx[d];
-        const double sn = zs[d], cs = zc[d];  // exp(-i w f) = cs - i sn
-        const double hre = sre * cs + sim * sn;
-        const double him = sim * cs - sre * sn;
-        const double2 dd = s_d[d][j];
-        // utils.py:118-138: conj(h) * d / S
-        dre[d] += (hre * dd.x + him * dd.y) * is;
-        dim[d] += (hre * dd.y - him * dd.x) * is;
-        hh[d] += (hre * hre + him * him) * is;
-      }
-#pragma unroll
-      for (int d = 0; d < D; ++d) rotate(zc[d], zs[d], rc[d], rs[d]);
-    }
-  }
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    double* out = a.part + (((int64_t)blockIdx.y * D + d) * kPartStride) * a.B + i;
-    out[0 * a.B] = dre[d];
-    out[1 * a.B] = dim[d];
-    out[2 * a.B] = hh[d];
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1228,16 +1205,11 @@ __device__ void detector_totals(const LaunchArgs& a, int64_t i, int64_t G, const
   double sdr = 0.0, sdi = 0.0, shh = 0.0;
   for (int d = 0; d < a.n_det; ++d) {
     double p[kPartStride] = {0, 0, 0, 0, 0, 0};
-    if (a.precision == GWL_PRECISION_FP64) sum_groups<3>(a, i, d, G, p);
-    else if (a.model == GWL_MODEL_SINEGAUSSIAN) sum_groups<4>(a, i, d, G, p);
+    if (a.model == GWL_MODEL_SINEGAUSSIAN) sum_groups<4>(a, i, d, G, p);
     else if (a.cplx) sum_groups<2>(a, i, d, G, p);
     else sum_groups<1>(a, i, d, G, p);
     double dr, di, h;
-    if (a.precision == GWL_PRECISION_FP64) {
-      dr = norm * p[0];
-      di = norm * p[1];
-      h = norm * p[2];
-    } else if (a.model == GWL_MODEL_SINEGAUSSIAN) {
+    if (a.model == GWL_MODEL_SINEGAUSSIAN) {
       // conj(h) = M (a hp + i c hx) e^{+i theta}, M = |(Fp P, Fx X)| (see k_mixed_sg)
       const double M = hypot(r.fp[d] * r.amp, r.fx[d] * r.amp2), ws = a.w_scale[d], vs = a.v_scale[d];
       dr = norm * ws * M * p[0];
@@ -1256,10 +1228,9 @@ __device__ void detector_totals(const LaunchArgs& a, int64_t i, int64_t G, const
   *hh = shh;
 }
 
-// Components of a partial-sum record: <d|h> re/im and <h|h> (float64 kernels),
-// the six sums of the sine-Gaussian mixed kernel, re/im for TaylorF2 mixed.
+// Components of a mixed kernel's partial-sum record: the four sums of the
+// sine-Gaussian, re/im or re of TaylorF2.
 __device__ __host__ __forceinline__ int part_components(const LaunchArgs& a) {
-  if (a.precision == GWL_PRECISION_FP64) return 3;  // (TaylorF2 in float64 has its own finalize, gwl_wide.cu)
   return a.model == GWL_MODEL_SINEGAUSSIAN ? 4 : (a.cplx ? 2 : 1);
 }
 
@@ -1805,12 +1776,6 @@ cudaError_t launch_prologue(const LaunchArgs& a, cudaStream_t s) {
     case 3: KERNEL<3><<<GRID, BLOCK, SMEM, STREAM>>>(ARGS); break;      \
     default: KERNEL<4><<<GRID, BLOCK, SMEM, STREAM>>>(ARGS); break;     \
   }
-
-cudaError_t launch_plain(const LaunchArgs& a, cudaStream_t s) {
-  dim3 grid((unsigned)((a.B + kPointsPerCta - 1) / kPointsPerCta), (unsigned)a.n_chunks);
-  GWL_DISPATCH_D(k_plain_sg, grid, kPointsPerCta, 0, s, a);
-  return cudaGetLastError();
-}
 
 template <int D>
 constexpr auto k_mixed_tf2_c = k_mixed_tf2<D, true>;

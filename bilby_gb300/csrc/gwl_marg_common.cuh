@@ -302,14 +302,13 @@ __device__ inline void finish_point(const LaunchArgs& a, const PointRec& r, int6
   a.out[i] = lnl;
 }
 
-// <d|h>_d = dr + i di and <h|h>_d of TaylorF2 from the sums p of f^(-7/6) d / S
+// <d|h>_d = dr + i di (and <h|h>_d) of TaylorF2 from the sums p of f^(-7/6) d / S
 // e^{i phase}: conj(h_d) = A0 f^(-7/6) conj(Q) e^{+i Phi}, Q = Fp (1 + c^2) / 2 - i Fx c
-__device__ inline void tf2_detector_totals(const LaunchArgs& a, const PointRec& r, int d, const double* p, double* dr,
-                                           double* di, double* h) {
-  const double norm = 4.0 / a.duration;
+__device__ inline void tf2_project(const LaunchArgs& a, const PointRec& r, int d, double scale, const double* p,
+                                   double* dr, double* di) {
   const double ci = r.cos_i;
   const double qr = r.fp[d] * (1.0 + ci * ci) / 2.0, qi = -r.fx[d] * ci;
-  const double s = norm * a.w_scale[d] * r.amp;
+  const double s = scale * r.amp;
   if (a.cplx) {
     // (qr - i qi) * (p0 + i p1)
     *dr = s * (qr * p[0] + qi * p[1]);
@@ -319,9 +318,22 @@ __device__ inline void tf2_detector_totals(const LaunchArgs& a, const PointRec& 
     *dr = s * r.qabs[d] * p[0];
     *di = 0.0;
   }
+}
+
+// <h|h>_d = norm A0^2 |Q|^2 sum, sum the band's f^(-7/3) / S
+__device__ inline double tf2_norm(const PointRec& r, int d, double norm, double sum) {
+  const double ci = r.cos_i;
+  const double qr = r.fp[d] * (1.0 + ci * ci) / 2.0, qi = -r.fx[d] * ci;
+  return norm * r.amp * r.amp * (qr * qr + qi * qi) * sum;
+}
+
+__device__ inline void tf2_detector_totals(const LaunchArgs& a, const PointRec& r, int d, const double* p, double* dr,
+                                           double* di, double* h) {
+  const double norm = 4.0 / a.duration;
+  tf2_project(a, r, d, norm * a.w_scale[d], p, dr, di);
   const int64_t k1 = min(r.k_end, a.n_bins), k0 = min(r.k_start, k1);
   const double* pre = a.hh_prefix[d];
-  *h = norm * r.amp * r.amp * (qr * qr + qi * qi) * (pre[k1] - pre[k0]);
+  *h = tf2_norm(r, d, norm, pre[k1] - pre[k0]);
 }
 
 // exp(-2 pi i t / L) for t < L / 2 in float64 and float32, one pair of tables

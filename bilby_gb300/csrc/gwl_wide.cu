@@ -22,65 +22,13 @@
 #include "gwl_internal.h"
 #include "gwl_marg_common.cuh"
 #include "gwl_wide.cuh"
+#include "gwl_wide_basis.cuh"
 
 namespace gwl {
 
 constexpr int kSub = 32;                       // bins per sub-block
 constexpr int kSubs = kChunkPlain / kSub;      // sub-blocks per chunk
 constexpr int kWideThreads = 32 * kSubs;       // one warp per sub-block
-
-// The point's coefficients (LaunchArgs::wide_c, point fastest).
-template <int D>
-struct WidePoint {
-  uint64_t c[kNumBasis], c0, x[D], q[D];
-  int shift;
-  __device__ __forceinline__ void load(const LaunchArgs& a, int64_t i) {
-    const uint64_t* w = a.wide_c + i;
-#pragma unroll
-    for (int b = 0; b < kNumBasis; ++b) c[b] = w[(int64_t)b * a.B];
-    c0 = w[(int64_t)kNumBasis * a.B];
-    shift = (int)w[(int64_t)(kNumBasis + 1) * a.B];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      x[d] = w[(int64_t)(kNumBasis + 2 + d) * a.B];
-      q[d] = w[(int64_t)(kNumBasis + 2 + kMaxDet + d) * a.B];
-    }
-  }
-  // Phi at the bin whose table row is m (kNumBasis entries)
-  __device__ __forceinline__ uint64_t phase(const uint4* m) const {
-    int64_t acc = 0, cross = 0;
-#pragma unroll
-    for (int b = 0; b < kNumBasis / 2; ++b) {
-      const uint4 v = m[b];
-      wide_mac(acc, cross, (int32_t)(c[2 * b] >> 32), (int32_t)c[2 * b], (int32_t)v.x, (int32_t)v.y);
-      wide_mac(acc, cross, (int32_t)(c[2 * b + 1] >> 32), (int32_t)c[2 * b + 1], (int32_t)v.z, (int32_t)v.w);
-    }
-    return c0 + wide_fraction(acc, cross, shift);
-  }
-};
-
-// The terms of a pair of bins of one detector, um their weights' magnitudes and
-// ut their angles (LaunchArgs::wide_w): |w| cos 2 pi (a + arg w) as p + e, the
-// sine's as pi + ei.
-template <bool CPLX>
-__device__ __forceinline__ void wide_pair(uint64_t a0, uint64_t a1, const uint4& um, const uint4& ut, const float4* tab,
-                                          float2& p, float2& e, float2& pi, float2& ei) {
-  a0 += ((uint64_t)ut.y << 32) | ut.x;
-  a1 += ((uint64_t)ut.w << 32) | ut.z;
-  uint32_t q0, q1, ra0, ra1, rb0, rb1;
-  wide_remainder(a0, q0, ra0, rb0);
-  wide_remainder(a1, q1, ra1, rb1);
-  const WideArg x = wide_arg2(ra0, rb0, ra1, rb1);
-  const float2 wh = make_float2(__uint_as_float(um.x), __uint_as_float(um.y));
-  const float2 wl = make_float2(__uint_as_float(um.z), __uint_as_float(um.w));
-  float2 ch, cl;
-  wide_cos2(tab[q0], tab[q1], x, ch, cl);
-  wide_term2(wh, wl, ch, cl, p, e);
-  if (CPLX) {
-    wide_cos2(tab[(q0 - kWideTable / 4) & (kWideTable - 1)], tab[(q1 - kWideTable / 4) & (kWideTable - 1)], x, ch, cl);
-    wide_term2(wh, wl, ch, cl, pi, ei);
-  }
-}
 
 // The cosine table, the chunk's phase basis and the chunk's weights.
 template <int D>
@@ -91,6 +39,32 @@ __device__ __forceinline__ void wide_stage(const LaunchArgs& a, int64_t k0, floa
 #pragma unroll
   for (int d = 0; d < D; ++d)
     for (int q = threadIdx.x; q < kChunkPlain; q += kWideThreads) w[d * kChunkPlain + q] = a.wide_w[d][k0 + q];
+}
+
+// The sub-block at table row k: its first grid index and stride.
+struct WideRows {
+  int64_t first, stride;
+};
+__device__ __forceinline__ WideRows wide_block(const LaunchArgs& a, int64_t k) {
+  if (!a.wide_sub) return WideRows{k, 1};
+  const int2 s = a.wide_sub[k / kSub];
+  return WideRows{s.x, s.y};
+}
+// The grid index of the point's band end, for a list beyond the grid's last too.
+__device__ __forceinline__ int64_t wide_end(const LaunchArgs& a, int64_t i) {
+  return a.wide_sub ? (int64_t)a.wide_c[(int64_t)kWideEnd * a.B + i] : a.rec[i].k_end;
+}
+// Its rows [j0, j1) inside the band [lo, hi) of grid indices (a list's lower end
+// is in its weights: its frequencies, not the grid's, are tested on the host).
+__device__ __forceinline__ void wide_rows(const WideRows& b, int64_t lo, int64_t hi, int& j0, int& j1) {
+  if (b.stride == 1) {
+    j0 = (int)min(max(lo - b.first, (int64_t)0), (int64_t)kSub);
+    j1 = (int)min(max(hi - b.first, (int64_t)0), (int64_t)kSub);
+  } else {
+    j0 = 0;
+    j1 = hi > b.first ? (int)min((hi - b.first + b.stride - 1) / b.stride, (int64_t)kSub) : 0;
+  }
+  if (j1 <= j0) j1 = 0;
 }
 
 // Batches.  CTA (chunk, point slice): one warp per sub-block, lane = point, 32
@@ -109,21 +83,17 @@ __global__ void __launch_bounds__(kWideThreads, 2) k_wide_tf2(LaunchArgs a, int 
   uint4* phi = reinterpret_cast<uint4*>(tab + kWideTable);
   uint4* w = reinterpret_cast<uint4*>(phi + kChunkPlain * kNumBasis / 2);
   double* sums = reinterpret_cast<double*>(w + D * kChunkPlain);  // [kSubs][D * NC][32]
-  const int64_t k0 = a.k_base + (int64_t)blockIdx.x * kChunkPlain;
+  const int64_t k0 = a.wide_base + (int64_t)blockIdx.x * kChunkPlain;
   wide_stage<D>(a, k0, tab, phi, w);
   __syncthreads();
   const int lane = threadIdx.x & 31, sub = threadIdx.x >> 5;
-  const int64_t ks = k0 + sub * kSub;
+  const WideRows rows = wide_block(a, k0 + sub * kSub);
   const int64_t t1 = min((int64_t)(blockIdx.y + 1) * tiles, (a.B + 31) / 32);
   for (int64_t t = (int64_t)blockIdx.y * tiles; t < t1; ++t) {
     const bool have = t * 32 + lane < a.B;
     const int64_t i = have ? (a.order ? (int64_t)a.order[t * 32 + lane] : t * 32 + lane) : 0;
-    int64_t lo = 0, hi = 0;
-    if (have && a.rec[i].valid) {
-      lo = max(a.rec[i].k_start, ks);
-      hi = min(a.rec[i].k_end, ks + kSub);
-    }
-    const int j0 = (int)(lo - ks), j1 = hi > lo ? (int)(hi - ks) : 0;  // this lane's bins [j0, j1) of the sub-block
+    int j0 = 0, j1 = 0;  // this lane's rows [j0, j1) of the sub-block
+    if (have && a.rec[i].valid) wide_rows(rows, a.wide_sub ? 0 : a.rec[i].k_start, wide_end(a, i), j0, j1);
     float2 hr[D], lr[D], hm[D], lm[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) hr[d] = lr[d] = hm[d] = lm[d] = make_float2(0.f, 0.f);
@@ -132,7 +102,10 @@ __global__ void __launch_bounds__(kWideThreads, 2) k_wide_tf2(LaunchArgs a, int 
       pt.load(a, i);
       uint64_t sh[D];
 #pragma unroll
-      for (int d = 0; d < D; ++d) sh[d] = (uint64_t)ks * pt.x[d] + pt.q[d];
+      for (int d = 0; d < D; ++d) {
+        sh[d] = (uint64_t)rows.first * pt.x[d] + pt.q[d];
+        pt.x[d] *= (uint64_t)rows.stride;
+      }
       const uint4* m = phi + sub * kSub * (kNumBasis / 2);
       const uint4* ws = w + sub * kSub;
 #pragma unroll 1
@@ -176,7 +149,7 @@ __global__ void __launch_bounds__(kWideThreads, 2) k_wide_tf2(LaunchArgs a, int 
         double s = sums[c];
 #pragma unroll
         for (int q = 1; q < kSubs; ++q) s += sums[q * D * NC * 32 + c];
-        a.part[(ip * D * NC + (c >> 5)) * a.n_chunks + blockIdx.x] = s;
+        a.part[(ip * D * NC + (c >> 5)) * a.wide_chunks + blockIdx.x] = s;
       }
     }
     __syncthreads();
@@ -197,7 +170,7 @@ __global__ void __launch_bounds__(kPairThreads) k_wide_tf2_few(LaunchArgs a) {
   constexpr int kPer = kSub / 2, kRow = kPer + 1;  // pairs per sub-block, padded
   __shared__ float2 term[NS][2][kSubs][kRow];      // (p, e) of one bin
   __shared__ double part[NS][2][kSubs];
-  const int64_t k0 = a.k_base + (int64_t)blockIdx.x * kChunkPlain;
+  const int64_t k0 = a.wide_base + (int64_t)blockIdx.x * kChunkPlain;
   const int t = threadIdx.x, sub = t / kPer, pr = t % kPer;
   const int64_t k = k0 + 2 * t;
   uint4 m[kNumBasis];
@@ -209,92 +182,170 @@ __global__ void __launch_bounds__(kPairThreads) k_wide_tf2_few(LaunchArgs a) {
     w0[d] = a.wide_w[d][k];
     w1[d] = a.wide_w[d][k + 1];
   }
-  for (int64_t i = blockIdx.y; i < a.B; i += gridDim.y) {
-    const PointRec& r = a.rec[i];
-    const int64_t lo = r.k_start, hi = r.valid ? r.k_end : 0;
-    const bool on0 = k >= lo && k < hi, on1 = k + 1 >= lo && k + 1 < hi;
-    WidePoint<D> pt;
-    uint64_t b0 = 0, b1 = 0;
+  const int64_t i = blockIdx.y;
+  const PointRec& r = a.rec[i];
+  const WideRows rows = wide_block(a, k0 + sub * kSub);
+  int j0 = 0, j1 = 0;
+  if (r.valid) wide_rows(rows, a.wide_sub ? 0 : r.k_start, wide_end(a, i), j0, j1);
+  const int j = 2 * pr;
+  const bool on0 = j >= j0 && j < j1, on1 = j + 1 >= j0 && j + 1 < j1;
+  WidePoint<D> pt;
+  uint64_t b0 = 0, b1 = 0;
+  if (on0 || on1) {
+    pt.load(a, i);
+    b0 = pt.phase(m);
+    b1 = pt.phase(m + kNumBasis / 2);
+  }
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    float2 p, e, pi, ei;
+    p = e = pi = ei = make_float2(0.f, 0.f);
     if (on0 || on1) {
-      pt.load(a, i);
-      b0 = pt.phase(m);
-      b1 = pt.phase(m + kNumBasis / 2);
+      const uint64_t sh = (uint64_t)(rows.first + j * rows.stride) * pt.x[d] + pt.q[d];
+      wide_pair<CPLX>(b0 + sh, b1 + (sh + (uint64_t)rows.stride * pt.x[d]), w0[d], w1[d], a.wide_tab, p, e, pi, ei);
     }
+    term[d * NC][0][sub][pr] = on0 ? make_float2(p.x, e.x) : make_float2(0.f, 0.f);
+    term[d * NC][1][sub][pr] = on1 ? make_float2(p.y, e.y) : make_float2(0.f, 0.f);
+    if (CPLX) {
+      term[d * NC + 1][0][sub][pr] = on0 ? make_float2(pi.x, ei.x) : make_float2(0.f, 0.f);
+      term[d * NC + 1][1][sub][pr] = on1 ? make_float2(pi.y, ei.y) : make_float2(0.f, 0.f);
+    }
+  }
+  __syncthreads();
+  for (int c = t; c < NS * 2 * kSubs; c += kPairThreads) {
+    const float2* src = &term[0][0][0][0] + (int64_t)c * kRow;
+    float h = 0.f, l = 0.f;
 #pragma unroll
-    for (int d = 0; d < D; ++d) {
-      float2 p, e, pi, ei;
-      p = e = pi = ei = make_float2(0.f, 0.f);
-      if (on0 || on1) {
-        const uint64_t sh = (uint64_t)k * pt.x[d] + pt.q[d];
-        wide_pair<CPLX>(b0 + sh, b1 + (sh + pt.x[d]), w0[d], w1[d], a.wide_tab, p, e, pi, ei);
-      }
-      term[d * NC][0][sub][pr] = on0 ? make_float2(p.x, e.x) : make_float2(0.f, 0.f);
-      term[d * NC][1][sub][pr] = on1 ? make_float2(p.y, e.y) : make_float2(0.f, 0.f);
-      if (CPLX) {
-        term[d * NC + 1][0][sub][pr] = on0 ? make_float2(pi.x, ei.x) : make_float2(0.f, 0.f);
-        term[d * NC + 1][1][sub][pr] = on1 ? make_float2(pi.y, ei.y) : make_float2(0.f, 0.f);
-      }
+    for (int q = 0; q < kPer; ++q) {
+      const float2 v = src[q];
+      const float s = __fadd_rn(h, v.x), bb = __fsub_rn(s, h);
+      const float err = __fadd_rn(__fsub_rn(h, __fsub_rn(s, bb)), __fsub_rn(v.x, bb));
+      h = s;
+      l = __fadd_rn(l, __fadd_rn(err, v.y));
     }
-    __syncthreads();
-    for (int c = t; c < NS * 2 * kSubs; c += kPairThreads) {
-      const float2* src = &term[0][0][0][0] + (int64_t)c * kRow;
-      float h = 0.f, l = 0.f;
+    (&part[0][0][0])[c] = (double)h + (double)l;
+  }
+  __syncthreads();
+  if (t < NS) {
+    double s = part[t][0][0] + part[t][1][0];
 #pragma unroll
-      for (int q = 0; q < kPer; ++q) {
-        const float2 v = src[q];
-        const float s = __fadd_rn(h, v.x), bb = __fsub_rn(s, h);
-        const float err = __fadd_rn(__fsub_rn(h, __fsub_rn(s, bb)), __fsub_rn(v.x, bb));
-        h = s;
-        l = __fadd_rn(l, __fadd_rn(err, v.y));
-      }
-      (&part[0][0][0])[c] = (double)h + (double)l;
-    }
-    __syncthreads();
-    if (t < NS) {
-      double s = part[t][0][0] + part[t][1][0];
-#pragma unroll
-      for (int q = 1; q < kSubs; ++q) s += part[t][0][q] + part[t][1][q];
-      a.part[(i * NS + t) * a.n_chunks + blockIdx.x] = s;
-    }
+    for (int q = 1; q < kSubs; ++q) s += part[t][0][q] + part[t][1][q];
+    a.part[(i * NS + t) * a.wide_chunks + blockIdx.x] = s;
   }
 }
 
-// One warp per point: the chunks' sums in a fixed order, the totals and the
-// lnL.
-constexpr int kWideFinWarps = 4;
+// The chunks' sums in a fixed order, the totals and the lnL.
+constexpr int kWideFinThreads = 128;
 
-__global__ void __launch_bounds__(32 * kWideFinWarps) k_wide_finalize(LaunchArgs a) {
-  const int lane = threadIdx.x & 31;
-  const int64_t i = (int64_t)blockIdx.x * kWideFinWarps + (threadIdx.x >> 5);
-  if (i >= a.B) return;  // uniform over the warp
+__global__ void __launch_bounds__(kWideFinThreads) k_wide_finalize(LaunchArgs a) {
+  const int lanes = wide_lanes(a.wide_chunks), lane = threadIdx.x & (lanes - 1);
+  const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / lanes, i = min(slot, a.B - 1);
   const PointRec& r = a.rec[i];
   const int nc = a.cplx ? 2 : 1;
   double p[2 * kMaxDet];
   for (int c = 0; c < a.n_det * nc; ++c) {
-    const double* q = a.part + (i * a.n_det * nc + c) * a.n_chunks;
-    double s = 0.0;
-    for (int64_t g = lane; g < a.n_chunks; g += 32) s += q[g];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    p[c] = s;
+    const double* q = a.part + (i * a.n_det * nc + c) * a.wide_chunks;
+    p[c] = wide_chunk_sum(q, a.wide_chunks, lane, lanes);
   }
-  if (lane == 0) {
-    double dr = 0.0, di = 0.0, hh = 0.0;
+  double sum[kMaxDet];  // <h|h> per A0^2 |Q|^2 and norm
+  for (int d = 0; d < a.n_det; ++d) {
+    if (!a.wide_sub) {
+      const int64_t k1 = min(r.k_end, a.n_bins), k0 = min(r.k_start, k1);
+      sum[d] = a.hh_prefix[d][k1] - a.hh_prefix[d][k0];
+      continue;
+    }
+    const int64_t end = wide_end(a, i);
+    double s = 0.0;
+    for (int b = lane; b < a.wide_bands; b += lanes) {
+      const int4 v = a.wide_band[b];
+      const int64_t n = end > v.z ? min((end - v.z + v.w - 1) / v.w, (int64_t)v.y) : 0;
+      s += a.wide_q[d][v.x + n] - a.wide_q[d][v.x];
+    }
+    for (int o = lanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    sum[d] = s;
+  }
+  if (lane == 0 && slot < a.B) {
+    double dr = 0.0, di = 0.0, hh = r.valid ? mb_fft_hh_total(a, i) : 0.0;
     for (int d = 0; d < a.n_det; ++d) {
-      double x, z, h;
-      tf2_detector_totals(a, r, d, p + d * nc, &x, &z, &h);
+      double x, z;
+      tf2_project(a, r, d, a.wide_norm * a.wide_wscale[d], p + d * nc, &x, &z);
       dr += x;
       di += z;
-      hh += h;
+      hh += tf2_norm(r, d, a.wide_norm, sum[d]);
     }
     finish_point(a, r, i, dr, di, hh);
   }
 }
 
+// ---------------------------------------------------------------------------
+// tables
+// ---------------------------------------------------------------------------
+struct WideScale {
+  double inv[kNumBasis];
+};
+
+__device__ __forceinline__ uint64_t fraction64(double hi, double lo) {
+  return (uint64_t)ldexp(hi, 64) + (uint64_t)__double2ll_rn(ldexp(lo, 64));
+}
+
+__global__ void k_wide_basis(const double* f, int64_t k0, int64_t n, int64_t pad, double lnref, WideScale sc, uint4* out) {
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= pad) return;
+  uint64_t v[kNumBasis];
+#pragma unroll
+  for (int b = 0; b < kNumBasis; ++b) v[b] = 0;
+  if (k >= k0 && k < n && f[k] > 0) {
+    double hi[kNumBasis], lo[kNumBasis];
+    wide_basis(f[k], lnref, hi, lo);
+#pragma unroll
+    for (int b = 0; b < kNumBasis; ++b)  // rounded to 58 bits (below 1: the scale leaves a margin of 1e-9)
+      v[b] = (fraction64(hi[b] * sc.inv[b], lo[b] * sc.inv[b]) + 32) >> 6;
+  }
+#pragma unroll
+  for (int b = 0; b < kNumBasis / 2; ++b)
+    out[k * (kNumBasis / 2) + b] =
+        make_uint4((uint32_t)(v[2 * b] & 0x7ffffff), (uint32_t)(v[2 * b] >> 27), (uint32_t)(v[2 * b + 1] & 0x7ffffff),
+                   (uint32_t)(v[2 * b + 1] >> 27));
+}
+
+// thread: a pair of rows
+__global__ void k_wide_weights(const double2* z, const double* u, const double4* ftab, double inv_scale, int64_t n,
+                               uint4* out) {
+  const int64_t k = 2 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+  if (k >= n) return;
+  float2 m[2];
+  uint64_t t[2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const double g = (ftab ? ftab[k + q].w : 1.0) * u[k + q] * inv_scale;
+    const double x = g == 0.0 ? 0.0 : g * z[k + q].x, y = g == 0.0 ? 0.0 : g * z[k + q].y;
+    const double h = hypot(x, y), c = atan2(y, x) / kTwoPi;
+    m[q].x = (float)h;
+    m[q].y = (float)(h - (double)m[q].x);
+    t[q] = fraction64(c < 0.0 ? c + 1.0 : c, 0.0);
+  }
+  out[k] = make_uint4(__float_as_uint(m[0].x), __float_as_uint(m[1].x), __float_as_uint(m[0].y), __float_as_uint(m[1].y));
+  out[k + 1] = make_uint4((uint32_t)t[0], (uint32_t)(t[0] >> 32), (uint32_t)t[1], (uint32_t)(t[1] >> 32));
+}
+
+cudaError_t launch_wide_basis(const double* f, int64_t k0, int64_t n, int64_t pad, double lnref, const double* scale,
+                              uint4* out, cudaStream_t s) {
+  WideScale sc;
+  for (int b = 0; b < kNumBasis; ++b) sc.inv[b] = 1.0 / scale[b];
+  k_wide_basis<<<(unsigned)((pad + 127) / 128), 128, 0, s>>>(f, k0, n, pad, lnref, sc, out);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_wide_weights(const double2* z, const double* u, const double4* ftab, double inv_scale, int64_t n,
+                                uint4* out, cudaStream_t s) {
+  k_wide_weights<<<(unsigned)((n / 2 + 127) / 128), 128, 0, s>>>(z, u, ftab, inv_scale, n, out);
+  return cudaGetLastError();
+}
+
 template <int D, bool CPLX>
 static cudaError_t launch_wide_d(const LaunchArgs& a, cudaStream_t s) {
   if (a.B <= kWideFewPoints) {
-    const dim3 grid((unsigned)a.n_chunks, (unsigned)a.B);
+    const dim3 grid((unsigned)a.wide_chunks, (unsigned)a.B);
     k_wide_tf2_few<D, CPLX><<<grid, kPairThreads, 0, s>>>(a);
     return cudaGetLastError();
   }
@@ -307,8 +358,8 @@ static cudaError_t launch_wide_d(const LaunchArgs& a, cudaStream_t s) {
   // up to eight tiles share a CTA's tables while the grid stays at eight CTAs
   // per SM or more
   int per = 1;
-  while (per < 8 && a.n_chunks * (tiles / (2 * per)) >= 8 * 152) per *= 2;
-  const dim3 grid((unsigned)a.n_chunks, (unsigned)((tiles + per - 1) / per));
+  while (per < 8 && a.wide_chunks * (tiles / (2 * per)) >= 8 * 152) per *= 2;
+  const dim3 grid((unsigned)a.wide_chunks, (unsigned)((tiles + per - 1) / per));
   k_wide_tf2<D, CPLX><<<grid, kWideThreads, smem, s>>>(a, per);
   return cudaGetLastError();
 }
@@ -326,7 +377,7 @@ cudaError_t launch_wide(const LaunchArgs& a, cudaStream_t s) {
     default: e = launch_wide_d<4, true>(a, s); break;
   }
   if (e != cudaSuccess) return e;
-  k_wide_finalize<<<(unsigned)((a.B + kWideFinWarps - 1) / kWideFinWarps), 32 * kWideFinWarps, 0, s>>>(a);
+  k_wide_finalize<<<(unsigned)((a.B * wide_lanes(a.wide_chunks) + kWideFinThreads - 1) / kWideFinThreads), kWideFinThreads, 0, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -116,4 +116,69 @@ __device__ __forceinline__ void wide_add2(float2& hi, float2& lo, float2 p, floa
   lo = add2(lo, add2(err, e));
 }
 
+// The point's coefficients (LaunchArgs::wide_c, point fastest).
+template <int D>
+struct WidePoint {
+  uint64_t c[kNumBasis], c0, x[D], q[D];
+  int shift;
+  __device__ __forceinline__ void load(const LaunchArgs& a, int64_t i) {
+    const uint64_t* w = a.wide_c + i;
+#pragma unroll
+    for (int b = 0; b < kNumBasis; ++b) c[b] = w[(int64_t)b * a.B];
+    c0 = w[(int64_t)kNumBasis * a.B];
+    shift = (int)w[(int64_t)(kNumBasis + 1) * a.B];
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      x[d] = w[(int64_t)(kNumBasis + 2 + d) * a.B];
+      q[d] = w[(int64_t)(kNumBasis + 2 + kMaxDet + d) * a.B];
+    }
+  }
+  // Phi at the bin whose table row is m (kNumBasis entries)
+  __device__ __forceinline__ uint64_t phase(const uint4* m) const {
+    int64_t acc = 0, cross = 0;
+#pragma unroll
+    for (int b = 0; b < kNumBasis / 2; ++b) {
+      const uint4 v = m[b];
+      wide_mac(acc, cross, (int32_t)(c[2 * b] >> 32), (int32_t)c[2 * b], (int32_t)v.x, (int32_t)v.y);
+      wide_mac(acc, cross, (int32_t)(c[2 * b + 1] >> 32), (int32_t)c[2 * b + 1], (int32_t)v.z, (int32_t)v.w);
+    }
+    return c0 + wide_fraction(acc, cross, shift);
+  }
+};
+
+// The terms of a pair of bins of one detector, um their weights' magnitudes and
+// ut their angles (LaunchArgs::wide_w): |w| cos 2 pi (a + arg w) as p + e, the
+// sine's as pi + ei.
+template <bool CPLX>
+__device__ __forceinline__ void wide_pair(uint64_t a0, uint64_t a1, const uint4& um, const uint4& ut, const float4* tab,
+                                          float2& p, float2& e, float2& pi, float2& ei) {
+  a0 += ((uint64_t)ut.y << 32) | ut.x;
+  a1 += ((uint64_t)ut.w << 32) | ut.z;
+  uint32_t q0, q1, ra0, ra1, rb0, rb1;
+  wide_remainder(a0, q0, ra0, rb0);
+  wide_remainder(a1, q1, ra1, rb1);
+  const WideArg x = wide_arg2(ra0, rb0, ra1, rb1);
+  const float2 wh = make_float2(__uint_as_float(um.x), __uint_as_float(um.y));
+  const float2 wl = make_float2(__uint_as_float(um.z), __uint_as_float(um.w));
+  float2 ch, cl;
+  wide_cos2(tab[q0], tab[q1], x, ch, cl);
+  wide_term2(wh, wl, ch, cl, p, e);
+  if (CPLX) {
+    wide_cos2(tab[(q0 - kWideTable / 4) & (kWideTable - 1)], tab[(q1 - kWideTable / 4) & (kWideTable - 1)], x, ch, cl);
+    wide_term2(wh, wl, ch, cl, pi, ei);
+  }
+}
+
+// Lanes that add one point's chunks: lane l of them takes chunks l, l + n, ...,
+// then a fixed tree.  With 17 chunks (4 s at 2048 Hz) a whole warp per point
+// took 81 us for 10,000 points, nearly all of it in the tree's float64 adds.
+__host__ __device__ __forceinline__ int wide_lanes(int64_t n_chunks) { return n_chunks > 256 ? 32 : (n_chunks > 32 ? 8 : 4); }
+
+__device__ __forceinline__ double wide_chunk_sum(const double* q, int64_t n, int lane, int lanes) {
+  double s = 0.0;
+  for (int64_t g = lane; g < n; g += lanes) s += q[g];
+  for (int o = lanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
 }  // namespace gwl
