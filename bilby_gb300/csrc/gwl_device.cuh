@@ -20,9 +20,18 @@ constexpr double kPcSI = 3.085677581491367e16;      // parsec (m)
 constexpr double kGammaE = 0.5772156649015329;
 
 // GPS seconds at which each leap second was inserted (bilby/gw/time.py:74-93).
-__constant__ double c_leap_seconds[18] = {
+__constant__ long long c_leap_seconds[18] = {
     46828800, 78364801, 109900802, 173059203, 252028804, 315187205, 346723206, 393984007, 425520008,
     457056009, 504489610, 551750411, 599184012, 820108813, 914803214, 1025136015, 1119744016, 1167264017};
+
+// x / d for a constant d and its rounded reciprocal rd, correctly rounded: a
+// quotient within an ulp or two corrected by its exact remainder (Markstein, IBM
+// J. Res. Dev. 34, 111 (1990)); three operations where the division takes some
+// fifteen.
+__device__ __forceinline__ double div_const(double x, double d, double rd) {
+  const double q = __dmul_rn(x, rd);
+  return __fma_rn(__fma_rn(-q, d, x), rd, q);
+}
 
 // Greenwich mean sidereal time in radians, unreduced.  Same operation order
 // as bilby/gw/time.py:114-165 (gps -> barebones UTC datetime -> Julian day ->
@@ -30,28 +39,34 @@ __constant__ double c_leap_seconds[18] = {
 // does not contract the accumulation into FMAs.
 __device__ __forceinline__ double gmst_radians(double gps) {
   const double gps_int = floor(gps);
-  double nleap = 0.0;
+  const long long gps_whole = (long long)gps_int;
+  int n = 0;
 #pragma unroll
-  for (int i = 0; i < 18; ++i) nleap += (gps_int > c_leap_seconds[i]) ? 1.0 : 0.0;
+  for (int i = 0; i < 18; ++i) n += gps_whole > c_leap_seconds[i] ? 1 : 0;
+  const double nleap = (double)n;
   // 367*1980 - 7*(1980 + (1+9)//12)//4 + 275*1//9 + 6 = 723231 (time.py:57-66)
   const double second = __dsub_rn(gps_int, nleap);
-  const double jd = __dadd_rn(__dadd_rn(723231.0, __ddiv_rn(second, 86400.0)), 1721013.5);
-  const double t_hi = __ddiv_rn(__dsub_rn(jd, 2451545.0), 36525.0);
-  const double t_lo = __ddiv_rn(__dsub_rn(gps, gps_int), 3155760000.0);
+  const double jd = __dadd_rn(__dadd_rn(723231.0, div_const(second, 86400.0, 1.0 / 86400.0)), 1721013.5);
+  const double t_hi = div_const(__dsub_rn(jd, 2451545.0), 36525.0, 1.0 / 36525.0);
+  const double t_lo = div_const(__dsub_rn(gps, gps_int), 3155760000.0, 1.0 / 3155760000.0);
   const double t = __dadd_rn(t_hi, t_lo);
   double st = __dadd_rn(__dmul_rn(__dadd_rn(__dmul_rn(-6.2e-6, t), 0.093104), __dmul_rn(t, t)), 67310.54841);
   st = __dadd_rn(st, __dmul_rn(8640184.812866, t_lo));
   st = __dadd_rn(st, __dmul_rn(3155760000.0, t_lo));
   st = __dadd_rn(st, __dmul_rn(8640184.812866, t_hi));
   st = __dadd_rn(st, __dmul_rn(3155760000.0, t_hi));
-  return __ddiv_rn(__dmul_rn(__dmul_rn(st, 2.0), kPi), 86400.0);
+  return div_const(__dmul_rn(__dmul_rn(st, 2.0), kPi), 86400.0, 1.0 / 86400.0);
 }
 
-// Python's float modulo for a positive divisor.
-__device__ __forceinline__ double pymod(double x, double y) {
-  double r = fmod(x, y);
-  if (r < 0) r += y;
-  return r;
+// Python's float modulo 2 pi: x - n 2 pi is exact for the right n (it is what
+// fmod returns), and for |x| < 2^40 the rounded quotient is off by one at most.
+__device__ __forceinline__ double mod_two_pi(double x) {
+  if (!(fabs(x) < 1.0995e12)) {
+    const double r = fmod(x, kTwoPi);
+    return r < 0 ? r + kTwoPi : r;
+  }
+  const double r = __fma_rn(-floor(x * (1.0 / kTwoPi)), kTwoPi, x);
+  return r < 0 ? r + kTwoPi : (r >= kTwoPi ? r - kTwoPi : r);
 }
 
 // Sines and cosines of the sky frame of one point (shared by its detectors).
@@ -93,7 +108,8 @@ __device__ __forceinline__ void antenna_and_delay(const double* tensor, const do
   *fplus = fp;
   *fcross = fx;
   const double om[3] = {sth * cphi, sth * sphi, cth};
-  *delay = (om[0] * (0.0 - vertex[0]) + om[1] * (0.0 - vertex[1]) + om[2] * (0.0 - vertex[2])) / kSpeedOfLight;
+  *delay = (om[0] * (0.0 - vertex[0]) + om[1] * (0.0 - vertex[1]) + om[2] * (0.0 - vertex[2]));
+  *delay = div_const(*delay, kSpeedOfLight, 1.0 / kSpeedOfLight);
 }
 
 __device__ __forceinline__ void antenna_and_delay(const double* tensor, const double* vertex, double ra,
@@ -120,30 +136,30 @@ __device__ __host__ inline void taylorf2_coefficients(double m1, double m2, doub
     l[k] = 0.0;
   }
   a[0] = 1.0;
-  a[2] = 3715.0 / 756.0 + 55.0 * eta / 9.0;
-  a[3] = -16.0 * pi + 113.0 / 3.0 * delta * ca + (113.0 / 3.0 - 76.0 * eta / 3.0) * cs;
-  a[4] = 15293365.0 / 508032.0 + 27145.0 * eta / 504.0 + 3085.0 * eta * eta / 72.0 +
+  a[2] = 3715.0 / 756.0 + (55.0 / 9.0) * eta;
+  a[3] = -16.0 * pi + 113.0 / 3.0 * delta * ca + (113.0 / 3.0 - (76.0 / 3.0) * eta) * cs;
+  a[4] = 15293365.0 / 508032.0 + (27145.0 / 504.0) * eta + (3085.0 / 72.0) * eta * eta +
          (-405.0 / 8.0 + 200.0 * eta) * ca * ca - 405.0 / 4.0 * delta * cs * ca +
-         (-405.0 / 8.0 + 5.0 * eta / 2.0) * cs * cs;
-  const double gamma = (732985.0 / 2268.0 - 24260.0 * eta / 81.0 - 340.0 * eta * eta / 9.0) * cs +
-                       (732985.0 / 2268.0 + 140.0 * eta / 9.0) * delta * ca;
-  const double c5 = pi * (38645.0 / 756.0 - 65.0 * eta / 9.0) - gamma;
+         (-405.0 / 8.0 + (5.0 / 2.0) * eta) * cs * cs;
+  const double gamma = (732985.0 / 2268.0 - (24260.0 / 81.0) * eta - (340.0 / 9.0) * eta * eta) * cs +
+                       (732985.0 / 2268.0 + (140.0 / 9.0) * eta) * delta * ca;
+  const double c5 = pi * (38645.0 / 756.0 - (65.0 / 9.0) * eta) - gamma;
   a[5] = c5;
   l[5] = 3.0 * c5;
   a[6] = 11583231236531.0 / 4694215680.0 - 640.0 * pi * pi / 3.0 - 6848.0 * kGammaE / 21.0 -
          6848.0 / 21.0 * 1.3862943611198906 /* ln 4 */ +
-         eta * (-15737765635.0 / 3048192.0 + 2255.0 * pi * pi / 12.0) + 76055.0 * eta * eta / 1728.0 -
-         127825.0 * eta * eta * eta / 1296.0 +
+         eta * (-15737765635.0 / 3048192.0 + 2255.0 * pi * pi / 12.0) + (76055.0 / 1728.0) * eta * eta -
+         (127825.0 / 1296.0) * eta * eta * eta +
          pi * (2270.0 / 3.0 * delta * ca + (2270.0 / 3.0 - 520.0 * eta) * cs) +
-         (75515.0 / 144.0 - 8225.0 * eta / 18.0) * delta * cs * ca +
-         (75515.0 / 288.0 - 263245.0 * eta / 252.0 - 480.0 * eta * eta) * ca * ca +
-         (75515.0 / 288.0 - 232415.0 * eta / 504.0 + 1255.0 * eta * eta / 9.0) * cs * cs;
+         (75515.0 / 144.0 - (8225.0 / 18.0) * eta) * delta * cs * ca +
+         (75515.0 / 288.0 - (263245.0 / 252.0) * eta - 480.0 * eta * eta) * ca * ca +
+         (75515.0 / 288.0 - (232415.0 / 504.0) * eta + (1255.0 / 9.0) * eta * eta) * cs * cs;
   l[6] = -6848.0 / 21.0;
-  a[7] = pi * (77096675.0 / 254016.0 + 378515.0 * eta / 1512.0 - 74045.0 * eta * eta / 756.0) +
-         (-25150083775.0 / 3048192.0 + 10566655595.0 * eta / 762048.0 - 1042165.0 * eta * eta / 3024.0 +
-          5345.0 * eta * eta * eta / 36.0) *
+  a[7] = pi * (77096675.0 / 254016.0 + (378515.0 / 1512.0) * eta - (74045.0 / 756.0) * eta * eta) +
+         (-25150083775.0 / 3048192.0 + (10566655595.0 / 762048.0) * eta - (1042165.0 / 3024.0) * eta * eta +
+          (5345.0 / 36.0) * eta * eta * eta) *
              cs +
-         delta * (-25150083775.0 / 3048192.0 + 26804935.0 * eta / 6048.0 - 1985.0 * eta * eta / 48.0) * ca;
+         delta * (-25150083775.0 / 3048192.0 + (26804935.0 / 6048.0) * eta - (1985.0 / 48.0) * eta * eta) * ca;
 }
 
 // ---------------------------------------------------------------------------

@@ -29,7 +29,13 @@ __device__ __forceinline__ double par(const LaunchArgs& a, int slot, int64_t i) 
 // points marked for the accurate kernel take the upper half of the keys, so
 // that (buckets in descending order) they fill the first slots
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int order_key(const LaunchArgs& a, const PointRec& r) {
+struct OrderPoint {
+  int valid, refine;
+  int64_t k_start, k_end;
+  double sg_f0;
+};
+
+__device__ __forceinline__ int order_key(const LaunchArgs& a, const OrderPoint& r) {
   if (a.model == GWL_MODEL_SINEGAUSSIAN) {
     // sine-Gaussian: the bin of the centre frequency, so that the points of a
     // warp walk their Gaussians (k_mixed_sg) over runs of nearly equal length
@@ -57,10 +63,13 @@ __device__ __forceinline__ int order_key(const LaunchArgs& a, const PointRec& r)
 // ---------------------------------------------------------------------------
 // frac(x + lo) as a 64-bit fraction, |lo| < 1/2
 __device__ __forceinline__ uint64_t to_wide(double x, double lo) {
-  double fr = ldexp(x - floor(x), 64);
+  double fr = (x - floor(x)) * 18446744073709551616.0;  // 2^64: exact
   if (!(fr >= 0.0 && fr < 18446744073709551616.0)) fr = 0.0;
-  return (uint64_t)fr + (uint64_t)(int64_t)ldexp(lo, 64);
+  return (uint64_t)fr + (uint64_t)(int64_t)(lo * 18446744073709551616.0);
 }
+
+// 2^e as a double, -1022 <= e <= 1023
+__device__ __forceinline__ double two_to(int e) { return __hiloint2double((1023 + e) << 20, 0); }
 
 // frac(dt df) in cycles per bin
 __device__ __forceinline__ uint64_t wide_shift(const LaunchArgs& a, double dt) {
@@ -68,8 +77,9 @@ __device__ __forceinline__ uint64_t wide_shift(const LaunchArgs& a, double dt) {
   return to_wide(v, fma(dt, a.step, -v) + dt * a.step_lo);
 }
 
-__device__ __noinline__ void wide_coefficients(const LaunchArgs& a, const PointRec& r, int64_t i, double m1, double m2,
-                                               const double* c, double cconst) {
+__device__ __forceinline__ void wide_coefficients(const LaunchArgs& a, int64_t i, double m1, double m2, double eta,
+                                                  double m_sec, double u, double f_isco, int64_t k_end, const double* pn,
+                                                  const double* c, double cconst) {
   uint64_t* w = a.wide_c + i;
   // c_0 = 3 / (128 eta) (pi M)^(-5/3) / (2 pi) = K M^(1/3) / (m1 m2) to twice
   // float64's digits: its relative error is the same in every bin, where the
@@ -79,15 +89,15 @@ __device__ __noinline__ void wide_coefficients(const LaunchArgs& a, const PointR
   const double y = cbrt(m), p = y * y, pe = fma(y, y, -p), t = p * y, te = fma(p, y, -t) + pe * y;
   const double yl = ((m - t) - te + ml) / (3.0 * p);
   const double nh = kh * y, nl = fma(kh, y, -nh) + (kh * yl + kl * y);
-  const double dh = m1 * m2, dl = fma(m1, m2, -dh);
-  const double q0 = nh / dh, q1 = (fma(-q0, dh, nh) + (nl - q0 * dl)) / dh;
+  const double dh = m1 * m2, dl = fma(m1, m2, -dh), id = 1.0 / dh;
+  const double q0 = nh * id, q1 = (fma(-q0, dh, nh) + (nl - q0 * dl)) * id;
   // the others as the mixed kernels have them, u = (pi M)^(1/3); ln f relative to wide_lnref
   double x[kNumBasis], xl = q1;
   x[0] = q0;
-  const double P = 3.0 / (128.0 * r.eta) / kTwoPi, pm = kPi * r.m_sec, u = cbrt(pm);
-  x[1] = P * r.a[2] / pm;
-  x[2] = P * r.a[3] * u / pm;
-  x[3] = P * r.a[4] / u;
+  const double P = 3.0 / (128.0 * eta * kTwoPi), ip = P / (kPi * m_sec);
+  x[1] = ip * pn[2];
+  x[2] = ip * pn[3] * u;
+  x[3] = ip * pn[4] * u * u;
   x[4] = c[4];
   x[5] = c[5] + c[6] * a.wide_lnref;
   x[6] = c[6];
@@ -101,30 +111,27 @@ __device__ __noinline__ void wide_coefficients(const LaunchArgs& a, const PointR
   }
   xl *= a.wide_scale[0];
   const int s = top > 1.0 && isfinite(top) ? min(ilogb(top) + 1, 58) : 1;
+  const double f = two_to(58 - s);
 #pragma unroll
   for (int b = 0; b < kNumBasis; ++b) {
-    const int64_t n = __double2ll_rn(ldexp(x[b], 58 - s)) + (b == 0 ? __double2ll_rn(ldexp(xl, 58 - s)) : 0);
+    const int64_t n = __double2ll_rn(x[b] * f) + (b == 0 ? __double2ll_rn(xl * f) : 0);
     w[(int64_t)b * a.B] = ((uint64_t)(uint32_t)(int32_t)(n >> 27) << 32) | (uint32_t)(n & 0x7ffffff);
   }
   w[(int64_t)kNumBasis * a.B] = to_wide(cconst + c[4] * a.wide_lnref, 0.0);
   w[(int64_t)(kNumBasis + 1) * a.B] = (uint64_t)(s + 2);
-  for (int d = 0; d < a.n_det; ++d) {
-    w[(int64_t)(kNumBasis + 2 + d) * a.B] = wide_shift(a, r.dt[d]);
-    w[(int64_t)(kNumBasis + 2 + kMaxDet + d) * a.B] = ((uint64_t)r.qfix[d][1] << 32) | r.qfix[d][0];
-  }
   // a list's frequencies may lie beyond the grid's last
-  int64_t ke = r.k_end;
-  if (ke >= a.n_bins) ke = max(ke, (int64_t)fmin(ceil(r.f_isco / a.step), 9e15));
+  int64_t ke = k_end;
+  if (ke >= a.n_bins) ke = max(ke, (int64_t)fmin(ceil(f_isco / a.step), 9e15));
   w[(int64_t)kWideEnd * a.B] = (uint64_t)ke;
 }
 
 // ... and of gwl_wide_sg.cu: the centre frequency in bins, sqrt(y) = Q sqrt(log2 e
-// / 2) / f0 per bin to twice float64's digits, the bins to visit, the shifts and
-// arg(Fp P + i Fx X).
-__device__ __noinline__ void wide_coefficients_sg(const LaunchArgs& a, PointRec& r, int64_t i, double Q) {
+// / 2) / f0 per bin to twice float64's digits, and the bins to visit.
+__device__ __forceinline__ void wide_coefficients_sg(const LaunchArgs& a, int64_t i, double Q, double f0, int64_t& k_start,
+                                                     int64_t& k_end) {
   uint64_t* w = a.wide_c + i;
   const double ch = 0.8493218002880191, cl = -2.5959464104597403e-17;
-  double q0 = r.sg_f0 / a.step, q1 = (fma(-q0, a.step, r.sg_f0) - q0 * a.step_lo) / a.step;
+  double q0 = f0 / a.step, q1 = (fma(-q0, a.step, f0) - q0 * a.step_lo) / a.step;
   const double nh = fabs(Q) * ch, nl = fma(fabs(Q), ch, -nh) + fabs(Q) * cl;
   double s0 = nh / q0, s1 = (fma(-s0, q0, nh) + (nl - s0 * q1)) / q0;
   const double far = q0 * 3.469446951953614e-18;  // beyond 2^58 bins f - f0 = -f0 in float64 too
@@ -134,7 +141,7 @@ __device__ __noinline__ void wide_coefficients_sg(const LaunchArgs& a, PointRec&
     s0 *= far;
     s1 *= far;
   }
-  r.k_start = r.k_end = 0;
+  k_start = k_end = 0;
   if (!(q0 > 0.0 && isfinite(far) && s0 > 0.0 && isfinite(s0))) q0 = s0 = 1.0, q1 = s1 = 0.0;  // (an invalid point)
   const int frac = 61 - ilogb(q0 + (double)a.n_bins + 2.0), es = ilogb(s0) + 1;
   const uint64_t sm = (uint64_t)ldexp(s0, 64 - es), sv = sm + (uint64_t)(int64_t)ldexp(s1, 64 - es);
@@ -147,215 +154,308 @@ __device__ __noinline__ void wide_coefficients_sg(const LaunchArgs& a, PointRec&
   const double lo = (double)a.k_lo, hi = (double)(a.k_hi - 1), x = fmax(0.0, fmax(lo - q0, q0 - hi)), y = s0 * x * (s0 * x);
   if (y < 1020.0) {
     const double R = sqrt(fmin(y + 100.0, 1020.0)) / s0;
-    r.k_start = (int64_t)fmin(fmax(ceil(q0 - R), lo), hi);
-    r.k_end = (int64_t)fmin(fmax(floor(q0 + R), lo), hi) + 1;
-  }
-  for (int d = 0; d < a.n_det; ++d) {
-    w[(int64_t)(kNumBasis + 2 + d) * a.B] = wide_shift(a, r.dt[d]);
-    w[(int64_t)(kNumBasis + 2 + kMaxDet + d) * a.B] = to_wide(atan2(r.fx[d] * r.amp2, r.fp[d] * r.amp) / kTwoPi, 0.0);
+    k_start = (int64_t)fmin(fmax(ceil(q0 - R), lo), hi);
+    k_end = (int64_t)fmin(fmax(floor(q0 + R), lo), hi) + 1;
   }
 }
 
 // ---------------------------------------------------------------------------
 // prologue: per-point float64 set-up (sky frame, antenna, delays, model scalars)
 // ---------------------------------------------------------------------------
-__device__ __noinline__ void prologue_point(const LaunchArgs& a, int64_t i) {
-  PointRec r;
-  memset(&r, 0, sizeof(r));
-  const double ra = par(a, GWL_P_RA, i), dec = par(a, GWL_P_DEC, i), psi = par(a, GWL_P_PSI, i);
-  double tgeo = par(a, GWL_P_GEOCENT_TIME, i);
-  r.jitter = a.time_marg && a.jitter ? par(a, GWL_P_TIME_JITTER, i) : 0.0;
-  // base.py:427-428: the jitter is added to geocent_time before projection.
-  tgeo = tgeo + r.jitter;
-  const double gmst = pymod(gmst_radians(tgeo), kTwoPi);
-  bool ok = isfinite(ra) && isfinite(dec) && isfinite(psi) && isfinite(tgeo);
-  const SkyTrig sky = sky_trig(ra, dec, psi, gmst);
-  // an interferometer reference time (multiband.py:724-725, interferometer.py:333-336)
-  // fixes the time of the antenna patterns; the delay stays at geocent_time
-  const SkyTrig sky_ant =
-      a.antenna_fixed ? sky_trig(ra, dec, psi, pymod(gmst_radians(a.antenna_time), kTwoPi)) : sky;
-  for (int d = 0; d < a.n_det; ++d) {
-    double fp, fx, delay;
-    antenna_and_delay(a.det[d].tensor, a.det[d].vertex, sky, &fp, &fx, &delay);
-    double delay_ref = delay;
-    if (a.antenna_fixed) antenna_and_delay(a.det[d].tensor, a.det[d].vertex, sky_ant, &fp, &fx, &delay_ref);
-    r.fp[d] = fp;
-    r.fx[d] = fx;
-    // interferometer.py:355-358: subtract the two GPS times first, then add the delay.
-    const double dt_geocent = tgeo - a.det[d].start_time;
-    // ROQ with time marginalisation: the delay at the antenna time alone (roq.py:529-541)
-    r.dt[d] = a.roq_tm ? delay_ref : dt_geocent + delay;
-    // frac(dt * df) in cycles per bin as 0.64 fixed point, so that the phase
-    // 2 pi f_k dt = 2 pi k (dt df) reduces exactly modulo one cycle.
-    const double x = r.dt[d] * a.step;
-    const double frac = x - floor(x);
-    double scaled = ldexp(frac, 64);
-    if (!(scaled < 18446744073709551616.0)) scaled = 0.0;
-    const unsigned long long u = (unsigned long long)scaled;
-    r.xfix[d][0] = (uint32_t)(u & 0xffffffffull);
-    r.xfix[d][1] = (uint32_t)(u >> 32);
+// A CTA of four warps sets up 32 points, lane = point: the warps share out the
+// float64 chains of a point, in three steps with a barrier between them.
+//   1. sidereal time and hour angle | the other angles | the source's scalars and
+//      band | the phase coefficients
+//   2. warp d: detector d; the last warp also the phase basis coefficients
+//   3. the error bound, the ordering key, the time marginalisation's scalars
+// One thread per point took 38 us (sine-Gaussian) to 76 us (float64 TaylorF2) for
+// a single point and for thousands alike: the latency of one float64 chain.
+constexpr int kProloguePoints = 32;
+constexpr int kPrologueWarps = 4;
+
+struct PrologueShared {
+  double sphi[kProloguePoints], cphi[kProloguePoints], sth[kProloguePoints], cth[kProloguePoints];
+  double sps[kProloguePoints], cps[kProloguePoints], sphi_ant[kProloguePoints], cphi_ant[kProloguePoints];
+  double cos_i[kProloguePoints], amp[kProloguePoints], amp2[kProloguePoints];
+  double u[kProloguePoints], lnu[kProloguePoints], f_isco[kProloguePoints], hh[kMaxDet][kProloguePoints];
+  double qabs[kMaxDet][kProloguePoints], pn[8][kProloguePoints], pl[8][kProloguePoints];
+  int64_t k_start[kProloguePoints], k_end[kProloguePoints];
+  int ok[2][kProloguePoints];
+};
+
+__device__ __forceinline__ void put_fixed(uint32_t* out, uint64_t u) {
+  out[0] = (uint32_t)(u & 0xffffffffull);
+  out[1] = (uint32_t)(u >> 32);
+}
+
+// frac(x) as 0.64 fixed point
+__device__ __forceinline__ uint64_t fixed_fraction(double x) {
+  double scaled = (x - floor(x)) * 18446744073709551616.0;
+  if (!(scaled < 18446744073709551616.0)) scaled = 0.0;
+  return (uint64_t)scaled;
+}
+
+__device__ __forceinline__ void prologue_detector(const LaunchArgs& a, PrologueShared& sh, PointRec& r, int64_t i, int t, int d,
+                                                  double tgeo, bool tf2) {
+  const SkyTrig sky{sh.sphi[t], sh.cphi[t], sh.sth[t], sh.cth[t], sh.sps[t], sh.cps[t]};
+  double fp, fx, delay, delay_ref;
+  antenna_and_delay(a.det[d].tensor, a.det[d].vertex, sky, &fp, &fx, &delay);
+  delay_ref = delay;
+  if (a.antenna_fixed) {
+    const SkyTrig ant{sh.sphi_ant[t], sh.cphi_ant[t], sh.sth[t], sh.cth[t], sh.sps[t], sh.cps[t]};
+    antenna_and_delay(a.det[d].tensor, a.det[d].vertex, ant, &fp, &fx, &delay_ref);
   }
-  if (a.model == GWL_MODEL_SINEGAUSSIAN) {
-    // bilby/gw/source.py:1197-1207
-    const double hrss = par(a, GWL_P_HRSS, i), Q = par(a, GWL_P_Q, i), f0 = par(a, GWL_P_FREQUENCY, i);
-    const double tau = Q / (1.4142135623730951 * kPi * f0);
-    const double temp = Q / (4.0 * 1.7724538509055159 * f0);
-    r.a[0] = hrss * 1.7724538509055159 * tau / 2;          // plus and cross prefactor
-    r.a[1] = sqrt(temp * (1 + exp(-Q * Q)));                // plus denominator
-    r.a[2] = sqrt(temp * (1 - exp(-Q * Q)));                // cross denominator
-    r.a[3] = tau * tau;
-    r.sg_f0 = f0;
-    r.sg_a = 9.869604401089358 * tau * tau;  // pi^2 tau^2 for the mixed kernel
-    r.amp = r.a[0] / r.a[1];
-    r.amp2 = r.a[0] / r.a[2];
-    ok = ok && isfinite(r.amp) && isfinite(r.amp2) && isfinite(r.sg_a) && f0 > 0;
-    if (a.wide_c) wide_coefficients_sg(a, r, i, Q);
-  } else {
-    const double m1 = par(a, GWL_P_MASS_1, i), m2 = par(a, GWL_P_MASS_2, i);
-    const double chi1 = par(a, GWL_P_CHI_1, i), chi2 = par(a, GWL_P_CHI_2, i);
-    const double dl = par(a, GWL_P_LUMINOSITY_DISTANCE, i);
-    const double theta_jn = par(a, GWL_P_THETA_JN, i), phase = par(a, GWL_P_PHASE, i);
-    const double m = m1 + m2;
-    r.m_sec = m * kMtsunSI;
-    r.eta = m1 * m2 / (m * m);
-    r.f_isco = 1.0 / (6.0 * sqrt(6.0) * kPi * r.m_sec);
-    r.dist = dl;
-    // Mc^(5/6) = eta^(1/2) M^(5/6) and M^(5/6) = M (cbrt(pi) / u)^(1/2) with u = (pi M)^(1/3)
-    const double u = cbrt(kPi * r.m_sec);
-    const double mc56 = sqrt(r.eta) * r.m_sec * sqrt(1.4645918875615231 / u);
-    // sqrt(5/24) pi^(-2/3)
-    r.amp = 0.45643546458763845 * 0.46619407703541166 * mc56 * kSpeedOfLight / (dl * 1e6 * kPcSI);
-    r.cos_i = cos(theta_jn);
-    r.phase = phase;
+  r.fp[d] = fp;
+  r.fx[d] = fx;
+  // interferometer.py:355-358: subtract the two GPS times first, then add the delay.
+  const double dt_geocent = tgeo - a.det[d].start_time;
+  // ROQ with time marginalisation: the delay at the antenna time alone (roq.py:529-541)
+  const double dt = a.roq_tm ? delay_ref : dt_geocent + delay;
+  r.dt[d] = dt;
+  // frac(dt * df) in cycles per bin as 0.64 fixed point, so that the phase
+  // 2 pi f_k dt = 2 pi k (dt df) reduces exactly modulo one cycle.
+  put_fixed(r.xfix[d], fixed_fraction(dt * a.step));
+  if (a.wide_c) a.wide_c[(int64_t)(kNumBasis + 2 + d) * a.B + i] = wide_shift(a, dt);
+  const bool tm = a.time_marg && a.precision == GWL_PRECISION_MIXED && a.n_fft > 0 && !a.relbin && !a.mb_tm && !a.roq;
+  const double norm = 4.0 / a.duration;
+  if (tf2) {
     // Re <d|h>_d = |Q_d| Re sum w e^{i (phase_k + alpha_d)}, alpha_d = arg(conj(Q_d)): the real-part
-    // kernel carries alpha_d as a constant phase offset of detector d
-    for (int d = 0; d < a.n_det; ++d) {
-      const double qr = r.fp[d] * (1.0 + r.cos_i * r.cos_i) / 2.0, qi = -r.fx[d] * r.cos_i;
-      r.qabs[d] = hypot(qr, qi);
-      uint64_t u = 0;
-      if (!a.cplx) {
-        const double x = atan2(-qi, qr) / kTwoPi;
-        double scaled = ldexp(x - floor(x), 64);
-        if (!(scaled < 18446744073709551616.0)) scaled = 0.0;
-        u = (uint64_t)scaled;
-      }
-      r.qfix[d][0] = (uint32_t)(u & 0xffffffffull);
-      r.qfix[d][1] = (uint32_t)(u >> 32);
+    // kernels carry alpha_d as a constant phase offset of detector d
+    const double ci = sh.cos_i[t], amp = sh.amp[t];
+    const double qr = fp * (1.0 + ci * ci) / 2.0, qi = -fx * ci, qabs = hypot(qr, qi);
+    r.qabs[d] = qabs;
+    sh.qabs[d][t] = qabs;
+    const uint64_t u = a.cplx ? 0ull : fixed_fraction(atan2(-qi, qr) / kTwoPi);
+    put_fixed(r.qfix[d], u);
+    if (a.wide_c) a.wide_c[(int64_t)(kNumBasis + 2 + kMaxDet + d) * a.B + i] = u;
+    if (tm) {
+      const double s = norm * amp * a.w_scale[d];
+      r.tm_coef[2 * d] = (float)(s * fp * (1.0 + ci * ci) / 2.0);
+      r.tm_coef[2 * d + 1] = (float)(-s * fx * ci);
+      const int64_t k1 = min(sh.k_end[t], a.n_bins), k0 = min(sh.k_start[t], k1);
+      sh.hh[d][t] = norm * amp * amp * (qr * qr + qi * qi) * (a.hh_prefix[d][k1] - a.hh_prefix[d][k0]);
     }
-    taylorf2_coefficients(m1, m2, chi1, chi2, r.a, r.l);
-    ok = ok && m1 > 0 && m2 > 0 && dl > 0 && isfinite(r.amp) && isfinite(phase) && isfinite(chi1) &&
-         isfinite(chi2);
-    // band [k_start, k_end): f >= minimum_frequency and f < f_isco; k_end is
-    // the first k with freq[k] >= f_isco: guessed from the uniform grid and
-    // corrected against the frequency array (binary search if that fails)
-    int64_t ke = (int64_t)fmin(fmax(ceil(r.f_isco / a.step), 0.0), (double)a.n_bins);
-    for (int q = 0; q < 4 && ke > 0 && a.freq[ke - 1] >= r.f_isco; ++q) --ke;
-    for (int q = 0; q < 4 && ke < a.n_bins && a.freq[ke] < r.f_isco; ++q) ++ke;
-    if ((ke > 0 && a.freq[ke - 1] >= r.f_isco) || (ke < a.n_bins && a.freq[ke] < r.f_isco)) {
-      int64_t lo = 0, hi = a.n_bins;
-      while (lo < hi) {
-        const int64_t mid = (lo + hi) / 2;
-        if (a.freq[mid] >= r.f_isco) hi = mid; else lo = mid + 1;
-      }
-      ke = lo;
-    }
-    r.k_end = ke;
-    r.k_start = a.k_fmin;
-    // Psi / (2 pi) = sum_b c_b phi_b(f) + c_const with v = u f^(1/3), u = (pi M)^(1/3)
-    const double P = 3.0 / (128.0 * r.eta) / kTwoPi;
-    const double lnu = log(u);
-    double c[kNumBasis];
-    c[0] = P * r.a[0] / (u * u * u * u * u);   // f^(-5/3)
-    c[1] = P * r.a[2] / (u * u * u);           // f^(-1)
-    c[2] = P * r.a[3] / (u * u);               // f^(-2/3)
-    c[3] = P * r.a[4] / u;                     // f^(-1/3)
-    c[4] = P * r.l[5] / 3.0;                   // ln f
-    c[5] = P * (r.a[6] + r.l[6] * lnu) * u;    // f^(1/3)
-    c[6] = P * r.l[6] / 3.0 * u;               // f^(1/3) ln f
-    c[7] = P * r.a[7] * u * u;                 // f^(2/3)
-    const double cconst = P * (r.a[5] + r.l[5] * lnu) + (-2.0 * phase - kPi / 4) / kTwoPi;
-    for (int b = 0; b < kNumBasis; ++b) {
-      const ff s = ff_from_double(c[b]);
-      r.c_hi[b] = s.hi;
-      r.c_lo[b] = s.lo;
-    }
-    const ff s = ff_from_double(cconst - floor(cconst));
-    r.c_hi[kNumBasis] = s.hi;
-    r.c_lo[kNumBasis] = s.lo;
-    if (a.wide_c) wide_coefficients(a, r, i, m1, m2, c, cconst);
-  }
-  r.valid = ok ? 1 : 0;
-  if (a.rf_tol > 0 && a.rf_count && r.valid && a.model == GWL_MODEL_TAYLORF2) {
-    // error bound of the fast mixed-precision sums (kRefineL2): norms of the
-    // per-bin terms |<d|h>_k| = 4/T A0 |Q_d| f^(-7/6) |d_k| / S_k over the band
-    const int64_t k1 = min(r.k_end, a.n_bins), k0 = min(r.k_start, k1);
-    double l2 = 0.0, l1 = 0.0;
-    for (int d = 0; d < a.n_det; ++d) {
-      const double s = 4.0 / a.duration * a.w_scale[d] * r.amp * r.qabs[d];
-      l2 += s * s * (a.rf_p2[d][k1] - a.rf_p2[d][k0]);
-      l1 += s * (a.rf_p1[d][k1] - a.rf_p1[d][k0]);
-    }
-    // (times the distance slope bound: the lnL's change per unit <d|h>)
-    const double slope = a.dist_slope > 1.0 ? a.dist_slope : 1.0;
-    if (slope * (kRefineL2 * sqrt(fmax(l2, 0.0)) + kRefineL1 * l1) > a.rf_tol) {
-      r.refine = 1;
-      atomicAdd(a.rf_count, 1);
-      if (a.rf_total) atomicAdd(a.rf_total, 1);
+  } else {
+    const double A = fp * sh.amp[t], C = fx * sh.amp2[t];
+    if (a.wide_c) a.wide_c[(int64_t)(kNumBasis + 2 + kMaxDet + d) * a.B + i] = to_wide(atan2(C, A) / kTwoPi, 0.0);
+    if (tm) {
+      r.tm_coef[2 * d] = (float)(norm * a.w_scale[d] * fp * sh.amp[t]);
+      r.tm_coef[2 * d + 1] = (float)(norm * a.w_scale[d] * fx * sh.amp2[t]);
+      sh.hh[d][t] = 0.0;
     }
   }
-  if (a.time_marg && a.precision == GWL_PRECISION_MIXED && a.n_fft > 0 && !a.relbin && !a.mb_tm && !a.roq) {
+}
+
+// (not inlined: one compiled body for one and for several analyses, so that a point
+// has the same bits in both)
+__device__ __noinline__ void prologue_cta(const LaunchArgs& a, PrologueShared& sh, int64_t i, bool have) {
+  const int t = threadIdx.x % kProloguePoints, role = threadIdx.x / kProloguePoints;
+  const bool tf2 = a.model != GWL_MODEL_SINEGAUSSIAN;
+  PointRec& r = a.rec[i];
+  // base.py:427-428: the jitter is added to geocent_time before projection.
+  const double jitter = have && a.time_marg && a.jitter ? par(a, GWL_P_TIME_JITTER, i) : 0.0;
+  const double tgeo = have ? par(a, GWL_P_GEOCENT_TIME, i) + jitter : 0.0;
+  if (have) {
+    if (role == 0) {
+      const double ra = par(a, GWL_P_RA, i);
+      sincos(ra - mod_two_pi(gmst_radians(tgeo)), &sh.sphi[t], &sh.cphi[t]);
+      // an interferometer reference time (multiband.py:724-725, interferometer.py:333-336)
+      // fixes the time of the antenna patterns; the delay stays at geocent_time
+      if (a.antenna_fixed)
+        sincos(ra - mod_two_pi(gmst_radians(a.antenna_time)), &sh.sphi_ant[t], &sh.cphi_ant[t]);
+      sh.ok[0][t] = isfinite(ra) && isfinite(par(a, GWL_P_DEC, i)) && isfinite(par(a, GWL_P_PSI, i)) && isfinite(tgeo);
+      r.jitter = jitter;
+      r.refine = 0;
+    } else if (role == 1) {
+      sincos(kPi / 2 - par(a, GWL_P_DEC, i), &sh.sth[t], &sh.cth[t]);
+      sincos(par(a, GWL_P_PSI, i), &sh.sps[t], &sh.cps[t]);
+      if (tf2) sh.cos_i[t] = r.cos_i = cos(par(a, GWL_P_THETA_JN, i));
+    } else if (role == 2 && !tf2) {
+      // bilby/gw/source.py:1197-1207
+      const double hrss = par(a, GWL_P_HRSS, i), Q = par(a, GWL_P_Q, i), f0 = par(a, GWL_P_FREQUENCY, i);
+      const double tau = Q / (1.4142135623730951 * kPi * f0);
+      const double temp = Q / (4.0 * 1.7724538509055159 * f0), eq = exp(-Q * Q);
+      const double a0 = hrss * 1.7724538509055159 * tau / 2;  // plus and cross prefactor
+      const double a1 = sqrt(temp * (1 + eq));                // plus denominator
+      const double a2 = sqrt(temp * (1 - eq));                // cross denominator
+      const double sg_a = 9.869604401089358 * tau * tau;      // pi^2 tau^2 for the mixed kernel
+      const double amp = a0 / a1, amp2 = a0 / a2;
+      r.a[0] = a0;
+      r.a[1] = a1;
+      r.a[2] = a2;
+      r.a[3] = tau * tau;
+      r.sg_f0 = f0;
+      r.sg_a = sg_a;
+      r.amp = amp;
+      r.amp2 = amp2;
+      r.dist = 0.0;
+      sh.amp[t] = amp;
+      sh.amp2[t] = amp2;
+      sh.ok[1][t] = isfinite(amp) && isfinite(amp2) && isfinite(sg_a) && f0 > 0;
+    } else if (role == 3 && !tf2) {
+      int64_t k0 = 0, k1 = 0;
+      if (a.wide_c) wide_coefficients_sg(a, i, par(a, GWL_P_Q, i), par(a, GWL_P_FREQUENCY, i), k0, k1);
+      r.k_start = sh.k_start[t] = k0;
+      r.k_end = sh.k_end[t] = k1;
+    } else if (role == 2) {
+      const double m1 = par(a, GWL_P_MASS_1, i), m2 = par(a, GWL_P_MASS_2, i), dl = par(a, GWL_P_LUMINOSITY_DISTANCE, i);
+      const double phase = par(a, GWL_P_PHASE, i), m = m1 + m2, m_sec = m * kMtsunSI, eta = m1 * m2 / (m * m);
+      const double f_isco = 1.0 / (6.0 * sqrt(6.0) * kPi * m_sec);
+      // band [k_start, k_end): f >= minimum_frequency and f < f_isco; k_end is
+      // the first k with freq[k] >= f_isco: guessed from the uniform grid and
+      // corrected against the frequency array (binary search if that fails)
+      int64_t ke = (int64_t)fmin(fmax(ceil(f_isco / a.step), 0.0), (double)a.n_bins);
+      for (int q = 0; q < 4 && ke > 0 && a.freq[ke - 1] >= f_isco; ++q) --ke;
+      for (int q = 0; q < 4 && ke < a.n_bins && a.freq[ke] < f_isco; ++q) ++ke;
+      if ((ke > 0 && a.freq[ke - 1] >= f_isco) || (ke < a.n_bins && a.freq[ke] < f_isco)) {
+        int64_t lo = 0, hi = a.n_bins;
+        while (lo < hi) {
+          const int64_t mid = (lo + hi) / 2;
+          if (a.freq[mid] >= f_isco) hi = mid; else lo = mid + 1;
+        }
+        ke = lo;
+      }
+      r.k_end = sh.k_end[t] = ke;
+      r.k_start = sh.k_start[t] = a.k_fmin;
+      r.m_sec = m_sec;
+      r.eta = eta;
+      r.f_isco = sh.f_isco[t] = f_isco;
+      r.dist = dl;
+      r.phase = phase;
+      // Mc^(5/6) = eta^(1/2) M^(5/6) and M^(5/6) = M (cbrt(pi) / u)^(1/2) with u = (pi M)^(1/3)
+      const double u = cbrt(kPi * m_sec);
+      const double mc56 = sqrt(eta) * m_sec * sqrt(1.4645918875615231 / u);
+      // sqrt(5/24) pi^(-2/3)
+      const double amp = 0.45643546458763845 * 0.46619407703541166 * mc56 * kSpeedOfLight / (dl * 1e6 * kPcSI);
+      r.amp = sh.amp[t] = amp;
+      sh.u[t] = u;
+      sh.lnu[t] = log(u);
+      sh.ok[1][t] = m1 > 0 && m2 > 0 && dl > 0 && isfinite(amp) && isfinite(phase) &&
+                    isfinite(par(a, GWL_P_CHI_1, i)) && isfinite(par(a, GWL_P_CHI_2, i));
+    } else {
+      double pn[8], pl[8];
+      taylorf2_coefficients(par(a, GWL_P_MASS_1, i), par(a, GWL_P_MASS_2, i), par(a, GWL_P_CHI_1, i),
+                            par(a, GWL_P_CHI_2, i), pn, pl);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        r.a[k] = sh.pn[k][t] = pn[k];
+        r.l[k] = sh.pl[k][t] = pl[k];
+      }
+    }
+  }
+  __syncthreads();
+  if (have) {
+    for (int d = role; d < a.n_det; d += kPrologueWarps) prologue_detector(a, sh, r, i, t, d, tgeo, tf2);
+    if (role == kPrologueWarps - 1 && tf2) {
+      const double m1 = par(a, GWL_P_MASS_1, i), m2 = par(a, GWL_P_MASS_2, i), phase = par(a, GWL_P_PHASE, i);
+      const double m = m1 + m2, m_sec = m * kMtsunSI, eta = m1 * m2 / (m * m), u = sh.u[t], lnu = sh.lnu[t];
+      double pn[8], l5 = sh.pl[5][t], l6 = sh.pl[6][t];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) pn[k] = sh.pn[k][t];
+      // Psi / (2 pi) = sum_b c_b phi_b(f) + c_const with v = u f^(1/3), u = (pi M)^(1/3)
+      const double P = 3.0 / (128.0 * eta) / kTwoPi;
+      double c[kNumBasis];
+      c[0] = P * pn[0] / (u * u * u * u * u);   // f^(-5/3)
+      c[1] = P * pn[2] / (u * u * u);           // f^(-1)
+      c[2] = P * pn[3] / (u * u);               // f^(-2/3)
+      c[3] = P * pn[4] / u;                     // f^(-1/3)
+      c[4] = P * l5 / 3.0;                      // ln f
+      c[5] = P * (pn[6] + l6 * lnu) * u;        // f^(1/3)
+      c[6] = P * l6 / 3.0 * u;                  // f^(1/3) ln f
+      c[7] = P * pn[7] * u * u;                 // f^(2/3)
+      const double cconst = P * (pn[5] + l5 * lnu) + (-2.0 * phase - kPi / 4) / kTwoPi;
+      if (a.precision == GWL_PRECISION_MIXED) {
+#pragma unroll
+        for (int b = 0; b < kNumBasis; ++b) {
+          const ff s = ff_from_double(c[b]);
+          r.c_hi[b] = s.hi;
+          r.c_lo[b] = s.lo;
+        }
+        const ff s = ff_from_double(cconst - floor(cconst));
+        r.c_hi[kNumBasis] = s.hi;
+        r.c_lo[kNumBasis] = s.lo;
+      }
+      if (a.wide_c)
+        wide_coefficients(a, i, m1, m2, eta, m_sec, u, sh.f_isco[t], sh.k_end[t], pn, c, cconst);
+    }
+  }
+  __syncthreads();
+  if (!have) return;
+  const bool tm = a.time_marg && a.precision == GWL_PRECISION_MIXED && a.n_fft > 0 && !a.relbin && !a.mb_tm && !a.roq;
+  if (role == 0) {
+    const int valid = sh.ok[0][t] && sh.ok[1][t];
+    int refine = 0;
+    if (a.rf_tol > 0 && a.rf_count && valid && a.model == GWL_MODEL_TAYLORF2) {
+      // error bound of the fast mixed-precision sums (kRefineL2): norms of the
+      // per-bin terms |<d|h>_k| = 4/T A0 |Q_d| f^(-7/6) |d_k| / S_k over the band
+      const int64_t k1 = min(sh.k_end[t], a.n_bins), k0 = min(sh.k_start[t], k1);
+      double l2 = 0.0, l1 = 0.0;
+      for (int d = 0; d < a.n_det; ++d) {
+        const double s = 4.0 / a.duration * a.w_scale[d] * sh.amp[t] * sh.qabs[d][t];
+        l2 += s * s * (a.rf_p2[d][k1] - a.rf_p2[d][k0]);
+        l1 += s * (a.rf_p1[d][k1] - a.rf_p1[d][k0]);
+      }
+      // (times the distance slope bound: the lnL's change per unit <d|h>)
+      const double slope = a.dist_slope > 1.0 ? a.dist_slope : 1.0;
+      if (slope * (kRefineL2 * sqrt(fmax(l2, 0.0)) + kRefineL1 * l1) > a.rf_tol) {
+        refine = 1;
+        atomicAdd(a.rf_count, 1);
+        if (a.rf_total) atomicAdd(a.rf_total, 1);
+      }
+    }
+    r.valid = valid;
+    r.refine = refine;
+    if (a.order_hist) {
+      OrderPoint o{valid, refine, sh.k_start[t], sh.k_end[t], tf2 ? 0.0 : par(a, GWL_P_FREQUENCY, i)};
+      atomicAdd(&a.order_hist[order_key(a, o)], 1);
+    }
+  } else if (tm && role == 1) {
     // the mixed full-grid time-marginalised kernel's per-point scalars:
     // integrand coefficients, the TaylorF2 <h|h> and the exact sample window
-    const double norm = 4.0 / a.duration;
     double hh = 0.0;
-    for (int d = 0; d < a.n_det; ++d) {
-      if (a.model == GWL_MODEL_TAYLORF2) {
-        const double ci = r.cos_i;
-        const double s = norm * r.amp * a.w_scale[d];
-        r.tm_coef[2 * d] = (float)(s * r.fp[d] * (1.0 + ci * ci) / 2.0);
-        r.tm_coef[2 * d + 1] = (float)(-s * r.fx[d] * ci);
-        const double qr = r.fp[d] * (1.0 + ci * ci) / 2.0, qi = -r.fx[d] * ci;
-        const int64_t k1 = min(r.k_end, a.n_bins), k0 = min(r.k_start, k1);
-        hh += norm * r.amp * r.amp * (qr * qr + qi * qi) * (a.hh_prefix[d][k1] - a.hh_prefix[d][k0]);
-      } else {
-        r.tm_coef[2 * d] = (float)(norm * a.w_scale[d] * r.fp[d] * r.amp);
-        r.tm_coef[2 * d + 1] = (float)(norm * a.w_scale[d] * r.fx[d] * r.amp2);
-      }
-    }
+    for (int d = 0; d < a.n_det; ++d) hh += sh.hh[d][t];
     r.tm_hh = hh;
-    if (a.model == GWL_MODEL_TAYLORF2 && a.dist_marg) {
+    if (tf2 && a.dist_marg) {
       // the distance spline's row at this point's <h|h> (base.py:775-784)
-      const double sr = r.dist * a.inv_ref_dist;
+      const double sr = par(a, GWL_P_LUMINOSITY_DISTANCE, i) * a.inv_ref_dist;
       const SplineRowF row = bicubic_row_f(a.ty_f, a.ny, a.bbox, (float)(hh * sr * sr));
       r.tm_row_ly = row.Ly;
       r.tm_row_in = row.inside;
       for (int q = 0; q < 4; ++q) r.tm_row_hy[q] = row.hy[q];
     }
+  } else if (tm && role >= 2) {
     // samples j with t_j = start + (j + 1) T / L + jitter inside [t_min, t_max]
     // (base.py:1027-1035), tested as the float64 kernel tests them; t_j
-    // increases with j
+    // increases with j: a guess from the spacing, corrected (binary search if
+    // that fails)
     const int64_t L = a.n_fft;
-    int64_t lo = 0, hi = L;
-    while (lo < hi) {
-      const int64_t mid = (lo + hi) / 2;
-      if (tm_sample_time(a, mid, L, a.tm_step, r.jitter) >= a.t_min) hi = mid; else lo = mid + 1;
+    const bool first = role == 2;
+    const double bound = first ? a.t_min : a.t_max;
+    // first j with t_j >= t_min, or first with t_j > t_max
+    const auto past = [&](int64_t j) {
+      const double x = tm_sample_time(a, j, L, a.tm_step, jitter);
+      return first ? x >= bound : !(x <= bound);
+    };
+    int64_t j = (int64_t)fmin(fmax((bound - a.start_time0 - jitter) * a.tm_inv_step - 1.0, 0.0), (double)L);
+    for (int q = 0; q < 4 && j > 0 && past(j - 1); ++q) --j;
+    for (int q = 0; q < 4 && j < L && !past(j); ++q) ++j;
+    if ((j > 0 && past(j - 1)) || (j < L && !past(j))) {
+      int64_t lo = 0, hi = L;
+      while (lo < hi) {
+        const int64_t mid = (lo + hi) / 2;
+        if (past(mid)) hi = mid; else lo = mid + 1;
+      }
+      j = lo;
     }
-    int64_t lo2 = lo, hi2 = L;
-    while (lo2 < hi2) {
-      const int64_t mid = (lo2 + hi2) / 2;
-      if (tm_sample_time(a, mid, L, a.tm_step, r.jitter) <= a.t_max) lo2 = mid + 1; else hi2 = mid;
-    }
-    r.tm_j0 = lo;
-    r.tm_j1 = lo2 - 1;
+    if (first) r.tm_j0 = j;
+    else r.tm_j1 = j - 1;
   }
-  a.rec[i] = r;
-  if (a.order_hist) atomicAdd(&a.order_hist[order_key(a, r)], 1);
 }
 
-__global__ void k_prologue(LaunchArgs a) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.B) return;
-  prologue_point(a, i);
+__global__ void __launch_bounds__(kProloguePoints * kPrologueWarps) k_prologue(LaunchArgs a) {
+  __shared__ PrologueShared sh;
+  const int64_t i = (int64_t)blockIdx.x * kProloguePoints + threadIdx.x % kProloguePoints;
+  prologue_cta(a, sh, min(i, a.B - 1), i < a.B);
 }
 
 // Counts per bucket -> first slot of each bucket, buckets in descending order
@@ -395,7 +495,8 @@ __device__ void order_scan(const LaunchArgs& a) {
 // Slot of point i within its bucket (any order inside a bucket: the result of
 // a point does not depend on the slot it is evaluated in).
 __device__ __forceinline__ void order_scatter(const LaunchArgs& a, int64_t i) {
-  const int key = order_key(a, a.rec[i]);
+  const PointRec& r = a.rec[i];
+  const int key = order_key(a, OrderPoint{r.valid, r.refine, r.k_start, r.k_end, r.sg_f0});
   const int pos = a.order_hist[key] + atomicAdd(&a.order_hist[a.order_keys + key], 1);
   if (pos >= 0 && pos < a.B) a.order[pos] = (int32_t)i;
   else atomicExch(a.status, kDevStatusBadInput);
@@ -1764,8 +1865,7 @@ __global__ void k_finalize(LaunchArgs a) {
 constexpr int kPointThreads = 32;
 
 cudaError_t launch_prologue(const LaunchArgs& a, cudaStream_t s) {
-  const int threads = kPointThreads;
-  k_prologue<<<(unsigned)((a.B + threads - 1) / threads), threads, 0, s>>>(a);
+  k_prologue<<<(unsigned)((a.B + kProloguePoints - 1) / kProloguePoints), kProloguePoints * kPrologueWarps, 0, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -1956,11 +2056,12 @@ __device__ __forceinline__ int find_item(const int64_t* off, int n, int64_t p) {
   return lo;
 }
 
-__global__ void k_multi_prologue(MultiArgs m) {
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= m.total_points) return;
-  const int it = find_item(m.offsets, m.n_items, p);
-  prologue_point(m.args[it], p - m.offsets[it]);
+__global__ void __launch_bounds__(kProloguePoints * kPrologueWarps) k_multi_prologue(MultiArgs m) {
+  __shared__ PrologueShared sh;
+  const int64_t p = (int64_t)blockIdx.x * kProloguePoints + threadIdx.x % kProloguePoints;
+  const int64_t q = min(p, m.total_points - 1);
+  const int it = find_item(m.offsets, m.n_items, q);
+  prologue_cta(m.args[it], sh, q - m.offsets[it], p < m.total_points);
 }
 
 __global__ void __launch_bounds__(kOrderThreads) k_multi_order_scan(MultiArgs m) {
@@ -2116,7 +2217,8 @@ cudaError_t side_join(SideStream& side, cudaStream_t s) {
 cudaError_t launch_multi(const MultiArgs& m, const int* ctas, const int* ctas_acc, cudaStream_t s, SideStream* side) {
   const int threads = kPointThreads;
   const unsigned pblocks = (unsigned)((m.total_points + threads - 1) / threads);
-  k_multi_prologue<<<pblocks, threads, 0, s>>>(m);
+  k_multi_prologue<<<(unsigned)((m.total_points + kProloguePoints - 1) / kProloguePoints),
+                     kProloguePoints * kPrologueWarps, 0, s>>>(m);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (m.ordered) {

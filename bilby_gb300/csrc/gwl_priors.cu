@@ -136,14 +136,14 @@ __global__ void k_priors(const PriorEntry* entries, int n, const double* unit, i
     const double oy = R[3] * wx + R[4] * wy + R[5] * wz;
     const double oz = R[6] * wx + R[7] * wy + R[8] * wz;
     const double theta = acos(oz);
-    const double phi = pymod(atan2(oy, ox), kTwoPi);
-    params[(int64_t)GWL_P_RA * B + i] = pymod(phi + gmst_radians(t), kTwoPi);
+    const double phi = mod_two_pi(atan2(oy, ox));
+    params[(int64_t)GWL_P_RA * B + i] = mod_two_pi(phi + gmst_radians(t));
     params[(int64_t)GWL_P_DEC * B + i] = kPi / 2 - theta;
   }
   if (frame.has_vertex && has_tdet) {
     // geometry.py:319-343: geocent_time = t - time_delay_from_geocenter(vertex, ra, dec, t)
     const double ra = params[(int64_t)GWL_P_RA * B + i], dec = params[(int64_t)GWL_P_DEC * B + i];
-    const double gmst = pymod(gmst_radians(t), kTwoPi);
+    const double gmst = mod_two_pi(gmst_radians(t));
     const double ph = ra - gmst, th = kPi / 2 - dec;
     const double ox = sin(th) * cos(ph), oy = sin(th) * sin(ph), oz = cos(th);
     const double delay = ((0.0 - frame.vertex[0]) * ox + (0.0 - frame.vertex[1]) * oy + (0.0 - frame.vertex[2]) * oz) /

@@ -63,7 +63,7 @@ __global__ void k_response(DetGeom g, const double* freq, int64_t n, const doubl
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const double tgeo = p[GWL_P_GEOCENT_TIME];
-  const double gmst = pymod(gmst_radians(tgeo), kTwoPi);
+  const double gmst = mod_two_pi(gmst_radians(tgeo));
   double fp, fx, delay;
   antenna_and_delay(g.tensor, g.vertex, p[GWL_P_RA], p[GWL_P_DEC], p[GWL_P_PSI], gmst, &fp, &fx, &delay);
   const double dt = (tgeo - g.start_time) + delay;

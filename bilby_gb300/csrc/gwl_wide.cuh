@@ -176,7 +176,15 @@ __host__ __device__ __forceinline__ int wide_lanes(int64_t n_chunks) { return n_
 
 __device__ __forceinline__ double wide_chunk_sum(const double* q, int64_t n, int lane, int lanes) {
   double s = 0.0;
-  for (int64_t g = lane; g < n; g += lanes) s += q[g];
+  int64_t g = lane;
+  for (; g + 7 * lanes < n; g += 8 * lanes) {  // eight loads in flight
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = q[g + u * lanes];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s += v[u];
+  }
+  for (; g < n; g += lanes) s += q[g];
   for (int o = lanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   return s;
 }
