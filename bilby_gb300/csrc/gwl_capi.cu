@@ -910,7 +910,7 @@ int prepare_wide(gwl_analysis* a, LaunchArgs& L, cudaStream_t s) {
 // ... larger batches ordered so that a warp's points visit nearly the same bins
 // (LaunchArgs::order; launch_order follows the prologue)
 cudaError_t order_wide(gwl_analysis* a, LaunchArgs& L, cudaStream_t s) {
-  if (L.B < kWideOrderPoints) return cudaSuccess;
+  if (wide_few(L.B, L.wide_chunks) || L.B * L.wide_chunks < kOrderWideWork) return cudaSuccess;
   L.order = a->d_order;
   L.order_hist = a->d_order_hist;
   ordering_with_marks(L);
@@ -1093,7 +1093,12 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
   if (wide && (rc = prepare_wide(a, L, s))) return rc;
   if (d_dh) L.cplx = 1;  // complex <d|h> requested
   const bool ordered = precision == GWL_PRECISION_MIXED && a->model == GWL_MODEL_TAYLORF2 && !(a->time_marg && d_out);
-  if (ordered) {
+  const bool few = ordered && B * a->n_chunks_mixed * a->n_det <= kFewMixedWork && B <= 65535;
+  if (few) {
+    L.rf_count = L.rf_tol > 0 ? a->d_order_hist : nullptr;
+    a->last_rf_count = L.rf_count;
+    if (L.rf_count) GWL_CUDA(cudaMemsetAsync(L.rf_count, 0, sizeof(int32_t), s));
+  } else if (ordered) {
     // group the points by band end (see LaunchArgs::order)
     L.order = a->d_order;
     L.order_hist = a->d_order_hist;
@@ -1118,7 +1123,7 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
     L.rf_tol = 0.0;
   }
   GWL_CUDA(launch_prologue(L, s));
-  if (ordered || L.order) GWL_CUDA(launch_order(L, s));
+  if (L.order) GWL_CUDA(launch_order(L, s));
   if (a->profiling) GWL_CUDA(cudaEventRecord(a->ev_begin, s));
   if (a->time_marg && d_out) {
     // mixed TaylorF2: the whole-FFT kernel marks the points over its error
@@ -1148,7 +1153,7 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
     }
     return GWL_OK;
   }
-  const bool acc = precision == GWL_PRECISION_MIXED && a->model == GWL_MODEL_TAYLORF2 && L.rf_tol > 0;
+  const bool acc = precision == GWL_PRECISION_MIXED && a->model == GWL_MODEL_TAYLORF2 && L.rf_tol > 0 && !few;
   if (acc) {
     // the marked points in the accurate kernel on the side stream, beside the fast kernel
     GWL_CUDA(side_fork(a->side, s));
@@ -1156,6 +1161,8 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
   }
   if (wide) {
     GWL_CUDA(a->model == GWL_MODEL_SINEGAUSSIAN ? launch_wide_sg(L, s) : launch_wide(L, s));
+  } else if (few) {
+    GWL_CUDA(launch_mixed_few(L, s));
   } else {
     GWL_CUDA(launch_mixed(L, s));
   }
@@ -1164,7 +1171,7 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
     a->ev_pending = 1;
   }
   if (acc) GWL_CUDA(side_join(a->side, s));
-  if (wide) return GWL_OK;  // launch_wide ends with the totals
+  if (wide || few) return GWL_OK;  // (they end with the totals)
   GWL_CUDA(launch_finalize(L, s));
   if (precision == GWL_PRECISION_MIXED && a->model == GWL_MODEL_SINEGAUSSIAN && L.rf_tol > 0)
     GWL_CUDA(launch_sg_refine(L, s));

@@ -41,8 +41,21 @@ constexpr double kRefineL1 = 1e-7;
 constexpr double kRefineLoudPower = 10.0;
 constexpr double kRefineDefaultTol = 5e-4;
 constexpr int kCosTable = 1024;        // angles of the float-float cos / sin table of the accurate kernel
-constexpr int kWideOrderPoints = 64;   // ... and from this size on, ordered by band end
-constexpr int kWideFewPoints = 24;     // float64 TaylorF2 batches up to this size run one CTA per (chunk, point)
+// Mixed TaylorF2: launch_mixed_few up to this many points x chunks x detectors.
+// Measured per call (us), few against one lane per point: 128 s, 3 detectors, 94
+// points 196 / 227, 128 points 252 / 230; 32 s, 2 detectors, 256 points 104 / 392.
+constexpr int64_t kFewMixedWork = 144 << 10;
+// Float64: one CTA per (chunk, point) up to this many points, or points x chunks.
+// Measured: 128 s (1014 chunks), 8 points 95 / 129, 16 points 148 / 130; 32 s (255),
+// 8 points 44 / 50, 16 points 55 / 51; 8 s (32), 64 points 51 / 57, 128 points 61 / 57.
+constexpr int kFewWidePoints = 12;
+constexpr int64_t kFewWideWork = 3200;
+__host__ __device__ constexpr bool wide_few(int64_t points, int64_t chunks) {
+  return points <= kFewWidePoints || points * chunks <= kFewWideWork;
+}
+// ... and ordered by band end from this many points x chunks on: the ordering costs
+// 10 to 17 us and saves up to a quarter of the bins (8 s, 64 points 47 / 57).
+constexpr int64_t kOrderWideWork = 32 << 10;
 constexpr int kWideEnd = kNumBasis + 2 + 2 * kMaxDet, kWideWords = kWideEnd + 1;  // words per point of LaunchArgs::wide_c
 constexpr int kExpTable = 256;         // entries 2^(-i / 256) of gwl_wide_sg.cu
 constexpr int kWideTable = 2048;       // angles of the float-float cosine table of gwl_wide.cuh
@@ -353,6 +366,8 @@ cudaError_t launch_wide_basis(const double* f, int64_t k0, int64_t n, int64_t pa
 cudaError_t launch_wide_weights(const double2* z, const double* u, const double4* ftab, double inv_scale, int64_t n,
                                 uint4* out, cudaStream_t s);
 cudaError_t launch_mixed(const LaunchArgs& a, cudaStream_t s);
+// Few points of TaylorF2 in mixed precision, totals and lnL included (no ordering).
+cudaError_t launch_mixed_few(const LaunchArgs& a, cudaStream_t s);
 // The accurate kernel for the marked points (nothing when rf_tol <= 0).
 cudaError_t launch_mixed_acc(const LaunchArgs& a, cudaStream_t s);
 

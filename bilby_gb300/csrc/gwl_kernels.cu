@@ -597,16 +597,15 @@ __device__ __forceinline__ void acc_ff(float& hi, float& lo, float m, float c_hi
 
 // One 8-bin block of the anchored walk, two bins per packed pair.  top[d]:
 // detector d's 32-bit phase at the block start without the weight angle (on
-// return: at the block's last bin, with it); sl[d]: its slope per bin.  wq:
-// detector 0's four bin pairs of the block in the stage (detector d is
-// kChunkMixed / 2 pairs further per detector).  jj: (j, j + 1) of the first
+// return: at the block's last bin, with it); sl[d]: its slope per bin.  wq(d, p):
+// detector d's bin pair p of the block.  jj: (j, j + 1) of the first
 // pair relative to the anchor (advanced by 8).  A3, A4: the cubic and quartic
 // Taylor coefficients in radians (both lanes equal), a5, a6 the quintic and
 // sextic ones (zero below degree 5; HI blocks only), a2: the second
 // difference of the quadratic part, whose local remainder is C(i, 2) a2.
 // MASK: bins outside [lo, hi) contribute nothing (band edges).
-template <int D, bool CPLX, bool HI, bool MASK>
-__device__ __forceinline__ void tf2_block(uint32_t* top, const uint32_t* sl, const uint4* wq, float2& jj,
+template <int D, bool CPLX, bool HI, bool MASK, class W>
+__device__ __forceinline__ void tf2_block(uint32_t* top, const uint32_t* sl, const W& wq, float2& jj,
                                           float2 A3, float2 A4, float a5, float a6, float a2, int lo, int hi,
                                           float2* acc, float2* acci) {
   const float2 cc = make_float2(1.4629180792671596e-09f, 1.4629180792671596e-09f);  // 2 pi 2^-32
@@ -624,7 +623,7 @@ __device__ __forceinline__ void tf2_block(uint32_t* top, const uint32_t* sl, con
     jj = add2(jj, two);
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      const uint4 q = wq[d * (kChunkMixed / 2) + p];
+      const uint4 q = wq(d, p);
       const uint32_t ta = p == 0 ? top[d] + q.z : top[d] + sl[d] + q.z;
       const uint32_t tb = ta + sl[d] + q.w;
       top[d] = tb;
@@ -647,49 +646,105 @@ __device__ __forceinline__ void tf2_block(uint32_t* top, const uint32_t* sl, con
   }
 }
 
-// A chunk where no anchor interval meets the Taylor bound: the phase of every
-// bin in float-float from the per-bin basis table (sum_b c_b phi_b(f_k)),
-// the time shift exact in 0.64 fixed point; the weights from the plain polar
-// table in global memory.
+// kFold bins from bin jb of a chunk on with the phase of every bin in
+// float-float from the per-bin basis table (sum_b c_b phi_b(f_k)), the time
+// shift exact in 0.64 fixed point; the weights from the plain polar table in
+// global memory.
+template <int D, bool CPLX>
+__device__ __forceinline__ void direct_block(const LaunchArgs& a, int64_t k0, int64_t ks, int jb, int jlast,
+                                             const float* ch, const float* cl, const uint64_t* X, const uint64_t* Q,
+                                             float* are, float* aim) {
+#pragma unroll
+  for (int d = 0; d < D; ++d) are[d] = aim[d] = 0.f;
+  const int je = min(jb + kFold, jlast);
+  for (int j = jb; j < je; ++j) {
+    const int64_t k = k0 + j;
+    if (k < ks) continue;
+    const float4* bp = reinterpret_cast<const float4*>(a.basis + k * kNumBasis);
+    float s_hi = ch[kNumBasis], s_lo = cl[kNumBasis];
+#pragma unroll
+    for (int q = 0; q < kNumBasis / 2; ++q) {
+      const float4 v = __ldg(bp + q);
+      ff_mac(s_hi, s_lo, ch[2 * q], cl[2 * q], v.x, v.y);
+      ff_mac(s_hi, s_lo, ch[2 * q + 1], cl[2 * q + 1], v.z, v.w);
+    }
+    const uint32_t bu = (uint32_t)((to_fixed(s_hi, s_lo) + 0x80000000ull) >> 32);
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      const uint2 wv = __ldg(a.wp[d] + k);
+      const uint32_t top = bu + (uint32_t)(((uint64_t)k * X[d] + Q[d]) >> 32) + wv.y;
+      const float ph = __fmul_rn(__int2float_rn((int)top), 1.4629180792671596e-09f);
+      float sn, cs;
+      __sincosf(ph, &sn, &cs);
+      const float mag = __uint_as_float(wv.x);
+      are[d] = __fmaf_rn(mag, cs, are[d]);
+      if (CPLX) aim[d] = __fmaf_rn(mag, sn, aim[d]);
+    }
+  }
+}
+
+// A chunk where no anchor interval meets the Taylor bound.
 template <int D, bool CPLX>
 __device__ __forceinline__ void direct_chunk(const LaunchArgs& a, int64_t k0, int64_t ks, int jlast,
                                              const float* ch, const float* cl, const uint64_t* X, const uint64_t* Q,
                                              float* ahi, float* alo, float* bhi, float* blo) {
   for (int jb = 0; jb < jlast; jb += kFold) {
     float are[D], aim[D];
-#pragma unroll
-    for (int d = 0; d < D; ++d) are[d] = aim[d] = 0.f;
-    const int je = min(jb + kFold, jlast);
-    for (int j = jb; j < je; ++j) {
-      const int64_t k = k0 + j;
-      if (k < ks) continue;
-      const float4* bp = reinterpret_cast<const float4*>(a.basis + k * kNumBasis);
-      float s_hi = ch[kNumBasis], s_lo = cl[kNumBasis];
-#pragma unroll
-      for (int q = 0; q < kNumBasis / 2; ++q) {
-        const float4 v = __ldg(bp + q);
-        ff_mac(s_hi, s_lo, ch[2 * q], cl[2 * q], v.x, v.y);
-        ff_mac(s_hi, s_lo, ch[2 * q + 1], cl[2 * q + 1], v.z, v.w);
-      }
-      const uint32_t bu = (uint32_t)((to_fixed(s_hi, s_lo) + 0x80000000ull) >> 32);
-#pragma unroll
-      for (int d = 0; d < D; ++d) {
-        const uint2 wv = __ldg(a.wp[d] + k);
-        const uint32_t top = bu + (uint32_t)(((uint64_t)k * X[d] + Q[d]) >> 32) + wv.y;
-        const float ph = __fmul_rn(__int2float_rn((int)top), 1.4629180792671596e-09f);
-        float sn, cs;
-        __sincosf(ph, &sn, &cs);
-        const float mag = __uint_as_float(wv.x);
-        are[d] = __fmaf_rn(mag, cs, are[d]);
-        if (CPLX) aim[d] = __fmaf_rn(mag, sn, aim[d]);
-      }
-    }
+    direct_block<D, CPLX>(a, k0, ks, jb, jlast, ch, cl, X, Q, are, aim);
 #pragma unroll
     for (int d = 0; d < D; ++d) {
       two_sum_acc(ahi[d], alo[d], are[d]);
       if (CPLX) two_sum_acc(bhi[d], blo[d], aim[d]);
     }
   }
+}
+
+// Detector d's shift per bin, and its constant phase offset (real-part kernel).
+__device__ __forceinline__ uint64_t shift_of(const PointRec& r, int d) {
+  return ((uint64_t)r.xfix[d][1] << 32) | r.xfix[d][0];
+}
+template <bool CPLX>
+__device__ __forceinline__ uint64_t offset_of(const PointRec& r, int d) {
+  return CPLX ? 0ull : ((uint64_t)r.qfix[d][1] << 32) | r.qfix[d][0];
+}
+
+// The phase about anchor bin k: the exact quadratic part's value, step-8
+// differences and first differences (0.64 fixed point, detector 0's shift and
+// offset with it), the other detectors' relative shifts, and the coefficients of
+// the float32 remainder.
+template <int D, bool CPLX>
+__device__ __forceinline__ void anchor_state(const LaunchArgs& a, const PointRec& r, int64_t k, int J, float c0, uint64_t& E0,
+                                             uint64_t& E1, uint64_t& E2, uint64_t& F0, uint64_t& F1, uint64_t* L64,
+                                             float2& A3, float2& A4, float& a5, float& a6, float& a2, bool& hi_deg) {
+  const int deg = anchor_degree(c0 * __powf((float)k * (float)a.step, -5.0f / 3.0f), (float)J / (float)k);
+  AnchorTaylor t;
+  anchor_taylor(a.anchors, k, r.c_hi, r.c_lo, t);
+  const uint64_t q0 = offset_of<CPLX>(r, 0), X0 = shift_of(r, 0);
+  // Q(j) = A0 + A1 j + A2 j^2: Delta_8 Q(0) = 8 A1 + 64 A2, Delta_8^2 Q = 128 A2,
+  // dQ(0) = A1 + A2, Delta_8 dQ = 16 A2 (scalings by powers of two are exact)
+  float eh = 8.f * t.h[1], el = 8.f * t.l[1];
+  ff_add(eh, el, 64.f * t.h[2], 64.f * t.l[2]);
+  float fh = t.h[1], fl = t.l[1];
+  ff_add(fh, fl, t.h[2], t.l[2]);
+  E0 = to_fixed(t.h[0], t.l[0]) + (uint64_t)k * X0 + q0 + 0x80000000ull;
+  E1 = to_fixed(eh, el) + 8ull * X0;
+  E2 = to_fixed(128.f * t.h[2], 128.f * t.l[2]);
+  F0 = to_fixed(fh, fl) + X0 + 0x80000000ull;
+  F1 = to_fixed(16.f * t.h[2], 16.f * t.l[2]);
+#pragma unroll
+  for (int d = 1; d < D; ++d)
+    L64[d] = (uint64_t)k * (shift_of(r, d) - X0) + (offset_of<CPLX>(r, d) - q0) + 0x80000000ull;
+  // C(j) = j^3 (A3 + j (A4 + j (A5 + j A6))) in radians, truncated at degree deg
+  const float tp = 6.283185307179586f;
+  const float a3 = __fmul_rn(__fadd_rn(t.h[3], t.l[3]), tp), a4 = __fmul_rn(t.f[0], tp);
+  a5 = deg >= 5 ? __fmul_rn(t.f[1], tp) : 0.f;
+  a6 = deg >= 6 ? __fmul_rn(t.f[2], tp) : 0.f;
+  A3 = make_float2(a3, a3);
+  A4 = make_float2(a4, a4);
+  hi_deg = deg > 4;
+  // second difference of Q in radians: the local quadratic remainder
+  // Q(jb + i) - Q(jb) - i dQ(jb) = C(i, 2) 2 A2
+  a2 = __fmul_rn(2.f * t.h[2], tp);
 }
 
 // One work unit: the points of tile `tile` over the chunks g, g + G, ...
@@ -725,12 +780,8 @@ __device__ __noinline__ void tf2_unit(const LaunchArgs& a, int64_t tile, int64_t
   // from it where they are needed (anchor set-ups), not held in registers
   const PointRec* rp = have ? a.rec + i : a.rec;
   float c0 = 0.f;
-  // constant phase offset of detector d (real-part kernel), read when needed
-  const auto qoff = [&](int d) -> uint64_t {
-    if (CPLX) return 0;
-    return ((uint64_t)rp->qfix[d][1] << 32) | rp->qfix[d][0];
-  };
-  const auto xfix = [&](int d) -> uint64_t { return ((uint64_t)rp->xfix[d][1] << 32) | rp->xfix[d][0]; };
+  const auto qoff = [&](int d) { return offset_of<CPLX>(*rp, d); };
+  const auto xfix = [&](int d) { return shift_of(*rp, d); };
   if (have && valid) c0 = fabsf(rp->c_hi[0]);
   // float32 partial sums folded into float-float accumulators, over every
   // chunk of the unit (real part; imaginary part for the complex kernel)
@@ -818,34 +869,7 @@ __device__ __noinline__ void tf2_unit(const LaunchArgs& a, int64_t tile, int64_t
         for (int jb = 0; jb < jlast; jb += 8) {
           const int64_t k = k0 + jb;
           if ((jb & (J - 1)) == 0) {
-            const int deg = anchor_degree(c0 * __powf((float)k * (float)a.step, -5.0f / 3.0f), (float)J / (float)k);
-            AnchorTaylor t;
-            anchor_taylor(a.anchors, k, rp->c_hi, rp->c_lo, t);
-            const uint64_t q0 = qoff(0), X0 = xfix(0);
-            // Q(j) = A0 + A1 j + A2 j^2: Delta_8 Q(0) = 8 A1 + 64 A2, Delta_8^2 Q = 128 A2,
-            // dQ(0) = A1 + A2, Delta_8 dQ = 16 A2 (scalings by powers of two are exact)
-            float eh = 8.f * t.h[1], el = 8.f * t.l[1];
-            ff_add(eh, el, 64.f * t.h[2], 64.f * t.l[2]);
-            float fh = t.h[1], fl = t.l[1];
-            ff_add(fh, fl, t.h[2], t.l[2]);
-            E0 = to_fixed(t.h[0], t.l[0]) + (uint64_t)k * X0 + q0 + 0x80000000ull;
-            E1 = to_fixed(eh, el) + 8ull * X0;
-            E2 = to_fixed(128.f * t.h[2], 128.f * t.l[2]);
-            F0 = to_fixed(fh, fl) + X0 + 0x80000000ull;
-            F1 = to_fixed(16.f * t.h[2], 16.f * t.l[2]);
-#pragma unroll
-            for (int d = 1; d < D; ++d) L64[d] = (uint64_t)k * (xfix(d) - X0) + (qoff(d) - q0) + 0x80000000ull;
-            // C(j) = j^3 (A3 + j (A4 + j (A5 + j A6))) in radians, truncated at degree deg
-            const float tp = 6.283185307179586f;
-            const float a3 = __fmul_rn(__fadd_rn(t.h[3], t.l[3]), tp), a4 = __fmul_rn(t.f[0], tp);
-            a5 = deg >= 5 ? __fmul_rn(t.f[1], tp) : 0.f;
-            a6 = deg >= 6 ? __fmul_rn(t.f[2], tp) : 0.f;
-            A3 = make_float2(a3, a3);
-            A4 = make_float2(a4, a4);
-            hi_deg = deg > 4;
-            // second difference of Q in radians: the local quadratic remainder
-            // Q(jb + i) - Q(jb) - i dQ(jb) = C(i, 2) 2 A2
-            a2 = __fmul_rn(2.f * t.h[2], tp);
+            anchor_state<D, CPLX>(a, *rp, k, J, c0, E0, E1, E2, F0, F1, L64, A3, A4, a5, a6, a2, hi_deg);
             jj = make_float2(0.f, 1.f);
           }
           uint32_t top[D], sl[D];
@@ -855,7 +879,7 @@ __device__ __noinline__ void tf2_unit(const LaunchArgs& a, int64_t tile, int64_t
             top[d] = d == 0 ? e0 : e0 + (uint32_t)(L64[d] >> 32);
             sl[d] = d == 0 ? f0 : f0 + r32[d];
           }
-          const uint4* wq = w4 + (jb >> 1);
+          const auto wq = [&](int d, int p) { return w4[(jb >> 1) + d * (kChunkMixed / 2) + p]; };
           if (jb + 8 <= jlast && k >= ks) {
             // a whole block inside the band
             if (hi_deg) {
@@ -1009,6 +1033,147 @@ __global__ void __launch_bounds__(kAccThreads) k_mixed_tf2_acc(LaunchArgs a) {
   const int64_t nw = (int64_t)gridDim.x * wpc;
   for (int64_t u = (int64_t)blockIdx.x * wpc + (threadIdx.x >> 5); u < units; u += nw)
     acc_unit<D, CPLX>(a, a.order[u / a.n_groups], u % a.n_groups, tab);
+}
+
+// Few points: the results of k_mixed_tf2 (k_mixed_tf2_acc for marked points) bit
+// for bit, with the bins over the lanes.  CTA (group, point): the group's chunks
+// four at a time, thread = a unit of 16 bins, whose float32 partial sum k_mixed_tf2
+// folds as one; the exact phase sequences are jumped to the unit's start, and one
+// thread per sum folds the units in k_mixed_tf2's order.  There one thread walks
+// the 2048 bins of a group: 170 us for one point of the 128 s segment, and the
+// ordering and the reduction of the groups by single threads another 35.
+constexpr int kUnitBins = 16;
+constexpr int kFewUnits = 128;  // threads; units of four chunks
+
+template <int D, bool CPLX>
+__global__ void __launch_bounds__(kFewUnits) k_mixed_tf2_few(LaunchArgs a) {
+  constexpr int NC = CPLX ? 2 : 1, NS = D * NC, CH = kChunkMixed, UPC = CH / kUnitBins;
+  constexpr int kRow = kFewUnits + 1;
+  __shared__ float v0[NS][kRow], v1[NS][kRow];  // a unit's fold, and a second one in a directly evaluated chunk
+  __shared__ int direct[kFewUnits / UPC];
+  const int64_t g = blockIdx.x, i = blockIdx.y, G = a.n_groups;
+  const PointRec& r = a.rec[i];
+  const int t = threadIdx.x;
+  if (r.refine) {
+    if (t < 32) acc_unit<D, CPLX>(a, i, g, a.cos_tab);
+    return;
+  }
+  const int64_t ks = r.k_start, ke = r.valid ? r.k_end : 0;
+  const float c0 = fabsf(r.c_hi[0]);
+  float hi = 0.f, lo = 0.f;
+  for (int64_t m = 0; g + m * G < a.n_chunks && a.k_base + (g + m * G) * CH < ke; m += kFewUnits / UPC) {
+    const int64_t c = g + (m + t / UPC) * G, k0 = a.k_base + c * CH;
+    const int ub = (t % UPC) * kUnitBins;
+    float x0[NS], x1[NS];
+#pragma unroll
+    for (int q = 0; q < NS; ++q) x0[q] = x1[q] = 0.f;
+    int J = 1;
+    if (c < a.n_chunks && k0 < ke && k0 + CH > ks) {
+      J = anchor_interval(c0 * __powf((float)k0 * (float)a.step, -5.0f / 3.0f), (float)max(k0, (int64_t)8));
+      const int jlast = (int)min((int64_t)CH, ke - k0);
+      if (J == 0) {
+        float ch[kNumBasis + 1], cl[kNumBasis + 1];
+#pragma unroll
+        for (int b = 0; b <= kNumBasis; ++b) {
+          ch[b] = r.c_hi[b];
+          cl[b] = r.c_lo[b];
+        }
+        uint64_t X[D], Q[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          X[d] = shift_of(r, d);
+          Q[d] = offset_of<CPLX>(r, d);
+        }
+        float re[D], im[D];
+        if (ub < jlast) direct_block<D, CPLX>(a, k0, ks, ub, jlast, ch, cl, X, Q, re, im);
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          if (ub < jlast) x0[d * NC] = re[d];
+          if (CPLX && ub < jlast) x0[d * NC + 1] = im[d];
+        }
+        if (ub + kFold < jlast) direct_block<D, CPLX>(a, k0, ks, ub + kFold, jlast, ch, cl, X, Q, re, im);
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          if (ub + kFold < jlast) x1[d * NC] = re[d];
+          if (CPLX && ub + kFold < jlast) x1[d * NC + 1] = im[d];
+        }
+      } else {
+        uint64_t R8[D], L64[D];
+        uint32_t r32[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          const uint64_t Rd = shift_of(r, d) - shift_of(r, 0);
+          r32[d] = (uint32_t)((Rd + 0x80000000ull) >> 32);
+          R8[d] = Rd * 8ull;
+          L64[d] = 0;
+        }
+        const float2 zero2 = make_float2(0.f, 0.f);
+        float2 acc[D], acci[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) acc[d] = acci[d] = zero2;
+        uint64_t E0 = 0, E1 = 0, E2 = 0, F0 = 0, F1 = 0;
+        float2 A3 = zero2, A4 = zero2;
+        float a5 = 0.f, a6 = 0.f, a2 = 0.f;
+        bool hi_deg = false;
+#pragma unroll 1
+        for (int jb = ub; jb < min(ub + kUnitBins, jlast); jb += 8) {
+          const int64_t k = k0 + jb;
+          if (jb == ub || (jb & (J - 1)) == 0)
+            anchor_state<D, CPLX>(a, r, k0 + (jb & ~(J - 1)), J, c0, E0, E1, E2, F0, F1, L64, A3, A4, a5, a6, a2, hi_deg);
+          if (k + 8 <= ks) continue;
+          // the sequences n blocks after the anchor
+          const uint64_t n = (uint64_t)(jb & (J - 1)) >> 3;
+          const uint32_t e0 = (uint32_t)((E0 + n * E1 + (n * (n - 1) / 2) * E2) >> 32), f0 = (uint32_t)((F0 + n * F1) >> 32);
+          uint32_t top[D], sl[D];
+#pragma unroll
+          for (int d = 0; d < D; ++d) {
+            top[d] = d == 0 ? e0 : e0 + (uint32_t)((L64[d] + n * R8[d]) >> 32);
+            sl[d] = d == 0 ? f0 : f0 + r32[d];
+          }
+          float2 jj = make_float2((float)(8 * n), (float)(8 * n + 1));
+          const auto wq = [&](int d, int p) { return __ldg(a.wq[d] + (k >> 1) + p); };
+          if (jb + 8 <= jlast && k >= ks) {
+            if (hi_deg) {
+              tf2_block<D, CPLX, true, false>(top, sl, wq, jj, A3, A4, a5, a6, a2, 0, 8, acc, acci);
+            } else {
+              tf2_block<D, CPLX, false, false>(top, sl, wq, jj, A3, A4, a5, a6, a2, 0, 8, acc, acci);
+            }
+          } else {
+            const int first = (int)max((int64_t)0, ks - k), last = min(8, jlast - jb);
+            tf2_block<D, CPLX, true, true>(top, sl, wq, jj, A3, A4, a5, a6, a2, first, last, acc, acci);
+          }
+        }
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          x0[d * NC] = __fadd_rn(acc[d].x, acc[d].y);
+          if (CPLX) x0[d * NC + 1] = __fadd_rn(acci[d].x, acci[d].y);
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < NS; ++q) {
+      v0[q][t] = x0[q];
+      v1[q][t] = x1[q];
+    }
+    if (t % UPC == 0) direct[t / UPC] = J == 0;
+    __syncthreads();
+    if (t < NS) {
+      for (int b = 0; b < kFewUnits / UPC; ++b) {
+        const float *f0 = v0[t] + b * UPC, *f1 = v1[t] + b * UPC;
+        if (direct[b]) {
+          for (int u = 0; u < UPC; ++u) {
+            two_sum_acc(hi, lo, f0[u]);
+            two_sum_acc(hi, lo, f1[u]);
+          }
+        } else {
+#pragma unroll 8
+          for (int u = 0; u < UPC; ++u) two_sum_acc(hi, lo, f0[u]);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if (t < NS) a.part[((g * D + t / NC) * kPartStride + t % NC) * a.B + i] = (double)hi + (double)lo;
 }
 
 // Sine-Gaussian, mixed precision (bilby/gw/source.py:1197-1207 projected as
@@ -1850,6 +2015,30 @@ __global__ void __launch_bounds__(32 * kRelbinWarps) k_multiband_mixed(LaunchArg
   if (lane == 0) finish_point(a, r, i, sr, -si, hh);
 }
 
+// Few points: reduce_chain's sums (in its order) and the totals of one point per
+// CTA, the groups' partial sums read by all threads at once.
+constexpr int kFewFinThreads = 128;
+
+__global__ void __launch_bounds__(kFewFinThreads) k_few_finalize(LaunchArgs a) {
+  __shared__ double v[2 * kMaxDet][kFewFinThreads];
+  const int64_t i = blockIdx.x, G = a.n_groups, gs = (int64_t)a.n_det * kPartStride * a.B;
+  const int nq = part_components(a), chains = a.n_det * nq, t = threadIdx.x;
+  double p = 0.0;
+  for (int64_t c0 = 0; c0 < G; c0 += kFewFinThreads) {
+    const int n = (int)min(G - c0, (int64_t)kFewFinThreads);
+    if (t < n)
+      for (int q = 0; q < chains; ++q)
+        v[q][t] = a.part[(c0 + t) * gs + ((int64_t)(q / nq) * kPartStride + q % nq) * a.B + i];
+    __syncthreads();
+    if (t < chains)
+      for (int c = 0; c < n; ++c) p += v[t][c];
+    __syncthreads();
+  }
+  if (t < chains) a.part[((int64_t)(t / nq) * kPartStride + t % nq) * a.B + i] = p;
+  __syncthreads();
+  if (t == 0) finalize_point(a, i, 1);
+}
+
 __global__ void k_finalize(LaunchArgs a) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.B) return;
@@ -1963,6 +2152,24 @@ cudaError_t launch_mixed_acc(const LaunchArgs& a, cudaStream_t s) {
       GWL_DISPATCH_D(k_mixed_tf2_acc_r, g_acc, kAccThreads, 0, s, a);
     }
   }
+  return cudaGetLastError();
+}
+
+template <int D>
+constexpr auto k_mixed_tf2_few_c = k_mixed_tf2_few<D, true>;
+template <int D>
+constexpr auto k_mixed_tf2_few_r = k_mixed_tf2_few<D, false>;
+
+cudaError_t launch_mixed_few(const LaunchArgs& a, cudaStream_t s) {
+  const dim3 grid((unsigned)a.n_groups, (unsigned)a.B);
+  if (a.cplx) {
+    GWL_DISPATCH_D(k_mixed_tf2_few_c, grid, kFewUnits, 0, s, a);
+  } else {
+    GWL_DISPATCH_D(k_mixed_tf2_few_r, grid, kFewUnits, 0, s, a);
+  }
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  k_few_finalize<<<(unsigned)a.B, kFewFinThreads, 0, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -344,7 +344,7 @@ cudaError_t launch_wide_weights(const double2* z, const double* u, const double4
 
 template <int D, bool CPLX>
 static cudaError_t launch_wide_d(const LaunchArgs& a, cudaStream_t s) {
-  if (a.B <= kWideFewPoints) {
+  if (wide_few(a.B, a.wide_chunks)) {
     const dim3 grid((unsigned)a.wide_chunks, (unsigned)a.B);
     k_wide_tf2_few<D, CPLX><<<grid, kPairThreads, 0, s>>>(a);
     return cudaGetLastError();

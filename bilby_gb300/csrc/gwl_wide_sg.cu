@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(kWideFinThreads) k_wide_sg_finalize(LaunchArgs
 
 template <int D, bool CPLX>
 static cudaError_t launch_wide_sg_d(const LaunchArgs& a, cudaStream_t s) {
-  if (a.B <= kWideFewPoints) {
+  if (wide_few(a.B, a.n_chunks)) {
     const dim3 grid((unsigned)a.n_chunks, (unsigned)a.B);
     k_wide_sg_few<D, CPLX><<<grid, kPairThreads, 0, s>>>(a);
     return cudaGetLastError();

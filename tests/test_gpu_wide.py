@@ -35,12 +35,18 @@ def _case(detectors, duration, fs, masses):
     (4, 4.0, 2048.0, (0.5, 90.0)), (2, 4.0, 2048.0, (1e-3, 2e-3))])
 def test_against_the_oracle_in_every_launch_shape(gpu, detectors, duration, fs, masses):
     w, dets, an = _case(detectors, duration, fs, masses)
-    n = 97
+    n = 70
     p = draw_points(w, n, np.random.default_rng(5))
     block = params_block(p)
     full = an.log_likelihood_ratio_host(block, "fp64")
-    for size in (1, 24, 25, 32, 63, 64, 65):  # one point per CTA, then warps of points, then ordered
-        assert np.array_equal(an.log_likelihood_ratio_host(block[:, :size], "fp64"), full[:size]), size
+    # one CTA per point, then a lane per point, then ordered: the switches lie at 12
+    # points or 3200 points x chunks, and at 32768 points x chunks
+    chunks = -(-(int((fs / 2 - 20) * duration) + 17) // 256)
+    edge = max(12, 3200 // chunks)
+    for size in (1, 12, 13, 32, 33, edge, edge + 1, edge + 40, 32768 // chunks + 70):
+        many = np.ascontiguousarray(np.tile(block, -(-size // n))[:, :size])
+        got = an.log_likelihood_ratio_host(many, "fp64")
+        assert np.array_equal(got, np.tile(full, -(-size // n))[:size]), size
     src = OD.source_for(w.model, w.minimum_frequency)
     terms = [R.plain_terms(dets, src, point(p, i)) for i in range(n)]
     lnl = np.array([np.real(dh) - hh / 2 for dh, hh in terms])

@@ -26,7 +26,7 @@ def test_against_the_oracle_in_every_launch_shape(gpu, detectors, duration, fs):
     dets = OD.build_workload(w)
     dets = (dets + dets)[:detectors]
     an = device_analysis(dets, "sinegaussian", w)
-    n = 97
+    n = 70
     rng = np.random.default_rng(6)
     p = draw_points(w, n, rng)
     p["Q"] = 10 ** rng.uniform(-0.5, 2.3, n)
@@ -34,8 +34,14 @@ def test_against_the_oracle_in_every_launch_shape(gpu, detectors, duration, fs):
     p["frequency"][:20] = np.round(p["frequency"][:20])
     block = params_block(p)
     full = an.log_likelihood_ratio_host(block, "fp64")
-    for size in (1, 24, 25, 32, 63, 64, 65):  # one point per CTA, then warps of points, then ordered
-        assert np.array_equal(an.log_likelihood_ratio_host(block[:, :size], "fp64"), full[:size]), size
+    # one CTA per point, then a lane per point, then ordered (the switches of
+    # test_gpu_wide.py)
+    chunks = -(-(int((fs / 2 - 20) * duration) + 17) // 256)
+    edge = max(12, 3200 // chunks)
+    for size in (1, 12, 13, 32, 33, edge, edge + 1, edge + 40, 32768 // chunks + 70):
+        many = np.ascontiguousarray(np.tile(block, -(-size // n))[:, :size])
+        got = an.log_likelihood_ratio_host(many, "fp64")
+        assert np.array_equal(got, np.tile(full, -(-size // n))[:size]), size
     src = OD.source_for(w.model, w.minimum_frequency)
     terms = [R.plain_terms(dets, src, point(p, i)) for i in range(n)]
     scale = np.array([R.parity_scale(dh, hh) for dh, hh in terms])
