@@ -1090,8 +1090,10 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
     return GWL_OK;
   }
   const bool wide = precision == GWL_PRECISION_FP64 && !(a->time_marg && d_out);
-  if (wide && (rc = prepare_wide(a, L, s))) return rc;
-  if (d_dh) L.cplx = 1;  // complex <d|h> requested
+  const bool wide_tm = precision == GWL_PRECISION_FP64 && a->time_marg && d_out && wide_tm_fits(L);
+  if ((wide || wide_tm) && (rc = prepare_wide(a, L, s))) return rc;
+  if (wide_tm) L.cplx = 0;  // the detectors' arg(conj Q) goes with the phase
+  if (d_dh && !wide_tm) L.cplx = 1;  // complex <d|h> requested
   const bool ordered = precision == GWL_PRECISION_MIXED && a->model == GWL_MODEL_TAYLORF2 && !(a->time_marg && d_out);
   const bool few = ordered && B * a->n_chunks_mixed * a->n_det <= kFewMixedWork && B <= 65535;
   if (few) {
@@ -1144,7 +1146,7 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
       P.rf_count = nullptr;
       GWL_CUDA(launch_mixed(P, s));
     }
-    GWL_CUDA(launch_time_marginalized(L, s));
+    GWL_CUDA(wide_tm ? launch_wide_tm(L, s) : launch_time_marginalized(L, s));
     if (marks) GWL_CUDA(launch_time_marg_marks(L, s));
     if (marks && (rc = launch_window_refine(a, L, s, share))) return rc;
     if (a->profiling) {

@@ -394,6 +394,10 @@ void order_layout(int64_t n_chunks, int* keys, int* shift);
 void ordering_with_marks(LaunchArgs& L);
 void ordering_by_peak(LaunchArgs& L);
 cudaError_t launch_time_marginalized(const LaunchArgs& a, cudaStream_t s);
+// ... float64 TaylorF2 over the full grid (gwl_wide_tm.cu), where the prior
+// window's samples fit its convolution and no series is requested
+bool wide_tm_fits(const LaunchArgs& a);
+cudaError_t launch_wide_tm(const LaunchArgs& a, cudaStream_t s);
 // The mixed full-grid time-marginalised kernel's error bounds, from what it
 // stored in the point records: marks the points over the tolerance.
 cudaError_t launch_time_marg_marks(const LaunchArgs& a, cudaStream_t s);

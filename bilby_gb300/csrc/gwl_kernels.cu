@@ -61,11 +61,12 @@ __device__ __forceinline__ int order_key(const LaunchArgs& a, const OrderPoint& 
 // ---------------------------------------------------------------------------
 // The fixed-point coefficients of gwl_wide.cu (LaunchArgs::wide_c) of point i.
 // ---------------------------------------------------------------------------
-// frac(x + lo) as a 64-bit fraction, |lo| < 1/2
+// frac(x + lo) as a 64-bit fraction, |lo| < 1/2.  x - rint(x) is exact, where
+// x - floor(x) of a small negative x rounds to 2^-53 (a delay of -10 ms loses
+// 1e-16 of a cycle per bin by it)
 __device__ __forceinline__ uint64_t to_wide(double x, double lo) {
-  double fr = (x - floor(x)) * 18446744073709551616.0;  // 2^64: exact
-  if (!(fr >= 0.0 && fr < 18446744073709551616.0)) fr = 0.0;
-  return (uint64_t)fr + (uint64_t)(int64_t)(lo * 18446744073709551616.0);
+  const double two64 = 18446744073709551616.0;
+  return (uint64_t)__double2ll_rn((x - rint(x)) * two64) + (uint64_t)__double2ll_rn(lo * two64);
 }
 
 // 2^e as a double, -1022 <= e <= 1023

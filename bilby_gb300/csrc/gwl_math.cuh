@@ -69,15 +69,22 @@ __host__ __device__ inline int bspline_interval(const double* t, int n, int k, d
 }
 
 // Bicubic spline value at (x, y); -inf outside the bounding box
-// (BoundedRectBivariateSpline, bilby/core/utils/calculus.py:221-262).
-__host__ __device__ inline double bicubic_eval(const double* tx, int nx, const double* ty, int ny, const double* c,
-                                               const double* bbox, double x, double y) {
-  if (!(x >= bbox[0] && x <= bbox[1] && y >= bbox[2] && y <= bbox[3])) return -INFINITY;
-  const int Lx = bspline_interval(tx, nx, 3, x);
+// (BoundedRectBivariateSpline, bilby/core/utils/calculus.py:221-262), in two
+// parts for many x at one y: the y axis's interval (-1 outside the box) and
+// B-spline values hy, then the value at x.
+__host__ __device__ inline int bicubic_row(const double* ty, int ny, const double* bbox, double y, double* hy) {
+  if (!(y >= bbox[2] && y <= bbox[3])) return -1;
   const int Ly = bspline_interval(ty, ny, 3, y);
-  double hx[4], hy[4];
-  bspline_values(tx, 3, x, Lx, hx);
   bspline_values(ty, 3, y, Ly, hy);
+  return Ly;
+}
+
+__host__ __device__ inline double bicubic_at(const double* tx, int nx, int ny, const double* c, const double* bbox,
+                                             double x, int Ly, const double* hy) {
+  if (!(x >= bbox[0] && x <= bbox[1] && Ly >= 0)) return -INFINITY;
+  const int Lx = bspline_interval(tx, nx, 3, x);
+  double hx[4];
+  bspline_values(tx, 3, x, Lx, hx);
   const int ncy = ny - 4;
   double s = 0.0;
   for (int i = 0; i < 4; ++i) {
@@ -87,6 +94,13 @@ __host__ __device__ inline double bicubic_eval(const double* tx, int nx, const d
     s += r * hx[i];
   }
   return s;
+}
+
+__host__ __device__ inline double bicubic_eval(const double* tx, int nx, const double* ty, int ny, const double* c,
+                                               const double* bbox, double x, double y) {
+  double hy[4];
+  const int Ly = bicubic_row(ty, ny, bbox, y, hy);
+  return bicubic_at(tx, nx, ny, c, bbox, x, Ly, hy);
 }
 
 // ln I0(x) - x for x >= 0 in float32 (the large part x is added in float64

@@ -1,0 +1,61 @@
+"""The float64 TaylorF2 likelihood with time marginalisation on the 32-bit pipes
+(csrc/gwl_wide_tm.cu) against the oracle, where the convolution's plan changes.
+
+Tolerance: the marginalised lnL moves by at most the largest error of a sample's
+<d|h>(t_j), so the bound of tests/test_gpu_wide.py holds with the scale max(1,
+max_j |<d|h>(t_j)|, <h|h> / 2)."""
+import numpy as np
+import pytest
+
+from oracle import data as OD
+from oracle import restate as R
+from tests.gpu_helpers import device_analysis, draw_points, params_block, point, small_workload
+
+pytestmark = pytest.mark.gpu
+
+
+# samples of the prior window: two, 502 and 503 (the convolution's length goes from
+# 1024 to 2048), 2038 and 2039 (4096 to 8192), 4086 and 4087 (the longest, then the
+# whole transform); bands inside one block of the convolution (10-40 Msun), of many
+# (0.7-2 Msun at 8 s) and empty (f_ISCO below 20 Hz); FFT lengths 2^p, 3 2^p
+@pytest.mark.parametrize("detectors,duration,fs,masses,samples,phase", [
+    (2, 6.0, 2048.0, (10.0, 40.0), 410, True), (1, 4.0, 2048.0, (1.0, 2.0), 2, False),
+    (3, 8.0, 2048.0, (0.7, 2.0), 502, False), (3, 8.0, 2048.0, (0.7, 2.0), 503, True),
+    (4, 4.0, 4096.0, (5.0, 40.0), 2038, True), (2, 4.0, 4096.0, (5.0, 40.0), 2039, False),
+    (1, 8.0, 2048.0, (2.0, 60.0), 4086, False), (1, 8.0, 2048.0, (2.0, 60.0), 4087, True),
+    (2, 3.0, 640.0, (100.0, 300.0), 100, False), (2, 3.0, 1024.0, (3.0, 9.0), 100, True)])
+def test_against_the_oracle(gpu, detectors, duration, fs, masses, samples, phase):
+    w = small_workload("tf2_marg_8s", detectors=("H1", "L1", "V1")[:min(detectors, 3)], duration=duration,
+                       sampling_frequency=fs, mass_range=masses)
+    w = small_workload("tf2_marg_8s", **{**w.__dict__, "injection": dict(
+        w.injection, mass_1=masses[1], mass_2=masses[0], geocent_time=w.start_time + 0.6 * duration)})
+    dets = OD.build_workload(w)
+    dets = (dets + dets)[:detectors]
+    an = device_analysis(dets, "taylorf2", w)
+    mid, half = w.start_time + 0.6 * duration, samples / fs
+    lo, hi = max(mid - half, w.start_time - 0.01), mid + half
+    lo = hi - 2 * half if lo < mid - half else lo
+    an.set_time_marginalization(True, True, lo, hi)
+    an.set_phase_marginalization(phase)
+    p = draw_points(w, 7, np.random.default_rng(3))
+    for k in w.injection:
+        p[k][0] = w.injection[k]
+    p["geocent_time"] = np.full(7, w.start_time)
+    if phase:
+        p["phase"] = np.zeros(7)
+    block = params_block(p)
+    got = an.log_likelihood_ratio_host(block, "fp64")
+    assert np.array_equal(np.concatenate([an.log_likelihood_ratio_host(block[:, i:i + 1], "fp64") for i in range(7)]), got)
+    m = R.Marginalization(time=True, phase=phase)
+    R.setup_time_marginalization(m, w.start_time, duration, fs, lo, hi)
+    src = OD.source_for(w.model, w.minimum_frequency)
+    for i in range(7):
+        q = point(p, i)
+        ref = R.log_likelihood_ratio(dets, src, q, m, lambda t: np.full(len(t), 1 / (hi - lo)))
+        q["geocent_time"] += q["time_jitter"]
+        parts = [R.snrs(d, src(d.frequency, **q), q, True) for d in dets]
+        scale = max(1.0, np.max(np.abs(sum(x[2] for x in parts))), sum(x[1] for x in parts) / 2)
+        mc = (q["mass_1"] * q["mass_2"]) ** 0.6 / (q["mass_1"] + q["mass_2"]) ** 0.2 * 4.925490947641267e-06
+        psi = 3 / 128 * (np.pi * mc * 20.0) ** (-5 / 3)
+        assert abs(got[i] - ref) <= max(1e-9, 8 * 2.0 ** -53 * psi) * scale, (i, got[i], ref)
+    an.close()
