@@ -2016,22 +2016,30 @@ int gwl_set_relative_binning_time_weights(gwl_analysis* a, const double* weights
   bin.back() = (int32_t)(idx.size() - 2);
   int rc;
   if ((rc = upload(a, &a->rb_bin, bin))) return rc;
-  // mixed precision: f_k - (f_b + f_b+1) / 2 of each grid index, in float32
-  std::vector<RbBinF> bx(bin.size());
-  for (size_t q = 0; q < bin.size(); ++q) {
-    const int32_t b = bin[q];
-    const double fc = (a->h_freq[idx[(size_t)b]] + a->h_freq[idx[(size_t)b + 1]]) / 2;
-    bx[q] = RbBinF{b, (float)(a->h_freq[(size_t)k0 + q] - fc)};
+  // mixed precision: f_k - (f_b + f_b+1) / 2 of each grid index, in float32, in
+  // the order of the windowed kernel's reads
+  std::vector<int32_t> order;
+  a->rb_bx = nullptr;
+  const bool windowed = window_relbin_order(a->n_bins - 1, &order);
+  if (windowed) {
+    std::vector<RbBinF> bx(order.size());
+    for (size_t q = 0; q < order.size(); ++q) {
+      const int64_t k = std::min(std::max<int64_t>(order[q], k0), k1);
+      const int32_t b = bin[(size_t)(k - k0)];
+      const double fc = (a->h_freq[idx[(size_t)b]] + a->h_freq[idx[(size_t)b + 1]]) / 2;
+      bx[q] = RbBinF{b, (float)(a->h_freq[(size_t)k] - fc)};
+    }
+    if ((rc = upload(a, &a->rb_bx, bx))) return rc;
   }
-  if ((rc = upload(a, &a->rb_bx, bx))) return rc;
   for (int d = 0; d < a->n_det; ++d) {
     std::vector<double2> w((size_t)a->n_bins);
     for (int64_t k = 0; k < a->n_bins; ++k)
       w[(size_t)k] = make_double2(weights[((size_t)d * a->n_bins + k) * 2], weights[((size_t)d * a->n_bins + k) * 2 + 1]);
-    std::vector<float2> wf(bin.size());
-    for (size_t q = 0; q < wf.size(); ++q)
-      wf[q] = make_float2((float)w[(size_t)k0 + q].x, (float)w[(size_t)k0 + q].y);
     if ((rc = upload(a, &a->rb_g[d], w))) return rc;
+    if (!windowed) continue;
+    std::vector<float2> wf(order.size(), make_float2(0.f, 0.f));
+    for (size_t q = 0; q < wf.size(); ++q)
+      if (order[q] >= k0 && order[q] <= k1) wf[q] = make_float2((float)w[(size_t)order[q]].x, (float)w[(size_t)order[q]].y);
     if ((rc = upload(a, &a->rb_gf[d], wf))) return rc;
   }
   a->rb_tm = 1;

@@ -4,6 +4,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <vector>
 #include <string>
 
 #include <cuda_runtime.h>
@@ -217,10 +218,11 @@ struct LaunchArgs {
   // [rb_index[0], rb_index[rb_edges - 1]]
   const double2* rb_g[kMaxDet];         // [n_bins]
   const int32_t* rb_bin;                // [rb_index[last] - rb_index[0] + 1]
-  // ... and for the mixed-precision kernel over the same span: the weights in
-  // float32 and, per grid index, its bin with f - (f_b + f_b+1) / 2
-  const float2* rb_gf[kMaxDet];         // [rb_index[last] - rb_index[0] + 1]
-  const RbBinF* rb_bx;                  // [rb_index[last] - rb_index[0] + 1]
+  // ... and for the mixed-precision kernel, in the order it reads them
+  // (window_relbin_order): the weights in float32, zero outside that span, and
+  // per grid index its bin with f - (f_b + f_b+1) / 2
+  const float2* rb_gf[kMaxDet];
+  const RbBinF* rb_bx;
   int tw_refine_only;                   // float64 windowed time marginalisation: only the marked points
   float2* tw_scratch;                   // mixed windowed multi-banding: [tw_scratch_slots][mb_points] banded values
   int64_t tw_scratch_slots;
@@ -405,6 +407,9 @@ cudaError_t launch_time_marg_marks(const LaunchArgs& a, cudaStream_t s);
 // four-step transform (gwl_marg_window.cu): whether this launch's shared
 // memory fits, and the launch (mixed precision: relative binning only).
 bool time_marg_window_fits(const LaunchArgs& a);
+// the grid index at each position of the mixed relative-binning tables (-1: none);
+// false where that kernel does not take the length
+bool window_relbin_order(int64_t n_fft, std::vector<int32_t>* order);
 bool time_marg_window_mixed_ready(const LaunchArgs& a);  // the mixed kernel's tables and work space are there
 bool time_marg_window_refine_fits(const LaunchArgs& a);  // the float64 recomputation of marked points fits
 int64_t time_marg_window_slots();                        // work-space slots of the mixed multi-banding kernel

@@ -31,6 +31,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <vector>
 
 #include "gwl_device.cuh"
 #include "gwl_internal.h"
@@ -88,12 +89,33 @@ __host__ __device__ constexpr int win_first_stages() {
   return MIXED ? 4 : 3;
 }
 
-// padding: one slot after every 16 elements of a column; the columns are
-// win_stride(N2) elements apart, 4 more than a multiple of 16, so that the G
-// columns' blocks written by one half-warp fall in different banks
+// padding: one slot after every 16 elements of a column and one after every
+// 256; the columns are win_stride(N2) elements apart, 4 more than a multiple of
+// 16, so that the G columns' blocks written by one half-warp (consecutive, or 16
+// blocks apart) fall in different banks
+__device__ __forceinline__ int win_pad(int q) { return q + (q >> 4) + (q >> 8); }
+__host__ __device__ constexpr int win_stride(int n2) { return ((n2 + n2 / 16 + n2 / 256 + 15) & ~15) + 4; }
 
-__device__ __forceinline__ int win_pad(int q) { return q + (q >> 4); }
-__host__ __device__ constexpr int win_stride(int n2) { return n2 + n2 / 16 + 4; }
+// Relative binning, mixed: the block of the first stages at slot s of a column's
+// 2^nb blocks.  Slots 8 h .. 8 h + 7 are blocks 2^(nb - 3) apart, whose elements
+// q = bitrev(b) are the consecutive 8 h .. 8 h + 7: a warp's grid indices are then N1
+// apart, and its lanes mostly in one bin of the relative binning.  With the tables
+// in the order of these reads (window_relbin_order) a warp's load takes two lines
+// where four consecutive indices at eight places took eight.  128 s at 4096 Hz,
+// three detectors, 256 points: 663 us to 503 us (the twiddles 1 and -i of the first
+// stages without a product took off 15 us of it); then bound by issue (55%) and
+// the tables' latency from L2, two CTAs per SM by registers and shared memory.
+__host__ __device__ __forceinline__ int win_slot_block(int s, int nb) {
+  if (nb < 3) return s;
+  int r = 0;
+  for (int t = s >> 3, i = 0; i < nb - 3; ++i, t >>= 1) r = 2 * r + (t & 1);
+  return ((s & 7) << (nb - 3)) | r;
+}
+__host__ __device__ __forceinline__ int win_reverse(int b, int nb) {
+  int r = 0;
+  for (int i = 0; i < nb; ++i, b >>= 1) r = 2 * r + (b & 1);
+  return r;
+}
 
 // s + e += y with s + e kept as an unevaluated float pair (Knuth's TwoSum;
 // the adds are explicit so that nothing is contracted or reordered)
@@ -420,8 +442,9 @@ __global__ void __launch_bounds__(kWinThreads, MIXED ? 2 : 1)
     __syncthreads();
     const int j_lo = (int)s_jr[0];
     const int n_win = (int)(s_jr[1] - s_jr[0] + 1);
-    // integrand z_k (k < L): 4/T sum_d h_d,k conj(d_k) / S_k
-    const auto integrand = [&](int k) -> C {
+    // integrand z_k (k < L): 4/T sum_d h_d,k conj(d_k) / S_k; at = position of k in
+    // the tables of mixed relative binning
+    const auto integrand = [&](int k, int at) -> C {
       C z;
       z.x = 0;
       z.y = 0;
@@ -456,12 +479,9 @@ __global__ void __launch_bounds__(kWinThreads, MIXED ? 2 : 1)
         return z;
       } else if constexpr (!MB) {
         if constexpr (MIXED) {
-          // float32: ratio r0 + r1 (f - f_b) times the weight 4/T h0 conj(d) / S;
-          // no branch around the loads (a clamped index and a zero factor
-          // outside the bins' span), so that those of several k are in flight
-          const int kc = min(max(k, k0), k1) - k0;
-          const float in = (k >= k0 && k <= k1) ? 1.f : 0.f;
-          const float2 bxw = __ldg(reinterpret_cast<const float2*>(a.rb_bx) + kc);
+          // float32: ratio r0 + r1 (f - f_b) times the weight 4/T h0 conj(d) / S
+          // (zero outside the bins' span)
+          const float2 bxw = __ldg(reinterpret_cast<const float2*>(a.rb_bx) + at);
           const RbBinF bx{__float_as_int(bxw.x), bxw.y};
           const float2* coef_lo = reinterpret_cast<const float2*>(coef + D * nB);
 #pragma unroll
@@ -469,12 +489,10 @@ __global__ void __launch_bounds__(kWinThreads, MIXED ? 2 : 1)
             const float4 c = coef[d * nB + bx.bin];
             const float2 cl = coef_lo[d * nB + bx.bin];
             const float rr = fmaf(c.z, bx.x, c.x) + cl.x, ri = fmaf(c.w, bx.x, c.y) + cl.y;
-            const float2 g = __ldg(a.rb_gf[d] + kc);
+            const float2 g = __ldg(a.rb_gf[d] + at);
             z.x += g.x * rr - g.y * ri;
             z.y += g.x * ri + g.y * rr;
           }
-          z.x *= in;
-          z.y *= in;
           z2 += z.x * z.x + z.y * z.y;
         } else {
           if (k < k0 || k > k1) return z;
@@ -543,7 +561,8 @@ __global__ void __launch_bounds__(kWinThreads, MIXED ? 2 : 1)
       // stages, the RN0-point DFT of the column's elements q + m N2 / RN0
       // (m < RN0), q = bitrev(b) over log2(N2) - RB0 bits.
       for (int bb = threadIdx.x; bb < G * n2q; bb += blockDim.x) {
-        const int g = bb % G, b = bb / G, n1 = n1_0 + g;
+        const int g = bb % G, n1 = n1_0 + g;
+        const int b = MIXED && SRC == kSrcRelbin ? win_slot_block(bb / G, log2n2 - RB0) : bb / G;
         const int q = log2n2 > RB0 ? (int)bit_reverse((uint32_t)b, log2n2 - RB0) : 0;
         C x[RN0];
         if constexpr (SRC == kSrcTf2) {
@@ -567,7 +586,7 @@ __global__ void __launch_bounds__(kWinThreads, MIXED ? 2 : 1)
           // register slot m holds element bitrev(m) (decimation in time)
           const int mm = (int)(__brev((unsigned)m) >> (32 - RB0));
           if (n1 < N1) {
-            x[m] = integrand(n1 + N1 * (q + mm * n2q));
+            x[m] = integrand(n1 + N1 * (q + mm * n2q), ((n1_0 / G) * RN0 + m) * (G * n2q) + bb);
           } else {
             x[m].x = 0;
             x[m].y = 0;
@@ -579,9 +598,15 @@ __global__ void __launch_bounds__(kWinThreads, MIXED ? 2 : 1)
 #pragma unroll
           for (int k = 0; k < RN0; ++k) {
             if (k & h) continue;
-            // exp(-2 pi i (k mod h) / (2 h)) = w16[(k mod h) 16 / (2 h)]
-            const C w = s_w16[(k & (h - 1)) * (8 >> s)];
-            const C t = cmul(w, x[k | h]);
+            // exp(-2 pi i (k mod h) / (2 h)) = w16[(k mod h) 16 / (2 h)], 1 and -i without a product
+            const int e = (k & (h - 1)) * (8 >> s);
+            C t = x[k | h];
+            if (e == 4) {
+              t.x = x[k | h].y;
+              t.y = -x[k | h].x;
+            } else if (e != 0) {
+              t = cmul(s_w16[e], x[k | h]);
+            }
             x[k | h].x = x[k].x - t.x;
             x[k | h].y = x[k].y - t.y;
             x[k].x = x[k].x + t.x;
@@ -872,6 +897,26 @@ cudaError_t launch_win(const LaunchArgs& a, cudaStream_t s) {
 }
 
 }  // namespace
+
+bool window_relbin_order(int64_t n_fft, std::vector<int32_t>* order) {
+  int m_odd = 0, log2N = 0;
+  if (!fft_length_supported(n_fft, &m_odd, &log2N) || n_fft >= ((int64_t)1 << 30)) return false;
+  constexpr int G = win_columns<true, kSrcRelbin>(), RB0 = win_first_stages<true>(), RN0 = 1 << RB0;
+  const int log2n2 = std::min(log2N, win_max_log2_col<true, kSrcRelbin>());
+  if (log2n2 < RB0) return false;
+  const int nb = log2n2 - RB0, n2q = 1 << nb;
+  const int64_t N1 = n_fft >> log2n2, groups = (N1 + G - 1) / G;
+  order->assign((size_t)(groups * RN0 * G * n2q), -1);
+  int32_t* o = order->data();
+  for (int64_t c = 0; c < groups; ++c)
+    for (int m = 0; m < RN0; ++m)
+      for (int bb = 0; bb < G * n2q; ++bb, ++o) {
+        const int64_t n1 = c * G + bb % G;
+        const int q = win_reverse(win_slot_block(bb / G, nb), nb), mm = win_reverse(m, RB0);
+        if (n1 < N1) *o = (int32_t)(n1 + N1 * (q + (int64_t)mm * n2q));
+      }
+  return true;
+}
 
 bool time_marg_window_mixed_ready(const LaunchArgs& a) {
   if (a.relbin) return a.rb_bx != nullptr;
