@@ -42,8 +42,11 @@ def params_block(params: dict, n: int | None = None) -> np.ndarray:
                 n = max(n, s[0])
     block = np.zeros((_capi.NPARAM, n), dtype=np.float64)
     for key, slot in _capi.SLOT.items():
-        if key in params and params[key] is not None:
-            block[slot] = np.broadcast_to(np.asarray(params[key], dtype=np.float64), (n,))
+        v = params.get(key)
+        if isinstance(v, float):  # one point: 25 us of numpy's broadcasting for the twelve scalars, 3 us without
+            block[slot] = v
+        elif v is not None:
+            block[slot] = np.broadcast_to(np.asarray(v, dtype=np.float64), (n,))
     return block
 
 

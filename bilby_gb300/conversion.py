@@ -56,19 +56,33 @@ def _component_masses(p):
 
 def convert_to_lal_binary_black_hole_parameters(parameters):
     """Returns (converted parameters, added keys) like the reference."""
+    original = list(parameters.keys())
+    converted = _converted(parameters, spins=True)
+    added = [k for k in converted if k not in original]
+    return converted, added
+
+
+def convert_to_kernel_parameters(parameters):
+    """The same conversion without the spin magnitudes and tilts, which the
+    aligned-spin kernels do not read."""
+    return _converted(parameters, spins=False)
+
+
+def _converted(parameters, spins):
     converted = dict(parameters)
     original = list(converted.keys())
     if "luminosity_distance" not in original and ("redshift" in original or "comoving_distance" in original):
         raise NotImplementedError("redshift / comoving-distance inputs need a cosmology: pass luminosity_distance")
     converted = _component_masses(converted)
-    for idx in ("1", "2"):
-        key = f"chi_{idx}"
-        if key in original and f"a_{idx}" not in original:
-            converted[f"a_{idx}"] = abs(converted[key])
-            converted[f"cos_tilt_{idx}"] = _xp(converted[key]).sign(converted[key])
-    for key in ("phi_jl", "phi_12"):
-        converted.setdefault(key, 0.0)
-    for angle in ("tilt_1", "tilt_2", "theta_jn"):
+    if spins:
+        for idx in ("1", "2"):
+            key = f"chi_{idx}"
+            if key in original and f"a_{idx}" not in original:
+                converted[f"a_{idx}"] = abs(converted[key])
+                converted[f"cos_tilt_{idx}"] = _xp(converted[key]).sign(converted[key])
+        for key in ("phi_jl", "phi_12"):
+            converted.setdefault(key, 0.0)
+    for angle in ("tilt_1", "tilt_2", "theta_jn") if spins else ("theta_jn",):
         if f"cos_{angle}" in converted:
             with np.errstate(invalid="ignore"):
                 converted[angle] = _xp(converted[f"cos_{angle}"]).arccos(converted[f"cos_{angle}"])
@@ -77,5 +91,4 @@ def convert_to_lal_binary_black_hole_parameters(parameters):
             xp = _xp(converted["delta_phase"])
             converted["phase"] = xp.remainder(converted["delta_phase"] - xp.sign(xp.cos(converted["theta_jn"]))
                                               * converted["psi"], 2 * np.pi)
-    added = [k for k in converted if k not in original]
-    return converted, added
+    return converted

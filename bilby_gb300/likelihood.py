@@ -24,6 +24,7 @@ import numpy as np
 
 from . import _capi
 from .analysis import Analysis, DetectorData, params_block
+from .conversion import convert_to_kernel_parameters, convert_to_lal_binary_black_hole_parameters
 from .source import model_of
 
 logger = logging.getLogger("bilby")
@@ -140,7 +141,10 @@ class ParameterPreparer:
     def prepare(self, parameters: dict) -> dict:
         p = dict(parameters)
         p.update(self.sky_frame(p))
-        converted, _ = self.parameter_conversion(dict(p))
+        if self.parameter_conversion is convert_to_lal_binary_black_hole_parameters:
+            converted = convert_to_kernel_parameters(p)
+        else:
+            converted, _ = self.parameter_conversion(dict(p))
         if self.jitter:
             converted["time_jitter"] = p.get("time_jitter", 0.0)
         missing = [k for k in REQUIRED_PARAMETERS[self.model] if converted.get(k) is None]
