@@ -355,10 +355,7 @@ static cudaError_t launch_wide_d(const LaunchArgs& a, cudaStream_t s) {
       cudaFuncSetAttribute(k_wide_tf2<D, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (set != cudaSuccess) return set;
   const int64_t tiles = (a.B + 31) / 32;
-  // up to eight tiles share a CTA's tables while the grid stays at eight CTAs
-  // per SM or more
-  int per = 1;
-  while (per < 8 && a.wide_chunks * (tiles / (2 * per)) >= 8 * 152) per *= 2;
+  const int per = wide_tiles(a.wide_chunks, tiles);
   const dim3 grid((unsigned)a.wide_chunks, (unsigned)((tiles + per - 1) / per));
   k_wide_tf2<D, CPLX><<<grid, kWideThreads, smem, s>>>(a, per);
   return cudaGetLastError();

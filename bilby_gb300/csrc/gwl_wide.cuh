@@ -169,6 +169,18 @@ __device__ __forceinline__ void wide_pair(uint64_t a0, uint64_t a1, const uint4&
   }
 }
 
+// Tiles of 32 points that share a CTA's tables: one, as long as that leaves fewer
+// than 16,000 CTAs.  A CTA's work depends on its points' bands, and small ones fill
+// the gaps: measured per call, 1 / 2 / 4 / 8 tiles, sine-Gaussian 10,000 points 520 /
+// 541 / 574 / 703 us, 20,000 points 923 / 937 / 984 / 1061 us, multi-banding 4001 points
+// 613 / 616 / 651 / 678 us; 128 s, 512 points (16,000 CTAs) 1251 / 1247 / 1249 / 1265 us,
+// 2048 points 4707 / 4657 / 4661 / 4668 us.
+inline int wide_tiles(int64_t chunks, int64_t tiles) {
+  int per = 1;
+  while (per < 8 && chunks * (tiles / (2 * per)) >= 8192) per *= 2;
+  return per;
+}
+
 // Lanes that add one point's chunks: lane l of them takes chunks l, l + n, ...,
 // then a fixed tree.  With 17 chunks (4 s at 2048 Hz) a whole warp per point
 // took 81 us for 10,000 points, nearly all of it in the tree's float64 adds.

@@ -462,8 +462,7 @@ static cudaError_t launch_wide_sg_d(const LaunchArgs& a, cudaStream_t s) {
       cudaFuncSetAttribute(k_wide_sg<D, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (set != cudaSuccess) return set;
   const int64_t tiles = (a.B + 31) / 32;
-  int per = 1;
-  while (per < 8 && a.n_chunks * (tiles / (2 * per)) >= 8 * 152) per *= 2;
+  const int per = wide_tiles(a.n_chunks, tiles);
   const dim3 grid((unsigned)a.n_chunks, (unsigned)((tiles + per - 1) / per));
   k_wide_sg<D, CPLX><<<grid, kWideThreads, smem, s>>>(a, per);
   return cudaGetLastError();
