@@ -237,44 +237,66 @@ __global__ void __launch_bounds__(kPairThreads) k_wide_tf2_few(LaunchArgs a) {
 // The chunks' sums in a fixed order, the totals and the lnL.
 constexpr int kWideFinThreads = 128;
 
+// <h|h>_d per A0^2 |Q|^2 and norm, in every lane of the point's lanes
+__device__ __forceinline__ double wide_hh(const LaunchArgs& a, const PointRec& r, int64_t i, int d, int lane, int lanes) {
+  if (!a.wide_sub) {
+    const int64_t k1 = min(r.k_end, a.n_bins), k0 = min(r.k_start, k1);
+    return a.hh_prefix[d][k1] - a.hh_prefix[d][k0];
+  }
+  const int64_t end = wide_end(a, i);
+  double s = 0.0;
+  for (int b = lane; b < a.wide_bands; b += lanes) {
+    const int4 v = a.wide_band[b];
+    const int64_t n = end > v.z ? min((end - v.z + v.w - 1) / v.w, (int64_t)v.y) : 0;
+    s += a.wide_q[d][v.x + n] - a.wide_q[d][v.x];
+  }
+  for (int o = lanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+// (one compiled body, so that both kernels below round alike)
+__device__ __noinline__ void wide_totals(const LaunchArgs& a, int64_t i, const double* p, const double* sum) {
+  const PointRec& r = a.rec[i];
+  const int nc = a.cplx ? 2 : 1;
+  double dr = 0.0, di = 0.0, hh = r.valid ? mb_fft_hh_total(a, i) : 0.0;
+  for (int d = 0; d < a.n_det; ++d) {
+    double x, z;
+    tf2_project(a, r, d, a.wide_norm * a.wide_wscale[d], p + d * nc, &x, &z);
+    dr += x;
+    di += z;
+    hh += tf2_norm(r, d, a.wide_norm, sum[d]);
+  }
+  finish_point(a, r, i, dr, di, hh);
+}
+
 __global__ void __launch_bounds__(kWideFinThreads) k_wide_finalize(LaunchArgs a) {
   const int lanes = wide_lanes(a.wide_chunks), lane = threadIdx.x & (lanes - 1);
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / lanes, i = min(slot, a.B - 1);
-  const PointRec& r = a.rec[i];
   const int nc = a.cplx ? 2 : 1;
-  double p[2 * kMaxDet];
-  for (int c = 0; c < a.n_det * nc; ++c) {
-    const double* q = a.part + (i * a.n_det * nc + c) * a.wide_chunks;
-    p[c] = wide_chunk_sum(q, a.wide_chunks, lane, lanes);
+  double p[2 * kMaxDet], sum[kMaxDet];
+  for (int c = 0; c < a.n_det * nc; ++c)
+    p[c] = wide_chunk_sum(a.part + (i * a.n_det * nc + c) * a.wide_chunks, a.wide_chunks, lane, lanes);
+  for (int d = 0; d < a.n_det; ++d) sum[d] = wide_hh(a, a.rec[i], i, d, lane, lanes);
+  if (lane == 0 && slot < a.B) wide_totals(a, i, p, sum);
+}
+
+// Few points: a CTA per point and a warp per sum, 32 loads in flight per lane; the
+// additions are those of k_wide_finalize.  Bound by the latency of the chain: one
+// point of the 128 s segment (1015 chunks) 21.5 us there, 12.0 us here.
+__global__ void __launch_bounds__(64 * kMaxDet) k_wide_finalize_few(LaunchArgs a) {
+  __shared__ double s_p[2 * kMaxDet], s_sum[kMaxDet];
+  const int lanes = wide_lanes(a.wide_chunks), lane = threadIdx.x & (lanes - 1);
+  const int nc = a.cplx ? 2 : 1, c = threadIdx.x >> 5, d = c / nc;
+  const int64_t i = blockIdx.x;
+  double h = 0.0;
+  if (c == d * nc) h = wide_hh(a, a.rec[i], i, d, lane, lanes);
+  const double p = wide_chunk_sum<32>(a.part + (i * a.n_det * nc + c) * a.wide_chunks, a.wide_chunks, lane, lanes);
+  if ((threadIdx.x & 31) == 0) {
+    s_p[c] = p;
+    if (c == d * nc) s_sum[d] = h;
   }
-  double sum[kMaxDet];  // <h|h> per A0^2 |Q|^2 and norm
-  for (int d = 0; d < a.n_det; ++d) {
-    if (!a.wide_sub) {
-      const int64_t k1 = min(r.k_end, a.n_bins), k0 = min(r.k_start, k1);
-      sum[d] = a.hh_prefix[d][k1] - a.hh_prefix[d][k0];
-      continue;
-    }
-    const int64_t end = wide_end(a, i);
-    double s = 0.0;
-    for (int b = lane; b < a.wide_bands; b += lanes) {
-      const int4 v = a.wide_band[b];
-      const int64_t n = end > v.z ? min((end - v.z + v.w - 1) / v.w, (int64_t)v.y) : 0;
-      s += a.wide_q[d][v.x + n] - a.wide_q[d][v.x];
-    }
-    for (int o = lanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    sum[d] = s;
-  }
-  if (lane == 0 && slot < a.B) {
-    double dr = 0.0, di = 0.0, hh = r.valid ? mb_fft_hh_total(a, i) : 0.0;
-    for (int d = 0; d < a.n_det; ++d) {
-      double x, z;
-      tf2_project(a, r, d, a.wide_norm * a.wide_wscale[d], p + d * nc, &x, &z);
-      dr += x;
-      di += z;
-      hh += tf2_norm(r, d, a.wide_norm, sum[d]);
-    }
-    finish_point(a, r, i, dr, di, hh);
-  }
+  __syncthreads();
+  if (threadIdx.x == 0) wide_totals(a, i, s_p, s_sum);
 }
 
 // ---------------------------------------------------------------------------
@@ -374,7 +396,11 @@ cudaError_t launch_wide(const LaunchArgs& a, cudaStream_t s) {
     default: e = launch_wide_d<4, true>(a, s); break;
   }
   if (e != cudaSuccess) return e;
-  k_wide_finalize<<<(unsigned)((a.B * wide_lanes(a.wide_chunks) + kWideFinThreads - 1) / kWideFinThreads), kWideFinThreads, 0, s>>>(a);
+  if (wide_few(a.B, a.wide_chunks))
+    k_wide_finalize_few<<<(unsigned)a.B, 32 * a.n_det * (a.cplx ? 2 : 1), 0, s>>>(a);
+  else
+    k_wide_finalize<<<(unsigned)((a.B * wide_lanes(a.wide_chunks) + kWideFinThreads - 1) / kWideFinThreads), kWideFinThreads,
+                      0, s>>>(a);
   return cudaGetLastError();
 }
 

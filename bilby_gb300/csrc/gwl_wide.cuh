@@ -186,15 +186,26 @@ inline int wide_tiles(int64_t chunks, int64_t tiles) {
 // took 81 us for 10,000 points, nearly all of it in the tree's float64 adds.
 __host__ __device__ __forceinline__ int wide_lanes(int64_t n_chunks) { return n_chunks > 256 ? 32 : (n_chunks > 32 ? 8 : 4); }
 
+// N: loads in flight per lane
+template <int N = 8>
 __device__ __forceinline__ double wide_chunk_sum(const double* q, int64_t n, int lane, int lanes) {
   double s = 0.0;
   int64_t g = lane;
-  for (; g + 7 * lanes < n; g += 8 * lanes) {  // eight loads in flight
-    double v[8];
+  for (; g + (N - 1) * lanes < n; g += N * lanes) {
+    double v[N];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = q[g + u * lanes];
+    for (int u = 0; u < N; ++u) v[u] = q[g + u * lanes];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) s += v[u];
+    for (int u = 0; u < N; ++u) s += v[u];
+  }
+  if (N > 8) {  // the rest by 8, then one by one
+    for (; g + 7 * lanes < n; g += 8 * lanes) {
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = q[g + u * lanes];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s += v[u];
+    }
   }
   for (; g < n; g += lanes) s += q[g];
   for (int o = lanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
