@@ -271,10 +271,33 @@ __device__ __forceinline__ uint64_t tm_cycles(const TmPlan& p, uint64_t x) { ret
 __host__ __device__ constexpr int tm_threads(int log2m) { return log2m <= 12 ? (1 << log2m) / 8 : 512; }
 __host__ __device__ constexpr int tm_slots(int log2m) { return (1 << log2m) + (1 << log2m) / 8; }
 
-// One CTA per point.  Bound by latency and, at the samples' ln I0 and exp, by the
-// float64 pipe (55% of its cycles; the transforms leave it idle).  6 s at 2048 Hz,
-// two detectors, 2047 points, phase marginalised: 231 us, where the whole
-// float64 transform through global memory (k_time_marg) took 2240 us.  The error
+// Over the CTA, in a fixed order; red: a double per warp.
+__device__ __forceinline__ double block_max(double v, double* red) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  for (int w = 0; w < (int)blockDim.x / 32; ++w) v = fmax(v, red[w]);
+  return v;
+}
+__device__ __forceinline__ double block_sum(double v, double* red) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = 0.0;
+  for (int w = 0; w < (int)blockDim.x / 32; ++w) v += red[w];
+  return v;
+}
+
+constexpr double kTmBesselMax = 500.0;  // as ln_i0: I0(500) = 2.5e215, and its sum over the samples, are in range
+
+// One CTA per point.  Bound by latency and, at the samples' I0, by the float64
+// pipe (the transforms leave it idle).  6 s at 2048 Hz, two detectors, 2047 points,
+// phase marginalised: 189 us (231 us with a logarithm and an exponential per sample),
+// where the whole float64 transform through global memory (k_time_marg) took 2240 us.  The error
 // of a sample's <d|h> against 80-bit arithmetic, relative to the largest: 3e-15 rms
 // (k_time_marg 6e-15).
 template <int LOGM>
@@ -295,7 +318,7 @@ __global__ void __launch_bounds__(tm_threads(LOGM)) k_wide_tm(LaunchArgs a, TmPl
     return;
   }
   const int64_t L = a.n_fft;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, D = a.n_det;
+  const int D = a.n_det;
   if (threadIdx.x == 0) {
     // candidate window from the real-valued bounds, checked exactly per sample
     const double jl = floor((a.t_min - a.start_time0 - r.jitter) / a.tm_step) - 3.0;
@@ -400,47 +423,62 @@ __global__ void __launch_bounds__(tm_threads(LOGM)) k_wide_tm(LaunchArgs a, TmPl
     }
     __syncthreads();
   }
-  // the samples' lnL, their maximum, sum exp(l - max) in a fixed order
+  // The samples: with phase marginalisation alone the sum of their I0 itself where
+  // the largest argument leaves it in range (168 float64 instructions per sample
+  // with a logarithm and an exponential around each I0, 110 without), else their
+  // lnL and sum exp(l - max); sums in a fixed order.
   const double hh = s_hh[0], scale = s_hh[2], sr = r.dist / a.ref_dist, jit = r.jitter;
+  const bool bessel = a.phase_marg && !a.dist_marg;
   double most = -INFINITY;
   for (int t = threadIdx.x; t < n; t += T) {
-    double lw, l = -INFINITY;
-    if (tm_log_weight<false>(a, tm_sample_time(a, j0 + t, L, a.tm_step, jit), lw)) {
+    double pw = 1.0, l = -INFINITY;  // l: |X| with phase marginalisation alone
+    const double time = tm_sample_time(a, j0 + t, L, a.tm_step, jit);
+    if (a.tm_prior) pw = tm_prior_density(a, time);
+    if (time >= a.t_min && time <= a.t_max && pw > 0.0) {
       const float4 v = acc[t];
       const double xr = scale * ((double)v.x + (double)v.z), xi = scale * ((double)v.y + (double)v.w);
       if (a.dist_marg) {
         const double dx = a.phase_marg ? sqrt(xr * xr + xi * xi) * sr : xr * sr;
         l = bicubic_at(a.tx, a.nx, a.ny, a.tc, a.bbox, dx, s_ly, s_hy);
-      } else if (a.phase_marg) {
-        l = ln_i0(sqrt(xr * xr + xi * xi)) - hh / 2;
       } else {
-        l = xr - hh / 2;
+        l = bessel ? sqrt(xr * xr + xi * xi) : xr - hh / 2;
       }
-      l += lw;
+      if (!bessel && a.tm_prior) l += log(pw);
     }
     most = fmax(most, l);
-    *reinterpret_cast<double*>(acc + t) = l;
+    *reinterpret_cast<double2*>(acc + t) = make_double2(l, pw);
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) most = fmax(most, __shfl_xor_sync(0xffffffffu, most, o));
-  if (lane == 0) s_red[warp] = most;
-  __syncthreads();
-  for (int w = 0; w < kWarps; ++w) most = fmax(most, s_red[w]);
+  most = block_max(most, s_red);
+  if (bessel && !(most < kTmBesselMax)) {
+    most = -INFINITY;
+    for (int t = threadIdx.x; t < n; t += T) {
+      double2* v = reinterpret_cast<double2*>(acc + t);
+      if (!(v->x >= 0.0)) continue;
+      v->x = ln_i0(v->x) - hh / 2;
+      if (a.tm_prior) v->x += log(v->y);
+      most = fmax(most, v->x);
+    }
+    most = block_max(most, s_red);
+  } else if (bessel) {
+    double sum = 0.0;
+    for (int t = threadIdx.x; t < n; t += T) {
+      const double2 v = *reinterpret_cast<const double2*>(acc + t);
+      if (v.x >= 0.0) sum += v.y * cyl_bessel_i0(v.x);
+    }
+    sum = block_sum(sum, s_red);
+    if (threadIdx.x == 0)
+      a.out[i] = isfinite(most) ? log(sum * (a.tm_prior ? 1.0 : 1.0 / (a.t_max - a.t_min)) * a.delta_tc) - hh / 2 : most;
+    return;
+  }
   double sum = 0.0;
   if (isfinite(most))
     for (int t = threadIdx.x; t < n; t += T) {
-      const double l = *reinterpret_cast<const double*>(acc + t);
+      const double l = reinterpret_cast<const double2*>(acc + t)->x;
       if (isfinite(l)) sum += exp(l - most);
     }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  __syncthreads();
-  if (lane == 0) s_red[warp] = sum;
-  __syncthreads();
+  sum = block_sum(sum, s_red);
   if (threadIdx.x == 0) {
-    double total = 0.0;
-    for (int w = 0; w < kWarps; ++w) total += s_red[w];
-    total *= (a.tm_prior ? 1.0 : 1.0 / (a.t_max - a.t_min)) * a.delta_tc;
+    const double total = sum * (a.tm_prior ? 1.0 : 1.0 / (a.t_max - a.t_min)) * a.delta_tc;
     a.out[i] = isfinite(most) ? most + log(total) : most;
   }
 }

@@ -59,3 +59,35 @@ def test_against_the_oracle(gpu, detectors, duration, fs, masses, samples, phase
         psi = 3 / 128 * (np.pi * mc * 20.0) ** (-5 / 3)
         assert abs(got[i] - ref) <= max(1e-9, 8 * 2.0 ** -53 * psi) * scale, (i, got[i], ref)
     an.close()
+
+
+# the sum of the samples' I0 below 500, their lnL above; a flat and a tabulated prior
+@pytest.mark.parametrize("tabulated", [False, True])
+@pytest.mark.parametrize("largest", [3.0, 499.0, 501.0, 5000.0])
+def test_loudness(gpu, largest, tabulated):
+    w = small_workload("tf2_marg_8s", duration=4.0, sampling_frequency=2048.0)
+    w = small_workload("tf2_marg_8s", **{**w.__dict__, "injection": dict(w.injection, geocent_time=w.start_time + 2.0)})
+    dets = OD.build_workload(w)
+    an = device_analysis(dets, "taylorf2", w)
+    lo, hi = w.start_time + 1.9, w.start_time + 2.1
+    an.set_time_marginalization(True, True, lo, hi)
+    an.set_phase_marginalization(True)
+    density = lambda t: np.full(np.shape(t), 1 / (hi - lo))
+    if tabulated:  # linear in time: exact in the four-node interpolation
+        h, t0 = 2.0 ** -8, np.floor(lo * 2 ** 8 - 2) * 2.0 ** -8
+        nodes = t0 + h * np.arange(int((hi - t0) / h) + 4)
+        density = lambda t: 5.0 + 20.0 * (np.asarray(t) - (w.start_time + 2.0))
+        an.set_time_prior(np.maximum(density(nodes), 0.0), t0, h)
+    m = R.Marginalization(time=True, phase=True)
+    R.setup_time_marginalization(m, w.start_time, w.duration, w.sampling_frequency, lo, hi)
+    src = OD.source_for(w.model, w.minimum_frequency)
+    q = dict(w.injection, phase=0.0, geocent_time=w.start_time, time_jitter=1e-4)
+    late = dict(q, geocent_time=w.start_time + 1e-4)
+    arr = sum(R.snrs(d, src(d.frequency, **late), late, True)[2] for d in dets)
+    inside = (m.times + 1e-4 >= lo) & (m.times + 1e-4 <= hi)
+    q["luminosity_distance"] *= np.max(np.abs(arr[inside])) / largest
+    ref = R.log_likelihood_ratio(dets, src, q, m, density)
+    hh = sum(R.snrs(d, src(d.frequency, **q), q)[1] for d in dets)
+    got = an.log_likelihood_ratio_host(params_block(q), "fp64")[0]
+    assert abs(got - ref) <= 1e-9 * max(1.0, largest, hh / 2), (got, ref)
+    an.close()
