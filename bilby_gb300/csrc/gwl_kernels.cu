@@ -78,9 +78,12 @@ __device__ __forceinline__ uint64_t wide_shift(const LaunchArgs& a, double dt) {
   return to_wide(v, fma(dt, a.step, -v) + dt * a.step_lo);
 }
 
-__device__ __forceinline__ void wide_coefficients(const LaunchArgs& a, int64_t i, double m1, double m2, double eta,
-                                                  double m_sec, double u, double f_isco, int64_t k_end, const double* pn,
-                                                  const double* c, double cconst) {
+// 1 / x, x > 0, to float32's digits: for the low word of a quotient
+__device__ __forceinline__ double rough_inverse(double x) { return (double)(1.0f / fmaxf((float)x, 1e-37f)); }
+
+__device__ __forceinline__ void wide_coefficients(const LaunchArgs& a, int64_t i, double m1, double m2, double m_sec,
+                                                  double u, double f_isco, int64_t k_end, const double* pn, const double* c,
+                                                  double P, double cconst) {
   uint64_t* w = a.wide_c + i;
   // c_0 = 3 / (128 eta) (pi M)^(-5/3) / (2 pi) = K M^(1/3) / (m1 m2) to twice
   // float64's digits: its relative error is the same in every bin, where the
@@ -88,14 +91,14 @@ __device__ __forceinline__ void wide_coefficients(const LaunchArgs& a, int64_t i
   const double kh = 388209.13757985964, kl = -1.9320279142889344e-11;  // 3 / (256 pi) (pi G M_sun / c^3)^(-5/3)
   const double m = m1 + m2, ml = m1 > m2 ? m2 - (m - m1) : m1 - (m - m2);
   const double y = cbrt(m), p = y * y, pe = fma(y, y, -p), t = p * y, te = fma(p, y, -t) + pe * y;
-  const double yl = ((m - t) - te + ml) / (3.0 * p);
+  const double yl = ((m - t) - te + ml) * rough_inverse(3.0 * p);
   const double nh = kh * y, nl = fma(kh, y, -nh) + (kh * yl + kl * y);
   const double dh = m1 * m2, dl = fma(m1, m2, -dh), id = 1.0 / dh;
   const double q0 = nh * id, q1 = (fma(-q0, dh, nh) + (nl - q0 * dl)) * id;
   // the others as the mixed kernels have them, u = (pi M)^(1/3); ln f relative to wide_lnref
   double x[kNumBasis], xl = q1;
   x[0] = q0;
-  const double P = 3.0 / (128.0 * eta * kTwoPi), ip = P / (kPi * m_sec);
+  const double ip = P / (kPi * m_sec);
   x[1] = ip * pn[2];
   x[2] = ip * pn[3] * u;
   x[3] = ip * pn[4] * u * u;
@@ -132,9 +135,9 @@ __device__ __forceinline__ void wide_coefficients_sg(const LaunchArgs& a, int64_
                                                      int64_t& k_end) {
   uint64_t* w = a.wide_c + i;
   const double ch = 0.8493218002880191, cl = -2.5959464104597403e-17;
-  double q0 = f0 / a.step, q1 = (fma(-q0, a.step, f0) - q0 * a.step_lo) / a.step;
+  double q0 = f0 / a.step, q1 = (fma(-q0, a.step, f0) - q0 * a.step_lo) * rough_inverse(a.step);
   const double nh = fabs(Q) * ch, nl = fma(fabs(Q), ch, -nh) + fabs(Q) * cl;
-  double s0 = nh / q0, s1 = (fma(-s0, q0, nh) + (nl - s0 * q1)) / q0;
+  double s0 = nh / q0, s1 = (fma(-s0, q0, nh) + (nl - s0 * q1)) * rough_inverse(q0);
   const double far = q0 * 3.469446951953614e-18;  // beyond 2^58 bins f - f0 = -f0 in float64 too
   if (far > 1.0) {
     q0 /= far;
@@ -144,17 +147,18 @@ __device__ __forceinline__ void wide_coefficients_sg(const LaunchArgs& a, int64_
   }
   k_start = k_end = 0;
   if (!(q0 > 0.0 && isfinite(far) && s0 > 0.0 && isfinite(s0))) q0 = s0 = 1.0, q1 = s1 = 0.0;  // (an invalid point)
+  const double is = 1.0 / s0;
   const int frac = 61 - ilogb(q0 + (double)a.n_bins + 2.0), es = ilogb(s0) + 1;
   const uint64_t sm = (uint64_t)ldexp(s0, 64 - es), sv = sm + (uint64_t)(int64_t)ldexp(s1, 64 - es);
   w[0] = (uint64_t)(__double2ll_rn(ldexp(q0, frac)) + __double2ll_rn(ldexp(q1, frac)));
   w[a.B] = (sv >> 63) ? sv : sm;
   w[2 * a.B] = ((uint64_t)frac << 32) | (uint32_t)(es + 58 - frac);
-  w[3 * a.B] = (uint64_t)ldexp(fmin(sqrt(1020.0) / s0, ldexp(1.0, 62 - frac)), frac);
+  w[3 * a.B] = (uint64_t)ldexp(fmin(sqrt(1020.0) * is, ldexp(1.0, 62 - frac)), frac);
   // y < 1020 (float64's exponential underflows at 1075) and within 100 of the
   // smallest in-band y
   const double lo = (double)a.k_lo, hi = (double)(a.k_hi - 1), x = fmax(0.0, fmax(lo - q0, q0 - hi)), y = s0 * x * (s0 * x);
   if (y < 1020.0) {
-    const double R = sqrt(fmin(y + 100.0, 1020.0)) / s0;
+    const double R = sqrt(fmin(y + 100.0, 1020.0)) * is;
     k_start = (int64_t)fmin(fmax(ceil(q0 - R), lo), hi);
     k_end = (int64_t)fmin(fmax(floor(q0 + R), lo), hi) + 1;
   }
@@ -167,10 +171,15 @@ __device__ __forceinline__ void wide_coefficients_sg(const LaunchArgs& a, int64_
 // float64 chains of a point, in three steps with a barrier between them.
 //   1. sidereal time and hour angle | the other angles | the source's scalars and
 //      band | the phase coefficients
-//   2. warp d: detector d; the last warp also the phase basis coefficients
+//   2. warp d: detector d; the last warp also the phase basis coefficients, or the
+//      sine-Gaussian's coefficients and band where it has no detector
 //   3. the error bound, the ordering key, the time marginalisation's scalars
 // One thread per point took 38 us (sine-Gaussian) to 76 us (float64 TaylorF2) for
-// a single point and for thousands alike: the latency of one float64 chain.
+// a single point and for thousands alike: the latency of one float64 chain.  A
+// float64 instruction takes 64 cycles of its quarter of the SM whatever the active
+// lanes, so the count per warp is the time: 10,500 + 16,800 cycles for steps 1 and 2
+// of TaylorF2, 8,900 + 11,400 of a burst (15 us; 15,000 + 11,700 with its coefficients
+// in step 1 and two more divisions).
 constexpr int kProloguePoints = 32;
 constexpr int kPrologueWarps = 4;
 
@@ -178,7 +187,7 @@ struct PrologueShared {
   double sphi[kProloguePoints], cphi[kProloguePoints], sth[kProloguePoints], cth[kProloguePoints];
   double sps[kProloguePoints], cps[kProloguePoints], sphi_ant[kProloguePoints], cphi_ant[kProloguePoints];
   double cos_i[kProloguePoints], amp[kProloguePoints], amp2[kProloguePoints];
-  double u[kProloguePoints], lnu[kProloguePoints], f_isco[kProloguePoints], hh[kMaxDet][kProloguePoints];
+  double u[kProloguePoints], f_isco[kProloguePoints], hh[kMaxDet][kProloguePoints];
   double qabs[kMaxDet][kProloguePoints], pn[8][kProloguePoints], pl[8][kProloguePoints];
   int64_t k_start[kProloguePoints], k_end[kProloguePoints];
   int ok[2][kProloguePoints];
@@ -223,10 +232,10 @@ __device__ __forceinline__ void prologue_detector(const LaunchArgs& a, PrologueS
     // Re <d|h>_d = |Q_d| Re sum w e^{i (phase_k + alpha_d)}, alpha_d = arg(conj(Q_d)): the real-part
     // kernels carry alpha_d as a constant phase offset of detector d
     const double ci = sh.cos_i[t], amp = sh.amp[t];
-    const double qr = fp * (1.0 + ci * ci) / 2.0, qi = -fx * ci, qabs = hypot(qr, qi);
+    const double qr = fp * (1.0 + ci * ci) / 2.0, qi = -fx * ci, qabs = sqrt(fma(qr, qr, qi * qi));
     r.qabs[d] = qabs;
     sh.qabs[d][t] = qabs;
-    const uint64_t u = a.cplx ? 0ull : fixed_fraction(atan2(-qi, qr) / kTwoPi);
+    const uint64_t u = a.cplx ? 0ull : fixed_fraction(div_const(atan2(-qi, qr), kTwoPi, 1.0 / kTwoPi));
     put_fixed(r.qfix[d], u);
     if (a.wide_c) a.wide_c[(int64_t)(kNumBasis + 2 + kMaxDet + d) * a.B + i] = u;
     if (tm) {
@@ -238,13 +247,21 @@ __device__ __forceinline__ void prologue_detector(const LaunchArgs& a, PrologueS
     }
   } else {
     const double A = fp * sh.amp[t], C = fx * sh.amp2[t];
-    if (a.wide_c) a.wide_c[(int64_t)(kNumBasis + 2 + kMaxDet + d) * a.B + i] = to_wide(atan2(C, A) / kTwoPi, 0.0);
+    if (a.wide_c) a.wide_c[(int64_t)(kNumBasis + 2 + kMaxDet + d) * a.B + i] = to_wide(div_const(atan2(C, A), kTwoPi, 1.0 / kTwoPi), 0.0);
     if (tm) {
       r.tm_coef[2 * d] = (float)(norm * a.w_scale[d] * fp * sh.amp[t]);
       r.tm_coef[2 * d + 1] = (float)(norm * a.w_scale[d] * fx * sh.amp2[t]);
       sh.hh[d][t] = 0.0;
     }
   }
+}
+
+// The sine-Gaussian's coefficients and band.
+__device__ __forceinline__ void sg_band(const LaunchArgs& a, PrologueShared& sh, PointRec& r, int64_t i, int t) {
+  int64_t k0 = 0, k1 = 0;
+  if (a.wide_c) wide_coefficients_sg(a, i, par(a, GWL_P_Q, i), par(a, GWL_P_FREQUENCY, i), k0, k1);
+  r.k_start = sh.k_start[t] = k0;
+  r.k_end = sh.k_end[t] = k1;
 }
 
 // (not inlined: one compiled body for one and for several analyses, so that a point
@@ -256,6 +273,7 @@ __device__ __noinline__ void prologue_cta(const LaunchArgs& a, PrologueShared& s
   // base.py:427-428: the jitter is added to geocent_time before projection.
   const double jitter = have && a.time_marg && a.jitter ? par(a, GWL_P_TIME_JITTER, i) : 0.0;
   const double tgeo = have ? par(a, GWL_P_GEOCENT_TIME, i) + jitter : 0.0;
+  const bool late = a.n_det < kPrologueWarps;  // the last warp has no detector in step 2
   if (have) {
     if (role == 0) {
       const double ra = par(a, GWL_P_RA, i);
@@ -294,10 +312,7 @@ __device__ __noinline__ void prologue_cta(const LaunchArgs& a, PrologueShared& s
       sh.amp2[t] = amp2;
       sh.ok[1][t] = isfinite(amp) && isfinite(amp2) && isfinite(sg_a) && f0 > 0;
     } else if (role == 3 && !tf2) {
-      int64_t k0 = 0, k1 = 0;
-      if (a.wide_c) wide_coefficients_sg(a, i, par(a, GWL_P_Q, i), par(a, GWL_P_FREQUENCY, i), k0, k1);
-      r.k_start = sh.k_start[t] = k0;
-      r.k_end = sh.k_end[t] = k1;
+      if (!late) sg_band(a, sh, r, i, t);
     } else if (role == 2) {
       const double m1 = par(a, GWL_P_MASS_1, i), m2 = par(a, GWL_P_MASS_2, i), dl = par(a, GWL_P_LUMINOSITY_DISTANCE, i);
       const double phase = par(a, GWL_P_PHASE, i), m = m1 + m2, m_sec = m * kMtsunSI, eta = m1 * m2 / (m * m);
@@ -305,7 +320,7 @@ __device__ __noinline__ void prologue_cta(const LaunchArgs& a, PrologueShared& s
       // band [k_start, k_end): f >= minimum_frequency and f < f_isco; k_end is
       // the first k with freq[k] >= f_isco: guessed from the uniform grid and
       // corrected against the frequency array (binary search if that fails)
-      int64_t ke = (int64_t)fmin(fmax(ceil(f_isco / a.step), 0.0), (double)a.n_bins);
+      int64_t ke = (int64_t)fmin(fmax(ceil(f_isco * a.duration), 0.0), (double)a.n_bins);
       for (int q = 0; q < 4 && ke > 0 && a.freq[ke - 1] >= f_isco; ++q) --ke;
       for (int q = 0; q < 4 && ke < a.n_bins && a.freq[ke] < f_isco; ++q) ++ke;
       if ((ke > 0 && a.freq[ke - 1] >= f_isco) || (ke < a.n_bins && a.freq[ke] < f_isco)) {
@@ -325,12 +340,11 @@ __device__ __noinline__ void prologue_cta(const LaunchArgs& a, PrologueShared& s
       r.phase = phase;
       // Mc^(5/6) = eta^(1/2) M^(5/6) and M^(5/6) = M (cbrt(pi) / u)^(1/2) with u = (pi M)^(1/3)
       const double u = cbrt(kPi * m_sec);
-      const double mc56 = sqrt(eta) * m_sec * sqrt(1.4645918875615231 / u);
+      const double mc56 = m_sec * sqrt(eta * 1.4645918875615231 / u);
       // sqrt(5/24) pi^(-2/3)
       const double amp = 0.45643546458763845 * 0.46619407703541166 * mc56 * kSpeedOfLight / (dl * 1e6 * kPcSI);
       r.amp = sh.amp[t] = amp;
       sh.u[t] = u;
-      sh.lnu[t] = log(u);
       sh.ok[1][t] = m1 > 0 && m2 > 0 && dl > 0 && isfinite(amp) && isfinite(phase) &&
                     isfinite(par(a, GWL_P_CHI_1, i)) && isfinite(par(a, GWL_P_CHI_2, i));
     } else {
@@ -347,25 +361,26 @@ __device__ __noinline__ void prologue_cta(const LaunchArgs& a, PrologueShared& s
   __syncthreads();
   if (have) {
     for (int d = role; d < a.n_det; d += kPrologueWarps) prologue_detector(a, sh, r, i, t, d, tgeo, tf2);
+    if (role == kPrologueWarps - 1 && !tf2 && late) sg_band(a, sh, r, i, t);
     if (role == kPrologueWarps - 1 && tf2) {
       const double m1 = par(a, GWL_P_MASS_1, i), m2 = par(a, GWL_P_MASS_2, i), phase = par(a, GWL_P_PHASE, i);
-      const double m = m1 + m2, m_sec = m * kMtsunSI, eta = m1 * m2 / (m * m), u = sh.u[t], lnu = sh.lnu[t];
+      const double m = m1 + m2, m_sec = m * kMtsunSI, eta = m1 * m2 / (m * m), u = sh.u[t], lnu = log(u);
       double pn[8], l5 = sh.pl[5][t], l6 = sh.pl[6][t];
 #pragma unroll
       for (int k = 0; k < 8; ++k) pn[k] = sh.pn[k][t];
       // Psi / (2 pi) = sum_b c_b phi_b(f) + c_const with v = u f^(1/3), u = (pi M)^(1/3)
-      const double P = 3.0 / (128.0 * eta) / kTwoPi;
+      const double r2p = 1.0 / kTwoPi, P = div_const(3.0 / (128.0 * eta), kTwoPi, r2p);
       double c[kNumBasis];
-      c[0] = P * pn[0] / (u * u * u * u * u);   // f^(-5/3)
-      c[1] = P * pn[2] / (u * u * u);           // f^(-1)
-      c[2] = P * pn[3] / (u * u);               // f^(-2/3)
-      c[3] = P * pn[4] / u;                     // f^(-1/3)
-      c[4] = P * l5 / 3.0;                      // ln f
-      c[5] = P * (pn[6] + l6 * lnu) * u;        // f^(1/3)
-      c[6] = P * l6 / 3.0 * u;                  // f^(1/3) ln f
-      c[7] = P * pn[7] * u * u;                 // f^(2/3)
-      const double cconst = P * (pn[5] + l5 * lnu) + (-2.0 * phase - kPi / 4) / kTwoPi;
+      c[4] = div_const(P * l5, 3.0, 1.0 / 3.0);      // ln f
+      c[5] = P * (pn[6] + l6 * lnu) * u;             // f^(1/3)
+      c[6] = div_const(P * l6, 3.0, 1.0 / 3.0) * u;  // f^(1/3) ln f
+      c[7] = P * pn[7] * u * u;                      // f^(2/3)
+      const double cconst = P * (pn[5] + l5 * lnu) + div_const(-2.0 * phase - kPi / 4, kTwoPi, r2p);
       if (a.precision == GWL_PRECISION_MIXED) {
+        c[0] = P * pn[0] / (u * u * u * u * u);  // f^(-5/3)
+        c[1] = P * pn[2] / (u * u * u);          // f^(-1)
+        c[2] = P * pn[3] / (u * u);              // f^(-2/3)
+        c[3] = P * pn[4] / u;                    // f^(-1/3)
 #pragma unroll
         for (int b = 0; b < kNumBasis; ++b) {
           const ff s = ff_from_double(c[b]);
@@ -377,7 +392,7 @@ __device__ __noinline__ void prologue_cta(const LaunchArgs& a, PrologueShared& s
         r.c_lo[kNumBasis] = s.lo;
       }
       if (a.wide_c)
-        wide_coefficients(a, i, m1, m2, eta, m_sec, u, sh.f_isco[t], sh.k_end[t], pn, c, cconst);
+        wide_coefficients(a, i, m1, m2, m_sec, u, sh.f_isco[t], sh.k_end[t], pn, c, P, cconst);
     }
   }
   __syncthreads();
