@@ -1517,21 +1517,29 @@ __device__ __host__ __forceinline__ int part_components(const LaunchArgs& a) {
 }
 
 // One (point, detector, component) chain: the partial sums of all groups
-// added in group order (loads of 8 groups in flight) into group 0's slot.
+// added in group order into group 0's slot.  Bound by the loads' latency: 32
+// groups in flight (8: 25.8 us for 4096 points of three detectors and 127 groups, here 18.0 us).
 __device__ __forceinline__ void reduce_chain(const LaunchArgs& a, int64_t i, int d, int t) {
   const int64_t G = a.n_groups;
   const int64_t gs = (int64_t)a.n_det * kPartStride * a.B;
   double* q = a.part + ((int64_t)d * kPartStride + t) * a.B + i;
   double p = 0.0;
   int64_t c = 0;
-  for (; c + 8 <= G; c += 8) {
-    double v[8];
+  for (; c + 32 <= G; c += 32) {
+    double v[32];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = q[(c + u) * gs];
+    for (int u = 0; u < 32; ++u) v[u] = q[(c + u) * gs];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) p += v[u];
+    for (int u = 0; u < 32; ++u) p += v[u];
   }
-  for (; c < G; ++c) p += q[c * gs];
+  if (c < G) {
+    double v[32];
+#pragma unroll
+    for (int u = 0; u < 32; ++u) v[u] = c + u < G ? q[(c + u) * gs] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 32; ++u)
+      if (c + u < G) p += v[u];
+  }
   q[0] = p;
 }
 
