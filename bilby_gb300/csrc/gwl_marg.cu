@@ -878,11 +878,63 @@ __global__ void __launch_bounds__(512 >> LS, 1 << LS) k_tm_half(LaunchArgs a, co
         for (int v = 0; v < 16; ++v) buf[P(16 * bb + v)] = make_float2(yr[v], yi[v]);
       }
       __syncthreads();
+      // the window's values: X = sum over the parts of exp(-2 pi i j par / L) Y_par
+      const auto put = [&](int64_t t, const float2 v) {
+        if (par == 0) {
+          s_ew[t] = v;
+        } else {
+          const int64_t qq = ((j_lo + t) * par) & (L - 1);
+          float2 w = qq < hL ? tw(qq) : tw(qq - hL);
+          if (qq >= hL) w = make_float2(-w.x, -w.y);
+          const float2 e = s_ew[t];
+          s_ew[t] = make_float2(e.x + (w.x * v.x - w.y * v.y), e.y + (w.x * v.y + w.y * v.x));
+        }
+      };
+      bool direct = false;  // the last pass below has put them already
       // ---- B: stages 5 .. log2(M); a stage of half-length h has twiddles
       // exp(-2 pi i pos / (2 h)) = tw(pos L / (2 h))
       int stage = 5;
       for (; stage + 3 <= lM; stage += 4) {
         const int64_t h0 = (int64_t)1 << (stage - 1);
+        if (stage + 3 == lM && n_win > 0 && n_win <= 2 * h0) {
+          // the last four stages for the window's outputs alone: of a group's 16
+          // outputs pos + k h0 one or two are in it, and an output needs 15 of the
+          // 32 butterflies, one side of each (the same products and sums).  Beyond
+          // two outputs per group the whole pass does less.  8192 points of 8 s at
+          // 4096 Hz: the kernel 605 -> 587 us.
+          for (int64_t pos = threadIdx.x; pos < h0; pos += blockDim.x) {
+            int64_t t = (pos - j_lo) & (h0 - 1);
+            if (t >= n_win) continue;
+            float2 x[16], w0[4];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) x[k] = buf[P(pos + k * h0)];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) w0[j] = tw(pos * (L >> (stage + j)));
+            for (; t < n_win; t += h0) {
+              const int kk = (int)(((j_lo + t) & (M - 1)) >> (stage - 1));
+              float2 y[16];
+#pragma unroll
+              for (int k = 0; k < 16; ++k) y[k] = x[k];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const float2 u = s_w16[(kk & ((1 << j) - 1)) << (3 - j)];
+                // (rounded as the whole pass rounds them)
+                const float2 w = make_float2(__fmaf_rn(w0[j].x, u.x, -__fmul_rn(w0[j].y, u.y)),
+                                             __fmaf_rn(w0[j].y, u.x, __fmul_rn(w0[j].x, u.y)));
+                const bool minus = (kk >> j) & 1;
+#pragma unroll
+                for (int m = 0; m < (8 >> j); ++m) {
+                  const float2 p = y[2 * m], q = y[2 * m + 1];
+                  const float tr = __fmaf_rn(w.x, q.x, -__fmul_rn(w.y, q.y)), ti = __fmaf_rn(w.x, q.y, __fmul_rn(w.y, q.x));
+                  y[m] = minus ? make_float2(p.x - tr, p.y - ti) : make_float2(p.x + tr, p.y + ti);
+                }
+              }
+              put(t, y[0]);
+            }
+          }
+          direct = true;
+          continue;
+        }
         for (int64_t gi = threadIdx.x; gi < (M >> 4); gi += blockDim.x) {
           const int64_t pos = gi & (h0 - 1);
           const int64_t b0 = ((gi >> (stage - 1)) << (stage + 3)) + pos;
@@ -959,20 +1011,8 @@ __global__ void __launch_bounds__(512 >> LS, 1 << LS) k_tm_half(LaunchArgs a, co
         }
         __syncthreads();
       }
-      // the window's values: X = sum over the parts of exp(-2 pi i j par / L) Y_par
-      for (int64_t t = threadIdx.x; t < n_win; t += blockDim.x) {
-        const int64_t j = j_lo + t;
-        const float2 v = buf[P(j & (M - 1))];
-        if (par == 0) {
-          s_ew[t] = v;
-        } else {
-          const int64_t qq = (j * par) & (L - 1);
-          float2 w = qq < hL ? tw(qq) : tw(qq - hL);
-          if (qq >= hL) w = make_float2(-w.x, -w.y);
-          const float2 e = s_ew[t];
-          s_ew[t] = make_float2(e.x + (w.x * v.x - w.y * v.y), e.y + (w.x * v.y + w.y * v.x));
-        }
-      }
+      if (!direct)
+        for (int64_t t = threadIdx.x; t < n_win; t += blockDim.x) put(t, buf[P((j_lo + t) & (M - 1))]);
       __syncthreads();
     }
     // ---- C: the prior window, per sample in float32 without the point's

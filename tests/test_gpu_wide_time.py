@@ -91,3 +91,27 @@ def test_loudness(gpu, largest, tabulated):
     got = an.log_likelihood_ratio_host(params_block(q), "fp64")[0]
     assert abs(got - ref) <= 1e-9 * max(1.0, largest, hh / 2), (got, ref)
     an.close()
+
+
+# mixed precision at FFT length 16384: the last pass for the window's outputs alone up
+# to 512 of them (two per group of 16), the whole pass above.  Tolerance: the mixed
+# precision's 1e-3 against float64 (windows at the start, the middle and the wrap).
+@pytest.mark.parametrize("samples", [1, 255, 256, 257, 502, 503, 504, 700])
+@pytest.mark.parametrize("at", [0.02, 0.5, 0.999])
+def test_mixed_windows(gpu, samples, at):
+    w = small_workload("tf2_marg_8s")
+    w = small_workload("tf2_marg_8s", **{**w.__dict__, "injection": dict(w.injection, geocent_time=w.start_time + 8 * at)})
+    an = device_analysis(OD.build_workload(w), "taylorf2", w)
+    mid, half = w.start_time + 8 * at, (samples - 0.5) * 8 / 16384 / 2
+    an.set_time_marginalization(True, True, mid - half, mid + half)
+    an.set_phase_marginalization(True)
+    p = draw_points(w, 8, np.random.default_rng(6))
+    for k, v in w.injection.items():
+        p[k][:3] = v
+    p["geocent_time"], p["phase"] = np.full(8, w.start_time), np.zeros(8)
+    block = params_block(p)
+    fp64, mixed = an.log_likelihood_ratio_host(block, "fp64"), an.log_likelihood_ratio_host(block, "mixed")
+    same = np.isinf(fp64)
+    assert np.array_equal(mixed[same], fp64[same])
+    assert np.all(np.abs(mixed - fp64)[~same] <= 1e-3), np.abs(mixed - fp64).max()
+    an.close()
