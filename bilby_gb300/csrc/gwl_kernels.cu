@@ -470,6 +470,7 @@ __device__ __noinline__ void prologue_cta(const LaunchArgs& a, PrologueShared& s
 
 __global__ void __launch_bounds__(kProloguePoints * kPrologueWarps) k_prologue(LaunchArgs a) {
   __shared__ PrologueShared sh;
+  allow_next();
   const int64_t i = (int64_t)blockIdx.x * kProloguePoints + threadIdx.x % kProloguePoints;
   prologue_cta(a, sh, min(i, a.B - 1), i < a.B);
 }
@@ -1070,6 +1071,8 @@ __global__ void __launch_bounds__(kFewUnits) k_mixed_tf2_few(LaunchArgs a) {
   const int64_t g = blockIdx.x, i = blockIdx.y, G = a.n_groups;
   const PointRec& r = a.rec[i];
   const int t = threadIdx.x;
+  allow_next();
+  wait_previous();
   if (r.refine) {
     if (t < 32) acc_unit<D, CPLX>(a, i, g, a.cos_tab);
     return;
@@ -2048,6 +2051,7 @@ __global__ void __launch_bounds__(kFewFinThreads) k_few_finalize(LaunchArgs a) {
   const int64_t i = blockIdx.x, G = a.n_groups, gs = (int64_t)a.n_det * kPartStride * a.B;
   const int nq = part_components(a), chains = a.n_det * nq, t = threadIdx.x;
   double p = 0.0;
+  wait_previous();
   for (int64_t c0 = 0; c0 < G; c0 += kFewFinThreads) {
     const int n = (int)min(G - c0, (int64_t)kFewFinThreads);
     if (t < n)
@@ -2179,22 +2183,17 @@ cudaError_t launch_mixed_acc(const LaunchArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-template <int D>
-constexpr auto k_mixed_tf2_few_c = k_mixed_tf2_few<D, true>;
-template <int D>
-constexpr auto k_mixed_tf2_few_r = k_mixed_tf2_few<D, false>;
-
 cudaError_t launch_mixed_few(const LaunchArgs& a, cudaStream_t s) {
   const dim3 grid((unsigned)a.n_groups, (unsigned)a.B);
-  if (a.cplx) {
-    GWL_DISPATCH_D(k_mixed_tf2_few_c, grid, kFewUnits, 0, s, a);
-  } else {
-    GWL_DISPATCH_D(k_mixed_tf2_few_r, grid, kFewUnits, 0, s, a);
+  cudaError_t e;
+  switch (a.n_det) {
+    case 1: e = launch_after(a.cplx ? k_mixed_tf2_few<1, true> : k_mixed_tf2_few<1, false>, grid, kFewUnits, s, a); break;
+    case 2: e = launch_after(a.cplx ? k_mixed_tf2_few<2, true> : k_mixed_tf2_few<2, false>, grid, kFewUnits, s, a); break;
+    case 3: e = launch_after(a.cplx ? k_mixed_tf2_few<3, true> : k_mixed_tf2_few<3, false>, grid, kFewUnits, s, a); break;
+    default: e = launch_after(a.cplx ? k_mixed_tf2_few<4, true> : k_mixed_tf2_few<4, false>, grid, kFewUnits, s, a); break;
   }
-  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_few_finalize<<<(unsigned)a.B, kFewFinThreads, 0, s>>>(a);
-  return cudaGetLastError();
+  return launch_after(k_few_finalize, dim3((unsigned)a.B), kFewFinThreads, s, a);
 }
 
 // Group sums in parallel over (point, detector, component), then the

@@ -186,6 +186,8 @@ __global__ void __launch_bounds__(kPairThreads) k_wide_tf2_few(LaunchArgs a) {
   const PointRec& r = a.rec[i];
   const WideRows rows = wide_block(a, k0 + sub * kSub);
   int j0 = 0, j1 = 0;
+  allow_next();
+  wait_previous();
   if (r.valid) wide_rows(rows, a.wide_sub ? 0 : r.k_start, wide_end(a, i), j0, j1);
   const int j = 2 * pr;
   const bool on0 = j >= j0 && j < j1, on1 = j + 1 >= j0 && j + 1 < j1;
@@ -289,6 +291,7 @@ __global__ void __launch_bounds__(64 * kMaxDet) k_wide_finalize_few(LaunchArgs a
   const int nc = a.cplx ? 2 : 1, c = threadIdx.x >> 5, d = c / nc;
   const int64_t i = blockIdx.x;
   double h = 0.0;
+  wait_previous();
   if (c == d * nc) h = wide_hh(a, a.rec[i], i, d, lane, lanes);
   const double p = wide_chunk_sum<32>(a.part + (i * a.n_det * nc + c) * a.wide_chunks, a.wide_chunks, lane, lanes);
   if ((threadIdx.x & 31) == 0) {
@@ -368,8 +371,7 @@ template <int D, bool CPLX>
 static cudaError_t launch_wide_d(const LaunchArgs& a, cudaStream_t s) {
   if (wide_few(a.B, a.wide_chunks)) {
     const dim3 grid((unsigned)a.wide_chunks, (unsigned)a.B);
-    k_wide_tf2_few<D, CPLX><<<grid, kPairThreads, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_after(k_wide_tf2_few<D, CPLX>, grid, kPairThreads, s, a);
   }
   constexpr int NC = CPLX ? 2 : 1;
   constexpr int smem = kWideTable * 16 + kChunkPlain * (kNumBasis * 8 + D * 16) + kSubs * D * NC * 32 * 8;
@@ -397,10 +399,9 @@ cudaError_t launch_wide(const LaunchArgs& a, cudaStream_t s) {
   }
   if (e != cudaSuccess) return e;
   if (wide_few(a.B, a.wide_chunks))
-    k_wide_finalize_few<<<(unsigned)a.B, 32 * a.n_det * (a.cplx ? 2 : 1), 0, s>>>(a);
-  else
-    k_wide_finalize<<<(unsigned)((a.B * wide_lanes(a.wide_chunks) + kWideFinThreads - 1) / kWideFinThreads), kWideFinThreads,
-                      0, s>>>(a);
+    return launch_after(k_wide_finalize_few, dim3((unsigned)a.B), 32 * a.n_det * (a.cplx ? 2 : 1), s, a);
+  k_wide_finalize<<<(unsigned)((a.B * wide_lanes(a.wide_chunks) + kWideFinThreads - 1) / kWideFinThreads), kWideFinThreads, 0,
+                    s>>>(a);
   return cudaGetLastError();
 }
 

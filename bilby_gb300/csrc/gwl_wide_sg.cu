@@ -330,6 +330,8 @@ __global__ void __launch_bounds__(kPairThreads) k_wide_sg_few(LaunchArgs a) {
   const int t = threadIdx.x, sub = t / kPer, pr = t % kPer;
   const int64_t k = k0 + 2 * t, ks = k0 + sub * kSub;
   const int64_t i = blockIdx.y;
+  allow_next();
+  wait_previous();
   SgPoint<D> pt;
   pt.load(a, i);
   const SgBlock b = sg_block<D>(a, i, true, ks, pt);
@@ -459,6 +461,7 @@ __global__ void __launch_bounds__(128 * kMaxDet) k_wide_sg_finalize_few(LaunchAr
   const int lanes = wide_lanes(a.n_chunks), lane = threadIdx.x & (lanes - 1), c = threadIdx.x >> 5;
   const int64_t i = blockIdx.x;
   const int n = a.n_det * (a.cplx ? 4 : 3);
+  wait_previous();
   const double p = wide_chunk_sum<32>(a.part + (i * n + c) * a.n_chunks, a.n_chunks, lane, lanes);
   if ((threadIdx.x & 31) == 0) s_p[c] = p;
   __syncthreads();
@@ -469,8 +472,7 @@ template <int D, bool CPLX>
 static cudaError_t launch_wide_sg_d(const LaunchArgs& a, cudaStream_t s) {
   if (wide_few(a.B, a.n_chunks)) {
     const dim3 grid((unsigned)a.n_chunks, (unsigned)a.B);
-    k_wide_sg_few<D, CPLX><<<grid, kPairThreads, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_after(k_wide_sg_few<D, CPLX>, grid, kPairThreads, s, a);
   }
   constexpr int NC = CPLX ? 4 : 3;
   constexpr int smem = kWideTable * 16 + kChunkPlain * D * 24 + kExpTable * 8 + kSubs * D * NC * 32 * 8;
@@ -498,10 +500,9 @@ cudaError_t launch_wide_sg(const LaunchArgs& a, cudaStream_t s) {
   }
   if (e != cudaSuccess) return e;
   if (wide_few(a.B, a.n_chunks))
-    k_wide_sg_finalize_few<<<(unsigned)a.B, 32 * a.n_det * (a.cplx ? 4 : 3), 0, s>>>(a);
-  else
-    k_wide_sg_finalize<<<(unsigned)((a.B * wide_lanes(a.n_chunks) + kWideFinThreads - 1) / kWideFinThreads),
-                         kWideFinThreads, 0, s>>>(a);
+    return launch_after(k_wide_sg_finalize_few, dim3((unsigned)a.B), 32 * a.n_det * (a.cplx ? 4 : 3), s, a);
+  k_wide_sg_finalize<<<(unsigned)((a.B * wide_lanes(a.n_chunks) + kWideFinThreads - 1) / kWideFinThreads),
+                       kWideFinThreads, 0, s>>>(a);
   return cudaGetLastError();
 }
 
