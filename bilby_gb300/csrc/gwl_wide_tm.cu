@@ -297,11 +297,12 @@ constexpr double kTmBesselMax = 500.0;  // as ln_i0: I0(500) = 2.5e215, and its 
 // One CTA per point.  Bound by latency and, at the samples' I0, by the float64
 // pipe (the transforms leave it idle).  6 s at 2048 Hz, two detectors, 2047 points,
 // phase marginalised: 189 us (231 us with a logarithm and an exponential per sample),
-// where the whole float64 transform through global memory (k_time_marg) took 2240 us.  The error
-// of a sample's <d|h> against 80-bit arithmetic, relative to the largest: 3e-15 rms
+// where the whole float64 transform through global memory (k_time_marg) took 2240 us.
+// Seven CTAs per SM instead of six take the call from 267 to 259 us; eight spill more
+// and take 281 us.  The error of a sample's <d|h> against 80-bit arithmetic, relative to the largest: 3e-15 rms
 // (k_time_marg 6e-15).
 template <int LOGM>
-__global__ void __launch_bounds__(tm_threads(LOGM)) k_wide_tm(LaunchArgs a, TmPlan plan) {
+__global__ void __launch_bounds__(tm_threads(LOGM), LOGM == 10 ? 7 : 1) k_wide_tm(LaunchArgs a, TmPlan plan) {
   constexpr int M = 1 << LOGM, T = tm_threads(LOGM), kWarps = T / 32;
   extern __shared__ __align__(16) unsigned char smem[];
   float4* buf = reinterpret_cast<float4*>(smem);
