@@ -201,8 +201,7 @@ struct gwl_analysis {
   int64_t ws_B = 0;
   double* d_out = nullptr;
   PointRec* d_rec = nullptr;
-  uint64_t* d_wide = nullptr;  // float64 TaylorF2: [kWideWords][wide_B], from the first such evaluation on
-  int64_t wide_B = 0;
+  uint64_t* d_wide = nullptr;  // float64 kernels: [kWideWords][ws_B]
   double* d_part = nullptr;
   size_t part_bytes = 0;
   int32_t* d_order = nullptr;       // [ws_B] point ordering of the mixed TaylorF2 kernel
@@ -301,7 +300,6 @@ void free_workspace(gwl_analysis* a) {
   a->d_out = a->d_part = a->d_tm = nullptr;
   a->d_rec = nullptr;
   a->d_wide = nullptr;
-  a->wide_B = 0;
   a->d_order = a->d_order_hist = nullptr;
   a->last_rf_count = nullptr;
   a->ws_B = 0;
@@ -662,6 +660,7 @@ int ensure_workspace(gwl_analysis* a, int64_t B, const LaunchArgs& L) {
   if ((rc = dev_alloc(a, &a->d_out, (size_t)B, false))) return rc;
   if ((rc = dev_alloc(a, &a->d_rec, (size_t)B, false))) return rc;
   if ((rc = dev_alloc(a, &a->d_part, part / sizeof(double), false))) return rc;
+  if ((rc = dev_alloc(a, &a->d_wide, (size_t)kWideWords * B, false))) return rc;
   if ((rc = dev_alloc(a, &a->d_order, (size_t)B, false))) return rc;
   if ((rc = dev_alloc(a, &a->d_order_hist, (size_t)4 * kOrderMaxKeys + 1, false))) return rc;
   if (tm) {
@@ -889,19 +888,9 @@ int run_mb_fft(gwl_analysis* a, LaunchArgs& L, cudaStream_t s) {
 
 // A launch of the float64 kernels on the 32-bit pipes: the real part suffices
 // unless |<d|h>| is needed, and the prologue fills the points' coefficients.
-int prepare_wide(gwl_analysis* a, LaunchArgs& L, cudaStream_t s) {
+void prepare_wide(gwl_analysis* a, LaunchArgs& L) {
   L.cplx = a->phase_marg;
-  if (L.B > a->wide_B) {
-    GWL_CUDA(cudaStreamSynchronize(s));
-    cudaFree(a->d_wide);
-    a->d_wide = nullptr;
-    a->wide_B = 0;
-    int rc = dev_alloc(a, &a->d_wide, (size_t)kWideWords * a->ws_B, false);
-    if (rc) return rc;
-    a->wide_B = a->ws_B;
-  }
   L.wide_c = a->d_wide;
-  return GWL_OK;
 }
 
 // ... larger batches ordered so that a warp's points visit nearly the same bins
@@ -1014,7 +1003,7 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
     L.rf_tol = 0.0;
     const bool mbw = a->multiband && a->mb_wide && precision == GWL_PRECISION_FP64;
     if (mbw) {
-      if ((rc = prepare_wide(a, L, s))) return rc;
+      prepare_wide(a, L);
       if (d_dh) L.cplx = 1;
       L.wide_phi = a->mbw_phi;
       for (int d = 0; d < a->n_det; ++d) {
@@ -1035,7 +1024,7 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
     const bool rbw = a->relbin && a->rb_wide;
     if (rbw) {
       // (float64 results for either precision)
-      if ((rc = prepare_wide(a, L, s))) return rc;
+      prepare_wide(a, L);
       if (d_dh) L.cplx = 1;
       L.wide_phi = a->rbw_phi;
       for (int d = 0; d < a->n_det; ++d) {
@@ -1087,8 +1076,12 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
     return GWL_OK;
   }
   const bool wide = precision == GWL_PRECISION_FP64 && !(a->time_marg && d_out);
-  const bool wide_tm = precision == GWL_PRECISION_FP64 && a->time_marg && d_out && wide_tm_fits(L);
-  if ((wide || wide_tm) && (rc = prepare_wide(a, L, s))) return rc;
+  // (a mixed call builds the float64 kernel's tables too, as it does the float64
+  // twiddles: a float64 call captured after it allocates nothing)
+  bool wide_tm = a->time_marg && d_out && wide_tm_fits(L);
+  if (wide_tm) GWL_CUDA(wide_tm_ready(L, s, &wide_tm));
+  wide_tm = wide_tm && precision == GWL_PRECISION_FP64;
+  if (wide || wide_tm) prepare_wide(a, L);
   if (wide_tm) L.cplx = 0;  // the detectors' arg(conj Q) goes with the phase
   if (d_dh && !wide_tm) L.cplx = 1;  // complex <d|h> requested
   const bool ordered = precision == GWL_PRECISION_MIXED && a->model == GWL_MODEL_TAYLORF2 && !(a->time_marg && d_out);

@@ -399,6 +399,8 @@ cudaError_t launch_time_marginalized(const LaunchArgs& a, cudaStream_t s);
 // ... float64 TaylorF2 over the full grid (gwl_wide_tm.cu), where the prior
 // window's samples fit its convolution and no series is requested
 bool wide_tm_fits(const LaunchArgs& a);
+// ... whether its tables are there: built if not, except while s is captured
+cudaError_t wide_tm_ready(const LaunchArgs& a, cudaStream_t s, bool* ready);
 cudaError_t launch_wide_tm(const LaunchArgs& a, cudaStream_t s);
 // The mixed full-grid time-marginalised kernel's error bounds, from what it
 // stored in the point records: marks the points over the tolerance.

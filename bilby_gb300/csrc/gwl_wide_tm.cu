@@ -539,13 +539,15 @@ cudaError_t with_log2m(int log2m, F f) {
   }
 }
 
-cudaError_t tm_tables(int64_t L, int log2m, int cap, cudaStream_t s, TmTables* out) {
+// build: make them where they are missing (else cudaErrorNotReady)
+cudaError_t tm_tables(int64_t L, int log2m, int cap, cudaStream_t s, TmTables* out, bool build) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   const int M = 1 << log2m;
   const int64_t key = (L << 8) | ((int64_t)log2m << 4) | (8 * (int64_t)cap / M);
   return (cudaError_t)g_tm_tables.get(dev, key, out, [&](TmTables* t) -> int {
+    if (!build) return (int)cudaErrorNotReady;
     float4* p = nullptr;
     cudaError_t rc = cudaMalloc(reinterpret_cast<void**>(&p), 2 * (size_t)M * sizeof(float4));
     if (rc != cudaSuccess) return (int)rc;
@@ -585,16 +587,32 @@ bool wide_tm_fits(const LaunchArgs& a) {
          a.n_fft < ((int64_t)1 << 40) && a.B < ((int64_t)1 << 31) && tm_samples(a) <= (1 << (kTmMaxLog - 1));
 }
 
-cudaError_t launch_wide_tm(const LaunchArgs& a, cudaStream_t s) {
+static TmPlan tm_plan(const LaunchArgs& a) {
   const int64_t need = tm_samples(a);
-  TmPlan p;
+  TmPlan p = {};
   p.log2m = kTmMinLog;
   while ((1 << p.log2m) < 2 * need) ++p.log2m;
   const int M = 1 << p.log2m;
   p.cap = (int)((need + M / 8 - 1) / (M / 8)) * (M / 8);
   p.kb = M - p.cap;
+  return p;
+}
+
+cudaError_t wide_tm_ready(const LaunchArgs& a, cudaStream_t s, bool* ready) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(s, &capture);
+  if (e != cudaSuccess) return e;
+  const TmPlan p = tm_plan(a);
   TmTables t;
-  cudaError_t e = tm_tables(a.n_fft, p.log2m, p.cap, s, &t);
+  e = tm_tables(a.n_fft, p.log2m, p.cap, s, &t, capture == cudaStreamCaptureStatusNone);
+  *ready = e == cudaSuccess;
+  return e == cudaErrorNotReady ? cudaSuccess : e;
+}
+
+cudaError_t launch_wide_tm(const LaunchArgs& a, cudaStream_t s) {
+  TmPlan p = tm_plan(a);
+  TmTables t;
+  cudaError_t e = tm_tables(a.n_fft, p.log2m, p.cap, s, &t, false);  // built by wide_tm_ready
   if (e != cudaSuccess) return e;
   p.tw = t.tw;
   p.spec = t.spec;

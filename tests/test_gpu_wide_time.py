@@ -115,3 +115,29 @@ def test_mixed_windows(gpu, samples, at):
     assert np.array_equal(mixed[same], fp64[same])
     assert np.all(np.abs(mixed - fp64)[~same] <= 1e-3), np.abs(mixed - fp64).max()
     an.close()
+
+
+@pytest.mark.parametrize("time", [False, True])
+@pytest.mark.parametrize("workload", ["tf2_marg_8s", "sg_4s"])
+def test_float64_captured_after_a_mixed_call(gpu, workload, time):
+    """A mixed call leaves nothing for a float64 call of the same size to allocate."""
+    torch = pytest.importorskip("torch")
+    w = small_workload(workload, duration=4.0, sampling_frequency=2048.0)
+    w = small_workload(workload, **{**w.__dict__, "injection": dict(w.injection, geocent_time=w.start_time + 2.0)})
+    an = device_analysis(OD.build_workload(w), w.model, w)
+    if time:
+        an.set_time_marginalization(True, True, w.start_time + 1.92, w.start_time + 2.08)
+    p = draw_points(w, 40, np.random.default_rng(2))
+    block = torch.from_numpy(params_block(p)).cuda()
+    out = torch.zeros(40, dtype=torch.float64, device="cuda")
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        an.log_likelihood_ratio_device(block.data_ptr(), 40, out.data_ptr(), "mixed", stream.cuda_stream)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        an.log_likelihood_ratio_device(block.data_ptr(), 40, out.data_ptr(), "fp64", stream.cuda_stream)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(out.cpu().numpy(), an.log_likelihood_ratio_host(params_block(p), "fp64"))
+    an.close()
