@@ -268,6 +268,10 @@ __device__ __noinline__ void wide_totals(const LaunchArgs& a, int64_t i, const d
     di += z;
     hh += tf2_norm(r, d, a.wide_norm, sum[d]);
   }
+  if (!r.valid) {  // (nothing was summed, and the factors may be undefined)
+    dr = di = 0.0;
+    if (a.wide_sub) hh = 0.0;
+  }
   finish_point(a, r, i, dr, di, hh);
 }
 

@@ -116,6 +116,7 @@ __global__ void k_wide_relbin_finalize(LaunchArgs a) {
     di += z;
     hh += tf2_norm(r, d, 1.0, a.wide_q[d][n] + a.rbw_scale[d] * ((double)v[2] + (double)v[3]));
   }
+  if (!r.valid) dr = di = hh = 0.0;  // (nothing was summed, and the factors may be undefined)
   finish_point(a, r, i, dr, di, hh);
 }
 

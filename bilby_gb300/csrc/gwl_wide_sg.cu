@@ -442,6 +442,7 @@ __device__ __noinline__ void wide_sg_totals(const LaunchArgs& a, int64_t i, cons
     // M^2 (S1 + cos 2 beta S2) with M^2 cos 2 beta = A^2 - C^2
     hh += norm * ((A * A + C * C) * p[1] + (A - C) * (A + C) * p[2]);
   }
+  if (!r.valid) dr = di = hh = 0.0;  // (nothing was summed, and the factors may be undefined)
   finish_point(a, r, i, dr, di, hh);
 }
 

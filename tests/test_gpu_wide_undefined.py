@@ -1,0 +1,64 @@
+"""Points and data that are not defined, in the float64 kernels on the 32-bit pipes
+(csrc/gwl_wide*.cu): what they leave untouched and what they make undefined."""
+import numpy as np
+import pytest
+
+from bilby_gb300 import random as grandom
+from bilby_gb300.analysis import Analysis, DetectorData
+from bilby_gb300.detector import InterferometerList
+from bilby_gb300.multiband import MBGravitationalWaveTransient
+from bilby_gb300.relative import RelativeBinningGravitationalWaveTransient
+from bilby_gb300.source import taylorf2_aligned_frequency_sequence, taylorf2_aligned_relative_binning
+from bilby_gb300.waveform_generator import WaveformGenerator
+from oracle import data as OD
+from tests.gpu_helpers import device_analysis, draw_points, params_block, small_workload
+
+pytestmark = pytest.mark.gpu
+
+TF2_UNDEFINED = [dict(mass_1=-1.0), dict(mass_2=np.nan), dict(luminosity_distance=0.0), dict(phase=np.nan),
+                 dict(ra=np.inf), dict(geocent_time=np.nan), dict(chi_1=np.inf)]
+SG_UNDEFINED = [dict(Q=0.0), dict(Q=-5.0), dict(frequency=-100.0), dict(frequency=0.0), dict(hrss=np.nan), dict(ra=np.nan)]
+
+
+def _workload(name):
+    w = small_workload(name, duration=4.0, sampling_frequency=2048.0, mass_range=(10.0, 40.0))
+    inj = dict(w.injection, geocent_time=w.start_time + 2.5)
+    if w.model == "taylorf2":
+        inj.update(mass_1=30.0, mass_2=25.0)
+    return small_workload(name, **{**w.__dict__, "injection": inj})
+
+
+def _list_analysis(kind, w):
+    """The analysis of a multi-banded or relative-binning likelihood."""
+    grandom.seed(w.seed)
+    ifos = InterferometerList(list(w.detectors))
+    ifos.set_strain_data_from_power_spectral_densities(w.sampling_frequency, w.duration, w.start_time)
+    model = taylorf2_aligned_frequency_sequence if kind == "multiband" else taylorf2_aligned_relative_binning
+    wfg = WaveformGenerator(duration=w.duration, sampling_frequency=w.sampling_frequency, start_time=w.start_time,
+                            frequency_domain_source_model=model, waveform_arguments=dict(minimum_frequency=20.0))
+    if kind == "multiband":
+        return MBGravitationalWaveTransient(ifos, wfg, reference_chirp_mass=8.0)
+    return RelativeBinningGravitationalWaveTransient(ifos, wfg, fiducial_parameters=dict(w.injection))
+
+
+@pytest.mark.parametrize("many", [1, 700])  # one CTA per point, and a lane per point
+@pytest.mark.parametrize("kind", ["burst", "full", "multiband", "relbin"])
+def test_inner_products_of_an_undefined_point_are_zero(gpu, kind, many):
+    """Nothing is summed for it: <d|h> is 0 and, where <h|h> is a sum too, so is that."""
+    w = _workload("sg_4s" if kind == "burst" else "tf2_128s")
+    keep = _list_analysis(kind, w) if kind in ("multiband", "relbin") else None
+    an = keep.analysis if keep is not None else device_analysis(OD.build_workload(w), w.model, w)
+    bad = SG_UNDEFINED if kind == "burst" else TF2_UNDEFINED
+    n = (len(bad) + 1) * many
+    p = draw_points(w, n, np.random.default_rng(4))
+    for q, changes in enumerate(bad):
+        for k, v in changes.items():
+            p[k][q::len(bad) + 1] = v
+    dh, hh = an.inner_products_host(params_block(p), "fp64")
+    good = np.arange(n) % (len(bad) + 1) == len(bad)
+    assert np.all(dh[~good] == 0.0), dh[:len(bad)]
+    if kind != "full":
+        assert np.all(hh[~good] == 0.0), hh[:len(bad)]
+    assert np.all(np.isfinite(dh[good])) and np.all(hh[good] > 0.0)
+    lnl = an.log_likelihood_ratio_host(params_block(p), "fp64")
+    assert np.all(lnl[~good] == -1.7976931348623157e308) and np.all(np.isfinite(lnl[good]))
