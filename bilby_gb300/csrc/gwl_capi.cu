@@ -50,6 +50,7 @@ using namespace gwl;
 struct gwl_analysis {
   int model = 0, n_det = 0;
   int64_t n_bins = 0, n_pad = 0, k_lo = 0, k_hi = 0, k_base = 0, k_fmin = 0;
+  int64_t k_weight = 0;  // the first bin with a weight in any detector
   int64_t n_chunks_plain = 0, n_chunks_mixed = 0;
   double duration = 0, fs = 0, fmin = 0, step = 0, start0 = 0;
   DetGeom geom[kMaxDet];
@@ -1266,7 +1267,10 @@ int build_wide_tables(gwl_analysis* a) {
                                  tf2 ? a->ftab : nullptr, 1.0 / a->w_scale[d], P, a->wide_w[d], a->stream));
   }
   if (tf2) {
-    int64_t k0 = a->k_fmin;
+    // from the first bin that has a weight: the fixed point's digits go to the
+    // largest phase of the table, and at 128 s the first bin's of 1 / 128 Hz is
+    // 500,000 times that of 20 Hz
+    int64_t k0 = std::max(a->k_fmin, a->k_weight);
     while (k0 < a->n_bins && !(a->h_freq[(size_t)k0] > 0)) ++k0;
     if (k0 < a->n_bins) wide_scaling(a->h_freq[(size_t)k0], a->h_freq.back(), a->wide_scale, &a->wide_lnref);
     a->wide_phi = base + (size_t)a->n_det * P;
@@ -1430,6 +1434,7 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
       if ((rc = stage.add(&a->cos_tab, ct))) goto fail;
     }
     a->noise_lnl = 0.0;
+    a->k_weight = N;
     std::vector<double> f76, f73;  // f^(-7/6), f^(-7/3)
     if (a->model == GWL_MODEL_TAYLORF2) {
       f76.resize((size_t)N);
@@ -1449,6 +1454,7 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
         s[2 * k + 1] = det.strain[2 * k + 1];
         const double S = det.psd[k];
         ip[k] = (std::isfinite(S) && S > 0) ? 1.0 / S : 0.0;
+        if (ip[k] != 0.0) a->k_weight = std::min(a->k_weight, k);
         // base.py:402-411: |<d|d>| / 2 with <a|b> = 4/T sum conj(a) b / S
         dd.add((s[2 * k] * s[2 * k] + s[2 * k + 1] * s[2 * k + 1]) * ip[k]);
       }

@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(tm_threads(LOGM), LOGM == 10 ? 7 : 1) k_wide_t
     shift = (int)w[(int64_t)(kNumBasis + 1) * a.B];
   }
   __syncthreads();
-  const int64_t j0 = s_j0, ks = r.k_start, ke = min(r.k_end, L);
+  const int64_t j0 = s_j0, ks = max(r.k_start, a.k_lo), ke = min(r.k_end, L);  // (no weights below k_lo)
   const int n = s_n;
   for (int t = threadIdx.x; t < n; t += T) acc[t] = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int64_t k0 = ks & ~(int64_t)1; k0 < ke; k0 += plan.kb) {
