@@ -393,11 +393,19 @@ void wide_scaling(double lo, double hi, double* scale, double* lnref) {
   }
 }
 
+// The scale of float pairs: the largest finite magnitude.  An infinite or undefined
+// weight stays one, and makes undefined only the points that visit it.
+void wide_largest(double* top, double x) {
+  if (std::isfinite(x)) *top = std::max(*top, std::fabs(x));
+}
+
 // |w| (float pair) and arg(w) (0.64 cycles) of point k into LaunchArgs::wide_w
 void wide_weight(std::vector<uint4>* out, int64_t k, double x, double y) {
-  const double turn = std::atan2(y, x) / (2.0 * M_PI);
+  double turn = std::atan2(y, x) / (2.0 * M_PI);
+  turn -= std::floor(turn);
+  if (!(turn >= 0.0 && turn < 1.0)) turn = 0.0;  // (an undefined weight, or -1e-17)
   const float2 m = split_ff(std::hypot(x, y));
-  const uint64_t t = wide_fraction(turn < 0 ? turn + 1.0 : turn, 0.0);
+  const uint64_t t = wide_fraction(turn, 0.0);
   uint32_t* pair = reinterpret_cast<uint32_t*>(&(*out)[k & ~(int64_t)1]);
   std::memcpy(pair + (k & 1), &m.x, 4);
   std::memcpy(pair + 2 + (k & 1), &m.y, 4);
@@ -1262,9 +1270,8 @@ int build_wide_tables(gwl_analysis* a) {
   if (rc) return rc;
   for (int d = 0; d < a->n_det; ++d) {
     a->wide_w[d] = base + (size_t)d * P;
-    a->wide_wscale[d] = a->w_scale[d];
     GWL_CUDA(launch_wide_weights(reinterpret_cast<const double2*>(a->strain[d]), a->inv_psd[d],
-                                 tf2 ? a->ftab : nullptr, 1.0 / a->w_scale[d], P, a->wide_w[d], a->stream));
+                                 tf2 ? a->ftab : nullptr, 1.0 / a->wide_wscale[d], P, a->wide_w[d], a->stream));
   }
   if (tf2) {
     // from the first bin that has a weight: the fixed point's digits go to the
@@ -1463,7 +1470,7 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
       if ((rc = stage.add(&a->inv_psd[d], ip))) goto fail;
       // mixed-precision weights, scaled into float32 range
       std::vector<double> wr(P, 0.0), wi(P, 0.0);
-      double wmax = 0.0, vmax = 0.0;
+      double wmax = 0.0, vmax = 0.0, wide_max = 0.0;
       for (int64_t k = 0; k < N; ++k) {
         if (ip[k] == 0.0) continue;
         const double amp = a->model == GWL_MODEL_TAYLORF2 ? f76[k] : 1.0;
@@ -1471,8 +1478,11 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
         wi[k] = amp * s[2 * k + 1] * ip[k];
         wmax = std::max(wmax, std::max(std::fabs(wr[k]), std::fabs(wi[k])));
         vmax = std::max(vmax, ip[k]);
+        wide_largest(&wide_max, wr[k]);
+        wide_largest(&wide_max, wi[k]);
       }
       a->w_scale[d] = wmax > 0 ? wmax : 1.0;
+      a->wide_wscale[d] = wide_max > 0 ? wide_max : 1.0;
       a->v_scale[d] = vmax > 0 ? vmax : 1.0;
       std::vector<float2> wf(P, make_float2(0.f, 0.f));
       std::vector<float> vf(P, 0.f);
@@ -1911,17 +1921,18 @@ int build_wide_relbin(gwl_analysis* a, const std::vector<double>& fe, const doub
         // m = b0 / 2 |g_e| |g_{e+1}|; the phase enters with the opposite sign of arg g
         m[e] = v[4] / 2 * amp[e] * amp[e + 1] * std::hypot(g[2 * e], g[2 * e + 1]) * std::hypot(g[2 * e + 2], g[2 * e + 3]);
         turn[e] = (std::atan2(g[2 * e + 1], g[2 * e]) - std::atan2(g[2 * e + 3], g[2 * e + 2])) / (2.0 * M_PI);
-        mtop = std::max(mtop, std::fabs(m[e]));
+        wide_largest(&mtop, m[e]);
       }
       // w = conj(g) (...) f^(-7/6)
       x[e] = amp[e] * (g[2 * e] * wr + g[2 * e + 1] * wi);
       y[e] = amp[e] * (g[2 * e] * wi - g[2 * e + 1] * wr);
-      top = std::max(top, std::max(std::fabs(x[e]), std::fabs(y[e])));
+      wide_largest(&top, x[e]);
+      wide_largest(&top, y[e]);
       acc.add(amp[e] * amp[e] * (g[2 * e] * g[2 * e] + g[2 * e + 1] * g[2 * e + 1]) * c);
       q[e + 1] = acc.value();
     }
-    a->rbw_wscale[d] = top > 0 && std::isfinite(top) ? top : 1.0;
-    a->rbw_mscale[d] = mtop > 0 && std::isfinite(mtop) ? mtop : 1.0;
+    a->rbw_wscale[d] = top > 0 ? top : 1.0;
+    a->rbw_mscale[d] = mtop > 0 ? mtop : 1.0;
     // per edge the pair {w, m}
     std::vector<uint4> w(2 * n, make_uint4(0u, 0u, 0u, 0u));
     for (size_t e = 0; e < n; ++e) {
@@ -2099,7 +2110,8 @@ int build_wide_bands(gwl_analysis* a, const std::vector<double>& fr, const std::
       // conj(s) conj(L): the weight of e^{+i phase} is the conjugate coefficient
       x[(size_t)p] = linear[((size_t)d * n + k) * 2] * w;
       y[(size_t)p] = -linear[((size_t)d * n + k) * 2 + 1] * w;
-      top = std::max(top, std::max(std::fabs(x[(size_t)p]), std::fabs(y[(size_t)p])));
+      wide_largest(&top, x[(size_t)p]);
+      wide_largest(&top, y[(size_t)p]);
       q[(size_t)p + 1] = w * w * quadratic[(size_t)d * n + k];
     }
     a->mbw_wscale[d] = top > 0 ? top : 1.0;

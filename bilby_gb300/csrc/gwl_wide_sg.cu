@@ -436,7 +436,7 @@ __device__ __noinline__ void wide_sg_totals(const LaunchArgs& a, int64_t i, cons
   const double norm = 4.0 / a.duration;
   double dr = 0.0, di = 0.0, hh = 0.0;
   for (int d = 0; d < a.n_det; ++d, p += nc) {
-    const double A = r.fp[d] * r.amp, C = r.fx[d] * r.amp2, m = norm * a.w_scale[d] * hypot(A, C);
+    const double A = r.fp[d] * r.amp, C = r.fx[d] * r.amp2, m = norm * a.wide_wscale[d] * hypot(A, C);
     dr += m * p[0];
     if (a.cplx) di += m * p[3];
     // M^2 (S1 + cos 2 beta S2) with M^2 cos 2 beta = A^2 - C^2

@@ -62,3 +62,54 @@ def test_inner_products_of_an_undefined_point_are_zero(gpu, kind, many):
     assert np.all(np.isfinite(dh[good])) and np.all(hh[good] > 0.0)
     lnl = an.log_likelihood_ratio_host(params_block(p), "fp64")
     assert np.all(lnl[~good] == -1.7976931348623157e308) and np.all(np.isfinite(lnl[good]))
+
+
+def _with_infinite_bin(dets, w, model, k):
+    dd = []
+    for q, d in enumerate(dets):
+        strain = np.array(d.masked_strain)
+        if q == 0 and k is not None:
+            strain[k] = np.inf
+        dd.append(DetectorData(d.name, d.vertex, d.tensor, d.start_time, strain, d.psd, d.mask))
+    return Analysis(model, dets[0].frequency, dd, w.duration, w.sampling_frequency, w.minimum_frequency)
+
+
+@pytest.mark.parametrize("n", [4, 60])  # one CTA per point, and a lane per point
+@pytest.mark.parametrize("time", [False, True])
+def test_an_infinite_bin_beyond_the_band_changes_nothing(gpu, n, time):
+    """The templates that end below it keep their bits; the others are undefined."""
+    w = _workload("tf2_128s")
+    dets = OD.build_workload(w)
+    cut = 4400.0 / 40.0  # f_ISCO of 40 solar masses, 110 Hz
+    an = [_with_infinite_bin(dets, w, "taylorf2", k) for k in (None, int((cut + 8.0) * w.duration))]
+    p = draw_points(w, n, np.random.default_rng(4))
+    p["mass_1"], p["mass_2"] = np.where(np.arange(n) % 2, 25.0, 12.0), np.where(np.arange(n) % 2, 20.0, 11.0)
+    if time:
+        for a in an:
+            a.set_time_marginalization(True, True, w.start_time + 2.45, w.start_time + 2.55)
+        p["geocent_time"] = np.full(n, w.start_time)
+    clean, dirty = (a.log_likelihood_ratio_host(params_block(p), "fp64") for a in an)
+    heavy = np.arange(n) % 2 == 1
+    assert np.array_equal(dirty[heavy], clean[heavy])
+    assert np.all(np.isfinite(clean)) and not np.any(np.isfinite(dirty[~heavy]))
+
+
+@pytest.mark.parametrize("kind", ["multiband", "relbin"])
+def test_an_infinite_coefficient_beyond_the_band_changes_nothing(gpu, kind):
+    w = _workload("tf2_128s")
+    like = _list_analysis(kind, w)
+    n = 60
+    p = draw_points(w, n, np.random.default_rng(4))
+    # f_ISCO 63 and 191 Hz
+    p["mass_1"], p["mass_2"] = np.where(np.arange(n) % 2, 36.0, 12.0), np.where(np.arange(n) % 2, 34.0, 11.0)
+    clean = like.log_likelihood_ratio_batch(p)
+    name = like.interferometers[0].name
+    if kind == "multiband":
+        like.linear_coeffs[name][np.searchsorted(like.banded_frequency_points, 70.0)] = np.inf
+    else:
+        like.summary_data[name][0][np.searchsorted(like.bin_freqs, 70.0)] = np.inf
+    like._upload()
+    dirty = like.log_likelihood_ratio_batch(p)
+    heavy = np.arange(n) % 2 == 1
+    assert np.array_equal(dirty[heavy], clean[heavy])
+    assert np.all(np.isfinite(clean)) and not np.any(np.isfinite(dirty[~heavy]))
