@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <map>
 #include <mutex>
 #include <string>
@@ -51,6 +52,7 @@ struct gwl_analysis {
   int model = 0, n_det = 0;
   int64_t n_bins = 0, n_pad = 0, k_lo = 0, k_hi = 0, k_base = 0, k_fmin = 0;
   int64_t k_weight = 0;  // the first bin with a weight in any detector
+  bool finite_data[kMaxDet] = {};  // every weight is finite
   int64_t n_chunks_plain = 0, n_chunks_mixed = 0;
   double duration = 0, fs = 0, fmin = 0, step = 0, start0 = 0;
   DetGeom geom[kMaxDet];
@@ -1272,6 +1274,9 @@ int build_wide_tables(gwl_analysis* a) {
     a->wide_w[d] = base + (size_t)d * P;
     GWL_CUDA(launch_wide_weights(reinterpret_cast<const double2*>(a->strain[d]), a->inv_psd[d],
                                  tf2 ? a->ftab : nullptr, 1.0 / a->wide_wscale[d], P, a->wide_w[d], a->stream));
+    // a burst reaches every bin, also those whose Gaussians are below the sums'
+    // digits and are not visited: one undefined bin, and all are
+    if (!tf2 && !a->finite_data[d]) a->wide_wscale[d] = std::numeric_limits<double>::quiet_NaN();
   }
   if (tf2) {
     // from the first bin that has a weight: the fixed point's digits go to the
@@ -1471,6 +1476,7 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
       // mixed-precision weights, scaled into float32 range
       std::vector<double> wr(P, 0.0), wi(P, 0.0);
       double wmax = 0.0, vmax = 0.0, wide_max = 0.0;
+      a->finite_data[d] = true;
       for (int64_t k = 0; k < N; ++k) {
         if (ip[k] == 0.0) continue;
         const double amp = a->model == GWL_MODEL_TAYLORF2 ? f76[k] : 1.0;
@@ -1480,6 +1486,7 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
         vmax = std::max(vmax, ip[k]);
         wide_largest(&wide_max, wr[k]);
         wide_largest(&wide_max, wi[k]);
+        a->finite_data[d] = a->finite_data[d] && std::isfinite(wr[k]) && std::isfinite(wi[k]);
       }
       a->w_scale[d] = wmax > 0 ? wmax : 1.0;
       a->wide_wscale[d] = wide_max > 0 ? wide_max : 1.0;

@@ -113,3 +113,25 @@ def test_an_infinite_coefficient_beyond_the_band_changes_nothing(gpu, kind):
     heavy = np.arange(n) % 2 == 1
     assert np.array_equal(dirty[heavy], clean[heavy])
     assert np.all(np.isfinite(clean)) and not np.any(np.isfinite(dirty[~heavy]))
+
+
+@pytest.mark.parametrize("n", [2, 300])  # one CTA per point, and a lane per point
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_an_undefined_bin_of_the_data_is_noticed_by_every_burst(gpu, n, value):
+    """Also by those whose Gaussian at that bin is below the sums' last digit; outside
+    the mask it is not data."""
+    w = _workload("sg_4s")
+    dets = OD.build_workload(w)
+    dd, k = [], int(900 * w.duration)
+    p = draw_points(w, n, np.random.default_rng(4))
+    p["frequency"], p["Q"] = np.linspace(50.0, 300.0, n), np.full(n, 20.0)
+    lnl = []
+    for inside in (True, False):
+        for q, d in enumerate(dets):
+            strain, mask = np.array(d.masked_strain), np.array(d.mask)
+            strain[k] = value
+            mask[k] = inside
+            dd.append(DetectorData(d.name, d.vertex, d.tensor, d.start_time, strain, d.psd, mask))
+        an = Analysis("sinegaussian", dets[0].frequency, dd[-len(dets):], w.duration, w.sampling_frequency, 20.0)
+        lnl.append(an.log_likelihood_ratio_host(params_block(p), "fp64"))
+    assert not np.any(np.isfinite(lnl[0])) and np.all(np.isfinite(lnl[1]))
