@@ -209,6 +209,8 @@ struct gwl_analysis {
   size_t part_bytes = 0;
   int32_t* d_order = nullptr;       // [ws_B] point ordering of the mixed TaylorF2 kernel
   int32_t* d_order_hist = nullptr;  // [4 * kOrderMaxKeys + 1]: bucket counts and cursors, then the marked count
+  int32_t* d_order_wide = nullptr;  // [2 * kOrderMaxKeys + 1] after it, the float64 kernels' (gwl_last_refined
+                                    // reads the last mixed call's count whatever float64 calls came after it)
   int* last_rf_count = nullptr;     // marked points of the last mixed TaylorF2 evaluation (device)
   double* d_tm = nullptr;
   size_t tm_bytes = 0;
@@ -303,7 +305,7 @@ void free_workspace(gwl_analysis* a) {
   a->d_out = a->d_part = a->d_tm = nullptr;
   a->d_rec = nullptr;
   a->d_wide = nullptr;
-  a->d_order = a->d_order_hist = nullptr;
+  a->d_order = a->d_order_hist = a->d_order_wide = nullptr;
   a->last_rf_count = nullptr;
   a->ws_B = 0;
   a->part_bytes = a->tm_bytes = 0;
@@ -673,7 +675,8 @@ int ensure_workspace(gwl_analysis* a, int64_t B, const LaunchArgs& L) {
   if ((rc = dev_alloc(a, &a->d_part, part / sizeof(double), false))) return rc;
   if ((rc = dev_alloc(a, &a->d_wide, (size_t)kWideWords * B, false))) return rc;
   if ((rc = dev_alloc(a, &a->d_order, (size_t)B, false))) return rc;
-  if ((rc = dev_alloc(a, &a->d_order_hist, (size_t)4 * kOrderMaxKeys + 1, false))) return rc;
+  if ((rc = dev_alloc(a, &a->d_order_hist, (size_t)6 * kOrderMaxKeys + 2, false))) return rc;
+  a->d_order_wide = a->d_order_hist + 4 * kOrderMaxKeys + 1;
   if (tm) {
     if ((rc = dev_alloc(a, reinterpret_cast<char**>(&a->d_tm), tm, false))) return rc;
   }
@@ -909,7 +912,7 @@ void prepare_wide(gwl_analysis* a, LaunchArgs& L) {
 cudaError_t order_wide(gwl_analysis* a, LaunchArgs& L, cudaStream_t s) {
   if (wide_few(L.B, L.wide_chunks) || L.B * L.wide_chunks < kOrderWideWork) return cudaSuccess;
   L.order = a->d_order;
-  L.order_hist = a->d_order_hist;
+  L.order_hist = a->d_order_wide;
   ordering_with_marks(L);
   if (a->model == GWL_MODEL_SINEGAUSSIAN) L.order_keys = kOrderMaxKeys;  // 16 x 256 buckets (order_key)
   L.rf_count = nullptr;
