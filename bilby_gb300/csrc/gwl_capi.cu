@@ -69,6 +69,7 @@ struct gwl_analysis {
   int32_t* wide_ve[kMaxDet] = {};
   uint64_t* wide_exp = nullptr;
   uint4* wide_w[kMaxDet] = {};
+  const float4 *wide_tm_tw = nullptr, *wide_tm_spec = nullptr;  // for the window of gwl_set_time_marginalization
   double wide_scale[kNumBasis] = {}, wide_lnref = 0, step_lo = 0, wide_wscale[kMaxDet] = {};
   // float64 TaylorF2 multi-banding on the same kernels (mb_wide: its tables are set)
   int mb_wide = 0, mbw_bands = 0;
@@ -527,6 +528,8 @@ LaunchArgs make_args(gwl_analysis* a, int64_t B, int precision) {
     L.wide_ve[d] = a->wide_ve[d];
   }
   L.wide_exp = a->wide_exp;
+  L.wide_tm_tw = a->wide_tm_tw;
+  L.wide_tm_spec = a->wide_tm_spec;
   for (int b = 0; b < kNumBasis; ++b) L.wide_scale[b] = a->wide_scale[b];
   L.wide_lnref = a->wide_lnref;
   L.wide_base = a->k_base;
@@ -1090,11 +1093,7 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
     return GWL_OK;
   }
   const bool wide = precision == GWL_PRECISION_FP64 && !(a->time_marg && d_out);
-  // (a mixed call builds the float64 kernel's tables too, as it does the float64
-  // twiddles: a float64 call captured after it allocates nothing)
-  bool wide_tm = a->time_marg && d_out && wide_tm_fits(L);
-  if (wide_tm) GWL_CUDA(wide_tm_ready(L, s, &wide_tm));
-  wide_tm = wide_tm && precision == GWL_PRECISION_FP64;
+  const bool wide_tm = precision == GWL_PRECISION_FP64 && a->time_marg && d_out && wide_tm_fits(L);
   if (wide || wide_tm) prepare_wide(a, L);
   if (wide_tm) L.cplx = 0;  // the detectors' arg(conj Q) goes with the phase
   if (d_dh && !wide_tm) L.cplx = 1;  // complex <d|h> requested
@@ -1790,6 +1789,16 @@ int gwl_set_time_marginalization(gwl_analysis* a, int enable, int jitter, double
       return GWL_ERR_UNSUPPORTED;
     }
   }
+  const float4 *tw = nullptr, *spec = nullptr;
+  if (enable) {  // the float64 kernel's tables
+    LaunchArgs L = make_args(a, 1, GWL_PRECISION_FP64);
+    L.n_fft = a->n_bins - 1;
+    L.t_min = t_min;
+    L.t_max = t_max;
+    GWL_CUDA(wide_tm_tables(L, a->stream, &tw, &spec));
+  }
+  a->wide_tm_tw = tw;
+  a->wide_tm_spec = spec;
   a->time_marg = enable ? 1 : 0;
   a->jitter = jitter ? 1 : 0;
   a->t_min = t_min;

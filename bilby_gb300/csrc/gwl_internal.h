@@ -144,6 +144,7 @@ struct LaunchArgs {
   const int4* wide_band;
   int wide_bands;
   const double* wide_q[kMaxDet];
+  const float4 *wide_tm_tw, *wide_tm_spec;  // time marginalised: TmPlan::tw, spec (gwl_wide_tm.cu)
   double rbw_scale[kMaxDet];            // relative binning: scale of the cross terms' weights (gwl_wide_relbin.cu)
   const float4* wide_tab;               // [kWideTable] {cos hi, lo, -2 pi / kWideTable sin hi, lo}
   const uint4* wide_w[kMaxDet];         // [n_pad] per bin pair {|w| / w_scale of both, hi words then lo (floats)},
@@ -399,8 +400,9 @@ cudaError_t launch_time_marginalized(const LaunchArgs& a, cudaStream_t s);
 // ... float64 TaylorF2 over the full grid (gwl_wide_tm.cu), where the prior
 // window's samples fit its convolution and no series is requested
 bool wide_tm_fits(const LaunchArgs& a);
-// ... whether its tables are there: built if not, except while s is captured
-cudaError_t wide_tm_ready(const LaunchArgs& a, cudaStream_t s, bool* ready);
+// ... its tables for the analysis's time prior (LaunchArgs::wide_tm_tw, wide_tm_spec; nullptr where the window
+// does not fit), on the device when it returns
+cudaError_t wide_tm_tables(const LaunchArgs& a, cudaStream_t s, const float4** tw, const float4** spec);
 cudaError_t launch_wide_tm(const LaunchArgs& a, cudaStream_t s);
 // The mixed full-grid time-marginalised kernel's error bounds, from what it
 // stored in the point records: marks the points over the tolerance.

@@ -539,15 +539,13 @@ cudaError_t with_log2m(int log2m, F f) {
   }
 }
 
-// build: make them where they are missing (else cudaErrorNotReady)
-cudaError_t tm_tables(int64_t L, int log2m, int cap, cudaStream_t s, TmTables* out, bool build) {
+cudaError_t tm_tables(int64_t L, int log2m, int cap, cudaStream_t s, TmTables* out) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   const int M = 1 << log2m;
   const int64_t key = (L << 8) | ((int64_t)log2m << 4) | (8 * (int64_t)cap / M);
   return (cudaError_t)g_tm_tables.get(dev, key, out, [&](TmTables* t) -> int {
-    if (!build) return (int)cudaErrorNotReady;
     float4* p = nullptr;
     cudaError_t rc = cudaMalloc(reinterpret_cast<void**>(&p), 2 * (size_t)M * sizeof(float4));
     if (rc != cudaSuccess) return (int)rc;
@@ -582,9 +580,16 @@ int64_t tm_samples(const LaunchArgs& a) {
 // samples' sums, fills an SM's shared memory.  A longer window (2 s at 4096 Hz)
 // is a sizeable part of the segment, where the whole transform (gwl_marg.cu) does
 // little that is not needed.
+static bool tm_window_fits(const LaunchArgs& a) {
+  return a.model == GWL_MODEL_TAYLORF2 && a.n_fft > 0 && a.n_fft < ((int64_t)1 << 40) &&
+         tm_samples(a) <= (1 << (kTmMaxLog - 1));
+}
+
+// (the tables are there for every window that fits: which kernel runs depends on
+// the analysis alone, not on what ran before or whether the stream is captured)
 bool wide_tm_fits(const LaunchArgs& a) {
-  return a.model == GWL_MODEL_TAYLORF2 && !a.relbin && !a.multiband && !a.roq && !a.tm_series && a.n_fft > 0 &&
-         a.n_fft < ((int64_t)1 << 40) && a.B < ((int64_t)1 << 31) && tm_samples(a) <= (1 << (kTmMaxLog - 1));
+  return tm_window_fits(a) && a.wide_tm_tw && !a.relbin && !a.multiband && !a.roq && !a.tm_series &&
+         a.B < ((int64_t)1 << 31);
 }
 
 static TmPlan tm_plan(const LaunchArgs& a) {
@@ -598,24 +603,22 @@ static TmPlan tm_plan(const LaunchArgs& a) {
   return p;
 }
 
-cudaError_t wide_tm_ready(const LaunchArgs& a, cudaStream_t s, bool* ready) {
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  cudaError_t e = cudaStreamIsCapturing(s, &capture);
-  if (e != cudaSuccess) return e;
+cudaError_t wide_tm_tables(const LaunchArgs& a, cudaStream_t s, const float4** tw, const float4** spec) {
+  *tw = *spec = nullptr;
+  if (!tm_window_fits(a)) return cudaSuccess;
   const TmPlan p = tm_plan(a);
   TmTables t;
-  e = tm_tables(a.n_fft, p.log2m, p.cap, s, &t, capture == cudaStreamCaptureStatusNone);
-  *ready = e == cudaSuccess;
-  return e == cudaErrorNotReady ? cudaSuccess : e;
+  const cudaError_t e = tm_tables(a.n_fft, p.log2m, p.cap, s, &t);
+  if (e != cudaSuccess) return e;
+  *tw = t.tw;
+  *spec = t.spec;
+  return cudaSuccess;
 }
 
 cudaError_t launch_wide_tm(const LaunchArgs& a, cudaStream_t s) {
   TmPlan p = tm_plan(a);
-  TmTables t;
-  cudaError_t e = tm_tables(a.n_fft, p.log2m, p.cap, s, &t, false);  // built by wide_tm_ready
-  if (e != cudaSuccess) return e;
-  p.tw = t.tw;
-  p.spec = t.spec;
+  p.tw = a.wide_tm_tw;
+  p.spec = a.wide_tm_spec;
   const unsigned __int128 one = ~(unsigned __int128)0 / (unsigned __int128)(2 * a.n_fft);
   p.inv = (uint64_t)(one >> 64);
   p.inv_lo = (uint64_t)one;
