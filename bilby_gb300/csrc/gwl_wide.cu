@@ -379,8 +379,7 @@ static cudaError_t launch_wide_d(const LaunchArgs& a, cudaStream_t s) {
   }
   constexpr int NC = CPLX ? 2 : 1;
   constexpr int smem = kWideTable * 16 + kChunkPlain * (kNumBasis * 8 + D * 16) + kSubs * D * NC * 32 * 8;
-  static const cudaError_t set =
-      cudaFuncSetAttribute(k_wide_tf2<D, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const cudaError_t set = allow_shared(k_wide_tf2<D, CPLX>, smem);
   if (set != cudaSuccess) return set;
   const int64_t tiles = (a.B + 31) / 32;
   const int per = wide_tiles(a.wide_chunks, tiles);

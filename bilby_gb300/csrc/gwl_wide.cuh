@@ -181,6 +181,14 @@ inline int wide_tiles(int64_t chunks, int64_t tiles) {
   return per;
 }
 
+// The kernel's limit of dynamic shared memory, before each launch that needs more
+// than the 48 KB of the default: it belongs to the current device and context,
+// so that one setting per process left a second device's launches refused.
+template <class K>
+inline cudaError_t allow_shared(K kernel, int bytes) {
+  return bytes > 48 * 1024 ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) : cudaSuccess;
+}
+
 // Lanes that add one point's chunks: lane l of them takes chunks l, l + n, ...,
 // then a fixed tree.  With 17 chunks (4 s at 2048 Hz) a whole warp per point
 // took 81 us for 10,000 points, nearly all of it in the tree's float64 adds.

@@ -477,8 +477,7 @@ static cudaError_t launch_wide_sg_d(const LaunchArgs& a, cudaStream_t s) {
   }
   constexpr int NC = CPLX ? 4 : 3;
   constexpr int smem = kWideTable * 16 + kChunkPlain * D * 24 + kExpTable * 8 + kSubs * D * NC * 32 * 8;
-  static const cudaError_t set =
-      cudaFuncSetAttribute(k_wide_sg<D, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const cudaError_t set = allow_shared(k_wide_sg<D, CPLX>, smem);
   if (set != cudaSuccess) return set;
   const int64_t tiles = (a.B + 31) / 32;
   const int per = wide_tiles(a.n_chunks, tiles);
