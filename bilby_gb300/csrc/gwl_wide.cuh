@@ -175,9 +175,12 @@ __device__ __forceinline__ void wide_pair(uint64_t a0, uint64_t a1, const uint4&
 // 541 / 574 / 703 us, 20,000 points 923 / 937 / 984 / 1061 us, multi-banding 4001 points
 // 613 / 616 / 651 / 678 us; 128 s, 512 points (16,000 CTAs) 1251 / 1247 / 1249 / 1265 us,
 // 2048 points 4707 / 4657 / 4661 / 4668 us.
+// More than eight where the grid's second axis, which holds 65,535 CTAs, would not
+// take the batch (above 16.8 million points).
 inline int wide_tiles(int64_t chunks, int64_t tiles) {
   int per = 1;
   while (per < 8 && chunks * (tiles / (2 * per)) >= 8192) per *= 2;
+  while ((tiles + per - 1) / per > 65535) per *= 2;
   return per;
 }
 

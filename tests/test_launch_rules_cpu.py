@@ -110,3 +110,10 @@ def runtime(tmp_path_factory):
 def test_batches_on_a_second_device(runtime, detectors, cplx):
     one = (detectors, cplx, 17, 600)
     assert runtime(one + (0,), one + (0,), one + (1,), one + (2,)) == [0] * 8
+
+
+# 65,535 CTAs of eight tiles of 32 points, one point more, and many more
+@pytest.mark.parametrize("points", [65535 * 256, 65535 * 256 + 1, 20_000_000, 400_000_000])
+@pytest.mark.parametrize("chunks", [1, 17])
+def test_batches_beyond_the_grid_of_eight_tiles(runtime, points, chunks):
+    assert runtime((2, 0, chunks, points, 0), (1, 1, chunks, points, 0)) == [0] * 4
