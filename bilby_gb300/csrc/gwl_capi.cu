@@ -1098,7 +1098,7 @@ int run_eval(gwl_analysis* a, const double* d_params, int64_t B, int precision, 
   if (wide_tm) L.cplx = 0;  // the detectors' arg(conj Q) goes with the phase
   if (d_dh && !wide_tm) L.cplx = 1;  // complex <d|h> requested
   const bool ordered = precision == GWL_PRECISION_MIXED && a->model == GWL_MODEL_TAYLORF2 && !(a->time_marg && d_out);
-  const bool few = ordered && B * a->n_chunks_mixed * a->n_det <= kFewMixedWork && B <= 65535;
+  const bool few = ordered && mixed_few(B, a->n_chunks_mixed, a->n_det, a->duration);
   if (few) {
     L.rf_count = L.rf_tol > 0 ? a->d_order_hist : nullptr;
     a->last_rf_count = L.rf_count;

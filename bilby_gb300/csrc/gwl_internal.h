@@ -2,6 +2,7 @@
 // kernel translation units.  Not part of the public ABI (include/gwlnl.h).
 #pragma once
 
+#include <cmath>
 #include <cstddef>
 #include <cstdint>
 #include <vector>
@@ -42,10 +43,27 @@ constexpr double kRefineL1 = 1e-7;
 constexpr double kRefineLoudPower = 10.0;
 constexpr double kRefineDefaultTol = 5e-4;
 constexpr int kCosTable = 1024;        // angles of the float-float cos / sin table of the accurate kernel
-// Mixed TaylorF2: launch_mixed_few up to this many points x chunks x detectors.
-// Measured per call (us), few against one lane per point: 128 s, 3 detectors, 94
-// points 196 / 227, 128 points 252 / 230; 32 s, 2 detectors, 256 points 104 / 392.
+// Mixed TaylorF2: launch_mixed_few up to this many points x chunks x detectors, and
+// from kFewMixedLong seconds on up to kFewMixedSpan (at 128 s) points x chunks.
+// There its time grows with the work (a chunk costs about as much as four
+// detectors' sums in it), the lane per point's hardly, and the less the longer the
+// segment: its anchors get further apart.  Measured per call (us), few against one lane per
+// point: 128 s at 4096 Hz, 3 detectors, 96 points 222 / 284, 201 points 394 / 318, 1
+// detector, 145 points 173 / 181, 290 points 294 / 196; 128 s at 2048 Hz, 1 detector,
+// 292 points 197 / 178, 585 points 347 / 189; 256 s at 2048 Hz, 2 detectors, 73 points 165 /
+// 173, 146 points 273 / 196; 64 s at 2048 Hz, 1 detector, 585 points 213 / 229, 1170
+// points 374 / 239.  Below, few wins up to the first limit with the masses whose inspirals
+// fit the segment: 32 s at 4096 Hz, 1 detector, 1161 points 270 / 382; 8 s at 2048 Hz, 3
+// detectors, 3072 points 127 / 238; 4 s at 1024 Hz, 2 detectors, 18432 points 302 / 387 (with 30 to
+// 60 solar masses in 2 s, a band of some 60 bins, the lane per point wins from some
+// 7000 points of three detectors on: 9216 points 180 / 157).
 constexpr int64_t kFewMixedWork = 144 << 10;
+constexpr double kFewMixedLong = 48.0, kFewMixedSpan = 75e3;
+inline bool mixed_few(int64_t points, int64_t chunks, int detectors, double duration) {
+  const int64_t n = points * chunks;
+  if (points > 65535 || n * detectors > kFewMixedWork) return false;
+  return duration < kFewMixedLong || (double)n * (0.8 + 0.2 * detectors) <= kFewMixedSpan * std::cbrt(128.0 / duration);
+}
 // Float64: one CTA per (chunk, point) up to this many points, or points x chunks.
 // Measured: 128 s (1014 chunks), 8 points 95 / 129, 16 points 148 / 130; 32 s (255),
 // 8 points 44 / 50, 16 points 55 / 51; 8 s (32), 64 points 51 / 57, 128 points 61 / 57.
