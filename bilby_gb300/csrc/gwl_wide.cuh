@@ -37,9 +37,11 @@ __device__ __forceinline__ void two_sum2(float2 a, float2 b, float2& s, float2& 
 // 59-bit integer c 2^(58 - s) = ch 2^27 + cl, the table entry phi / scale as the
 // 58-bit fraction mh 2^-31 + ml 2^-58.  The leading partial product goes to
 // acc, the two cross ones to cross (16 of which stay below 2^62), in units of
-// 2^(s - 62) and 2^(s - 89) cycles.
-__device__ __forceinline__ void wide_mac(int64_t& acc, int64_t& cross, int32_t ch, int32_t cl, int32_t ml, int32_t mh) {
-  acc += (int64_t)ch * mh;
+// 2^(s - 62) and 2^(s - 89) cycles.  acc is meant modulo 2^64, 2^(s + 2) cycles:
+// products of nearly 2^62 add up to more (heavy masses, large spins).
+__host__ __device__ __forceinline__ void wide_mac(uint64_t& acc, int64_t& cross, int32_t ch, int32_t cl, int32_t ml,
+                                                  int32_t mh) {
+  acc += (uint64_t)((int64_t)ch * mh);
   cross += (int64_t)ch * ml;
   cross += (int64_t)cl * mh;
 }
@@ -47,8 +49,8 @@ __device__ __forceinline__ void wide_mac(int64_t& acc, int64_t& cross, int32_t c
 // The phase in cycles modulo one as 0.64 fixed point (shift = s + 2): an error
 // of about 2^(s - 58) cycles, where a float64 phase of up to 2^s cycles has
 // several 2^(s - 53).
-__device__ __forceinline__ uint64_t wide_fraction(int64_t acc, int64_t cross, int shift) {
-  return (uint64_t)(acc + (cross >> 27)) << shift;
+__host__ __device__ __forceinline__ uint64_t wide_fraction(uint64_t acc, int64_t cross, int shift) {
+  return (acc + (uint64_t)(cross >> 27)) << shift;
 }
 
 // The remainder of a 0.64 fixed-point angle about the nearest of the table's
@@ -135,7 +137,8 @@ struct WidePoint {
   }
   // Phi at the bin whose table row is m (kNumBasis entries)
   __device__ __forceinline__ uint64_t phase(const uint4* m) const {
-    int64_t acc = 0, cross = 0;
+    uint64_t acc = 0;
+    int64_t cross = 0;
 #pragma unroll
     for (int b = 0; b < kNumBasis / 2; ++b) {
       const uint4 v = m[b];

@@ -377,7 +377,8 @@ __global__ void __launch_bounds__(tm_threads(LOGM), LOGM == 10 ? 7 : 1) k_wide_t
         const uint4* m = a.wide_phi + k * (kNumBasis / 2);
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-          int64_t s = 0, cross = 0;
+          uint64_t s = 0;
+          int64_t cross = 0;
 #pragma unroll
           for (int v = 0; v < kNumBasis / 2; ++v) {
             const uint4 e = __ldg(m + u * (kNumBasis / 2) + v);
