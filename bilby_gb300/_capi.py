@@ -78,6 +78,7 @@ SIGNATURES = {
     "gwl_noalloc_status": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int)]),
     "gwl_selftest_bounded_wait": (ctypes.c_int, [ctypes.c_uint32, ctypes.c_void_p, ctypes.POINTER(ctypes.c_int),
                                                  ctypes.POINTER(ctypes.c_int)]),
+    "gwl_selftest_analysis_wait": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_uint32, ctypes.POINTER(ctypes.c_int)]),
     "gwl_inject_device_status": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]),
     "gwl_inner_products_device": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int32,
                                                  ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]),

@@ -3086,8 +3086,24 @@ int gwl_inject_device_status(gwl_analysis* a, int value) {
     return GWL_ERR_ARGUMENT;
   }
   std::lock_guard<std::mutex> g(a->mu);
+  GWL_CUDA(launch_set_status(a->status, value, a->stream));
   GWL_CUDA(cudaStreamSynchronize(a->stream));
-  *a->status = value;
+  return GWL_OK;
+}
+
+int gwl_selftest_analysis_wait(gwl_analysis* a, uint32_t poll_limit, int* arrived) {
+  if (!a || !arrived || poll_limit == 0) {
+    set_error("null argument or zero poll limit");
+    return GWL_ERR_ARGUMENT;
+  }
+  std::lock_guard<std::mutex> g(a->mu);
+  int* d = nullptr;
+  GWL_CUDA(cudaMalloc(&d, sizeof(int)));
+  cudaError_t e = launch_wait_selftest(poll_limit, a->status, d, a->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(arrived, d, sizeof(int), cudaMemcpyDeviceToHost, a->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(a->stream);
+  cudaFree(d);
+  GWL_CUDA(e);
   return GWL_OK;
 }
 

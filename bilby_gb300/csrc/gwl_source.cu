@@ -172,4 +172,12 @@ cudaError_t launch_wait_selftest(uint32_t limit, int* status, int* arrived, cuda
   return cudaGetLastError();
 }
 
+// A status recorded as the kernels record theirs.
+__global__ void k_set_status(int* status, int value) { atomicExch(status, value); }
+
+cudaError_t launch_set_status(int* status, int value, cudaStream_t s) {
+  k_set_status<<<1, 1, 0, s>>>(status, value);
+  return cudaGetLastError();
+}
+
 }  // namespace gwl

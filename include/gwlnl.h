@@ -489,11 +489,13 @@ int gwl_batcher_last_refined(gwl_batcher *b, void *stream, int64_t *count);
  * gwl_selftest_bounded_wait runs one CTA that arms a bulk-copy barrier for
  * 16 bytes and issues no copy, so the kernels' bounded wait must give up
  * after `poll_limit` polls: it returns GWL_ERR_TIMEOUT with *device_status = 1
- * and *arrived = 0, nothing left in flight.  gwl_inject_device_status writes
- * `value` into an analysis's device status word, as a kernel whose wait gave
- * up would, so that the next host evaluation reports it (GWL_ERR_TIMEOUT)
- * and clears it. */
+ * and *arrived = 0, nothing left in flight.  gwl_selftest_analysis_wait
+ * does so with the status word of an analysis, which the next host evaluation
+ * reports (GWL_ERR_TIMEOUT) and clears; it returns GWL_OK with *arrived = 0.
+ * gwl_inject_device_status has a kernel write `value` into that word, as one
+ * whose wait gave up or whose index check failed would. */
 int gwl_selftest_bounded_wait(uint32_t poll_limit, void *stream, int *device_status, int *arrived);
+int gwl_selftest_analysis_wait(gwl_analysis *a, uint32_t poll_limit, int *arrived);
 int gwl_inject_device_status(gwl_analysis *a, int value);
 
 /* Description of the last error on this thread ("" if none). */
