@@ -720,7 +720,7 @@ def bench_multiband(name, steps, warmup, batch=16384, seed=37):
             "value": res["fp64"]["value"], "unit": "evals/s", "ms_per_launch": res["fp64"]["ms_per_launch"],
             "precision": "fp64", "mixed": res["mixed"], "mixed_over_fp64": res["mixed"]["value"] / res["fp64"]["value"],
             "max_abs_dlnl_mixed_vs_fp64": float((omx - o64).abs().max().item()), "setup_s": setup_s,
-            "launch": "prologue + one warp per point over the banded frequencies",
+            "launch": "prologue, ordering and the full-grid float64 kernel over the list of banded frequencies (mixed: one warp per point)",
             "time_marginalized": tm, "ifft_fft": ifft}
 
 

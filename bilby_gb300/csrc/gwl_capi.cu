@@ -1414,7 +1414,7 @@ int gwl_analysis_create(const gwl_analysis_desc* desc, gwl_analysis** out) {
         for (int b = 0; b < kNumBasis; ++b) basis[(size_t)k * kNumBasis + b] = split_ff(vals[b]);
       }
       if ((rc = stage.add(&a->basis, basis))) goto fail;
-      // float64 powers of f for the plain kernel
+      // float64 powers of f: the weights' tables and the kernels in float64 (gwl_marg*.cu)
       std::vector<double4> ft((size_t)P, make_double4(0.0, 0.0, 0.0, 0.0));
       for (int64_t k = 0; k < N; ++k) {
         const double x = f[k];
@@ -2654,9 +2654,9 @@ int gwl_time_series_device(gwl_analysis* a, const double* params, int64_t B, dou
 namespace {
 // One evaluation of the B points in the pinned staging buffer h_params into
 // h_out (the caller holds the analysis lock): the launch sequence and one
-// synchronisation.  The kernels read the parameters (the prologue, once or twice)
-// and write the results in the pinned buffers themselves, over the link that the
-// copies would take: without the three copies and their hand-overs between
+// synchronisation.  The kernels read the parameters (the prologue's warps, each value
+// one to four times) and write the results in the pinned buffers themselves, over
+// the link that the copies would take: without the three copies and their hand-overs between
 // engines a call takes less at every size, 64 -> 58 us for one neutron star, 92 ->
 // 79 us for 4096 and 228 -> 208 us for 16384 relative-binning points.
 int eval_staged(gwl_analysis* a, int64_t B, int32_t precision) {
@@ -2694,7 +2694,7 @@ int gwl_eval_host(gwl_analysis* a, const double* params, int64_t B, int32_t prec
   LaunchArgs L = make_args(a, B, precision);
   int rc = ensure_workspace(a, B, L);
   if (rc) return rc;
-  // stage through pinned buffers so that both copies are true async DMA
+  // the pinned buffers that the kernels read and write
   std::memcpy(a->h_params, params, sizeof(double) * GWL_NPARAM * B);
   if ((rc = eval_staged(a, B, precision))) return rc;
   std::memcpy(out, a->h_out, sizeof(double) * B);

@@ -1,12 +1,14 @@
-// Likelihood kernels: per-point prologue, fused float64 ("plain") kernels,
-// fused mixed-precision kernels and the per-point finalize step.
+// Likelihood kernels: the per-point prologue of every evaluation, the ordering of
+// the points, the fused mixed-precision kernels, relative binning, multi-banding
+// and ROQ per point, and the finalize steps (float64 over the full grid: gwl_wide.cu
+// and gwl_wide_sg.cu).
 //
-// Layout: one thread per parameter point (128 points per CTA), the CTA walks
-// one chunk of frequency bins whose data / PSD / basis tables are staged in
-// shared memory once and read by all 128 points (broadcast loads).  Partial
-// sums per (chunk, point, detector) go to a work buffer and are reduced in a
-// fixed order by the finalize kernel, so a point's result does not depend on
-// which other points share its batch.
+// Layout of the mixed batches: one thread per parameter point (128 points per
+// CTA), the CTA walks chunks of frequency bins whose weights are staged in shared
+// memory once and read by all 128 points (broadcast loads).  Partial sums per
+// (group of chunks, point, detector) go to a work buffer and are reduced in a
+// fixed order, so a point's result does not depend on which other points share
+// its batch.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -1369,9 +1371,9 @@ __global__ void __launch_bounds__(kSgPointsPerCta) k_mixed_sg(LaunchArgs a) {
 }
 
 // Sine-Gaussian points whose mixed-precision error bound exceeds the
-// tolerance: float64 totals over the in-band bins (the plain kernel's
-// arithmetic), one CTA per point, fixed-order reduction, then the point's
-// lnL replaces the mixed one.
+// tolerance: totals over the in-band bins in float64 (exp and sincos per bin),
+// one CTA per point, fixed-order reduction, then the point's lnL replaces the
+// mixed one.
 constexpr int kSgRefineThreads = 256;
 
 template <int D>

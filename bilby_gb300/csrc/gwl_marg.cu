@@ -900,8 +900,10 @@ __global__ void __launch_bounds__(512 >> LS, 1 << LS) k_tm_half(LaunchArgs a, co
           // the last four stages for the window's outputs alone: of a group's 16
           // outputs pos + k h0 one or two are in it, and an output needs 15 of the
           // 32 butterflies, one side of each (the same products and sums).  Beyond
-          // two outputs per group the whole pass does less.  8192 points of 8 s at
-          // 4096 Hz: the kernel 605 -> 587 us.
+          // two outputs per group the whole pass does less.  Where log2 M is 8 or 12
+          // the passes end in one of four stages: L = 1024 or 16384.  8192 points of
+          // 8 s at 4096 Hz (L = 16384): the kernel 605 -> 587 us; L = 4096 and 8192 end
+          // in a shorter pass, whose last stages are cut to the window below.
           for (int64_t pos = threadIdx.x; pos < h0; pos += blockDim.x) {
             int64_t t = (pos - j_lo) & (h0 - 1);
             if (t >= n_win) continue;

@@ -68,7 +68,7 @@ __device__ __forceinline__ double mb_fft_hh_total(const LaunchArgs& a, int64_t i
   return s;
 }
 
-// float64 source polarisations of the plain kernels at one frequency.
+// Source polarisations at one frequency, in float64 throughout.
 __device__ __forceinline__ bool plain_pols(const LaunchArgs& a, const PointRec& r, double f, double2& hp, double2& hx) {
   if (a.model == GWL_MODEL_SINEGAUSSIAN) {
     const double pi2 = 9.869604401089358;

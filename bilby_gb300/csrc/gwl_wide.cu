@@ -12,8 +12,9 @@
 // Summation order, the same for every batch size and launch shape: a chunk of
 // kChunkPlain bins is cut into sub-blocks of 32; in a sub-block the even and
 // the odd bins are added in order into one float-float sum each; the
-// sub-blocks' sums are added in order in float64; the finalize adds the chunks
-// (lane l of a warp takes chunks l, l + 32, ..., then a fixed tree).
+// sub-blocks' sums are added in order in float64; the finalize adds the n chunks
+// with wide_lanes(n) = 4, 8 or 32 lanes (lane l takes chunks l, l + lanes, ..., then
+// a fixed tree over the lanes), a number that depends on the analysis alone.
 #include <cuda_runtime.h>
 
 #include <cstdint>

@@ -11,7 +11,7 @@ likelihood itself is evaluated by the fused CUDA kernels behind the C ABI
 
 Extensions: ``log_likelihood_ratio_batch(params)`` evaluates a whole batch
 (numpy arrays -> numpy, or CUDA tensors -> CUDA tensor on the current stream),
-and ``precision`` selects the plain float64 kernels ("fp64", the default and
+and ``precision`` selects the float64 kernels ("fp64", the default and
 the drop-in) or the mixed-precision kernels ("mixed").
 """
 from __future__ import annotations

@@ -52,7 +52,7 @@ typedef enum {
 } gwl_model;
 
 typedef enum {
-  GWL_PRECISION_FP64 = 0,  /* plain fused float64 kernels: the drop-in */
+  GWL_PRECISION_FP64 = 0,  /* the drop-in: float64's accuracy */
   GWL_PRECISION_MIXED = 1  /* float-float phase + fixed-point time shift, float32 products */
 } gwl_precision;
 
@@ -118,7 +118,9 @@ int gwl_noise_log_likelihood(gwl_analysis *a, double *out);
 /* Time marginalisation (base.py:183-195, 325-330, 794-820, 1027-1035).
  * The geocent_time prior must be Uniform(t_min, t_max); jitter != 0 shifts
  * the time grid by each point's GWL_P_TIME_JITTER.  Requires the analysis
- * grid to have an even number of FFT points (n_bins - 1). */
+ * grid to have an even number of FFT points (n_bins - 1).  Builds the float64
+ * kernel's tables for the window on the device where the process has none yet
+ * (not to be called during a stream capture). */
 int gwl_set_time_marginalization(gwl_analysis *a, int enable, int jitter, double t_min, double t_max);
 
 /* A geocent_time prior other than Uniform for time marginalisation: the
@@ -358,7 +360,7 @@ int gwl_set_multiband_ifft_fft(gwl_analysis *a, int enable, const int32_t *ks, c
                                const double *sqrt_window, const double *odd_weights);
 
 /* NVTX ranges (no-ops unless a profiler is attached).  The library marks
- * its entry points (gwl_eval_device, gwl_eval_host with its h2d / launch /
+ * its entry points (gwl_eval_device, gwl_eval_host with its launch and
  * readback steps, gwl_batcher_eval); a caller marks its own phases, e.g. a
  * server's admission, with these.  No counterpart in the reference. */
 int gwl_trace_push(const char *name);
