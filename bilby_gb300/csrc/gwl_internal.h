@@ -162,7 +162,6 @@ struct LaunchArgs {
   const int4* wide_band;
   int wide_bands;
   const double* wide_q[kMaxDet];
-  const float4 *wide_tm_tw, *wide_tm_spec;  // time marginalised: TmPlan::tw, spec (gwl_wide_tm.cu)
   double rbw_scale[kMaxDet];            // relative binning: scale of the cross terms' weights (gwl_wide_relbin.cu)
   const float4* wide_tab;               // [kWideTable] {cos hi, lo, -2 pi / kWideTable sin hi, lo}
   const uint4* wide_w[kMaxDet];         // [n_pad] per bin pair {|w| / w_scale of both, hi words then lo (floats)},
@@ -328,6 +327,7 @@ struct LaunchArgs {
   double* roq_hh;                       // [roq_cn] <h|h>
   int64_t roq_c0, roq_cn;
   int rf_list_only;                     // float64 ROQ time marginalisation of the listed points alone
+  const float4 *wide_tm_tw, *wide_tm_spec;  // time marginalised: TmPlan::tw, spec (gwl_wide_tm.cu)
 };
 
 // A batch over several analyses evaluated by one persistent launch: per item
